@@ -1,11 +1,12 @@
 // clb_internal.cuh - device-side state and helpers shared by the sm_100a kernels of libclb200.
 #pragma once
 
-#include <cstdlib>
-
 #include <cstddef>
 #include <cstdint>
+#include <cstdlib>
 #include <cuda_runtime.h>
+
+#include "clb_div.h"
 
 namespace clb {
 

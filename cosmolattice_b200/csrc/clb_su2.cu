@@ -8,7 +8,7 @@
 
 #include "clb_gws.cuh"
 #include "clb_handle.cuh"
-#include "clb_su2.cuh"
+#include "clb_su2_sweep.cuh"
 #include "clb_vv.h"
 
 #include <cmath>
@@ -18,42 +18,6 @@
 #include <vector>
 
 namespace clb {
-
-using namespace su2d;
-
-namespace {
-constexpr int kSU2Blocks = 148 * 8; // 128-thread grid-stride sweeps
-}
-
-struct SU2Sector {
-  void *f = nullptr, *p = nullptr; // 22 and 19 x N^3 of double (FP64) or float (FP32 form)
-  bool fp32 = false;
-  size_t esz = 8;
-  State *d_st = nullptr;
-  double *d_part = nullptr, *d_sums = nullptr;
-  double *d_stage = nullptr; // one FP64 component, for FP32 conversions
-  void *ph = nullptr;        // U(1) link phases (12 x N^3, storage type), kept by the drifts
-  // kick sweeps: 0 one sweep, 1 two halves, 2 three parts, 3 four parts (S and phi; Phi; A; SU(2))
-  // (CLB_SU2_SPLIT sets both forms).  su2_create takes four parts in FP64 and three in FP32, by
-  // timing at 384^3 VV2 since the kick forms the field averages from its own products (ms per
-  // step): FP64 83.0 whole, 58.3 halves, 45.2 three parts, 40.9 four parts; FP32 44.0, 26.9, 23.3,
-  // 23.3 (at 192^3: FP64 9.20, 6.53, 5.10, 4.73; FP32 4.93, 3.18, 2.90, 2.93).  The tangent-linear
-  // sweep takes four parts in both (256^3 VV2, ms per tangent step, three / four parts: FP64 37.9,
-  // 31.4; FP32 21.5, 19.5).  Every form gives the same state to the last bit.
-  int split = 2;
-  int tan_split = 3;
-  int64_t steps_since_unitarize = 0;
-  Params prm{};
-  // tangent-linear form: d(state) along the coupling direction tan_cd, active while tangent
-  bool tangent = false;
-  CoupDot tan_cd{};
-  void *df = nullptr, *dp = nullptr;
-  TState *d_tst = nullptr;
-  double *d_tpart = nullptr, *d_tsums = nullptr;
-};
-
-// FP32 form: links re-unitarised every this many steps
-constexpr int64_t kUnitarizeEvery = 10;
 
 namespace {
 // PITensor.h's GW source for lphi4SU2U1: the singlet S (component 0), the complex scalar phi
@@ -93,11 +57,16 @@ Params su2_params(const clb_handle *h)
   a.dx2 = c.dx * c.dx;
   a.inv_dx2 = 1.0 / (c.dx * c.dx);
   a.inv_dx = 1.0 / c.dx;
+  const float dxf = (float)c.dx;
+  a.ddx = make_div(a.dx, dxf);
+  a.ddx2 = make_div(a.dx2, dxf * dxf);
   a.qG = m.couplings[0];
   a.qH = m.couplings[1];
   a.gC = m.couplings[2];
   a.gD = m.couplings[3];
   a.gS = m.couplings[4];
+  a.ngrad = ((a.inv_dx * a.inv_dx) * a.inv_dx) / a.gS;
+  a.ngrad_f = ((a.ddx.rf * a.ddx.rf) * a.ddx.rf) * (1.0f / (float)a.gS);
   a.c4 = m.couplings[5];
   const double rfo = m.fStar / m.omegaStar, rof = m.omegaStar / m.fStar;
   a.rfo2 = rfo * rfo;
@@ -141,124 +110,18 @@ Kick lf_kick(double dt, double w)
   return k;
 }
 
-template <class S> void sweep_t(clb_handle *h, int nk, bool rf, bool rp, const Kick &kc)
-{
-  SU2Sector *u = h->su2;
-  const int kind = nk == 0 ? K_U1_REDUCE : K_U1_KICK;
-  const S *f = static_cast<const S *>(u->f);
-  S *p = static_cast<S *>(u->p);
-  // kick sweeps run as two halves (sectors S, phi, Phi, A; then SU(2)) or three parts (S, phi, Phi;
-  // A; SU(2)), which hold fewer registers than one sweep over every sector; reduction-only sweeps
-  // run whole
-#define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
-  CLB_LAUNCH(h, kind, k_kick<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(                                  \
-                          f, p, u->prm, kc, u->d_st, u->d_part, static_cast<const S *>(u->ph)))
-#define CLB_SU2K(NK, RF, RP)                                                                                            \
-  do {                                                                                                                 \
-    if (NK > 0 && u->split == 3) {                                                                                     \
-      CLB_SU2K1(NK, RF, RP, 5);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 6);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->split == 2) {                                                                              \
-      CLB_SU2K1(NK, RF, RP, 3);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->split) {                                                                                   \
-      CLB_SU2K1(NK, RF, RP, 1);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
-    } else {                                                                                                           \
-      CLB_SU2K1(NK, RF, RP, 0);                                                                                        \
-    }                                                                                                                  \
-  } while (0)
-  if (nk == 0) {
-    if (rf && rp)
-      CLB_SU2K(0, true, true);
-    else if (rf)
-      CLB_SU2K(0, true, false);
-    else
-      CLB_SU2K(0, false, true);
-  } else if (nk == 1) {
-    if (rf && rp)
-      CLB_SU2K(1, true, true);
-    else if (rp)
-      CLB_SU2K(1, false, true);
-    else
-      CLB_SU2K(1, false, false);
-  } else {
-    if (rf && rp)
-      CLB_SU2K(2, true, true);
-    else
-      CLB_SU2K(2, false, false);
-  }
-#undef CLB_SU2K
-#undef CLB_SU2K1
-}
-
-template <class S> void sweep_tan_t(clb_handle *h, int nk, bool rf, bool rp, const Kick &kc)
-{
-  SU2Sector *u = h->su2;
-  const int kind = nk == 0 ? K_U1_REDUCE : K_U1_KICK;
-  const S *f = static_cast<const S *>(u->f), *df = static_cast<const S *>(u->df);
-  S *p = static_cast<S *>(u->p), *dp = static_cast<S *>(u->dp);
-#define CLB_SU2T1(NK, RF, RP, SECT)                                                                                     \
-  CLB_LAUNCH(h, kind,                                                                                                   \
-             k_kick_tan<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(f, df, p, dp, u->prm, kc, u->d_tst,    \
-                                                                                  u->tan_cd, u->d_tpart))
-#define CLB_SU2T(NK, RF, RP)                                                                                            \
-  do {                                                                                                                 \
-    if (NK > 0 && u->tan_split == 3) {                                                                                 \
-      CLB_SU2T1(NK, RF, RP, 5);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 6);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->tan_split == 2) {                                                                          \
-      CLB_SU2T1(NK, RF, RP, 3);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->tan_split) {                                                                               \
-      CLB_SU2T1(NK, RF, RP, 1);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
-    } else {                                                                                                           \
-      CLB_SU2T1(NK, RF, RP, 0);                                                                                        \
-    }                                                                                                                  \
-  } while (0)
-  if (nk == 0) {
-    if (rf && rp)
-      CLB_SU2T(0, true, true);
-    else if (rf)
-      CLB_SU2T(0, true, false);
-    else
-      CLB_SU2T(0, false, true);
-  } else if (nk == 1) {
-    if (rf && rp)
-      CLB_SU2T(1, true, true);
-    else if (rp)
-      CLB_SU2T(1, false, true);
-    else
-      CLB_SU2T(1, false, false);
-  } else {
-    if (rf && rp)
-      CLB_SU2T(2, true, true);
-    else
-      CLB_SU2T(2, false, false);
-  }
-#undef CLB_SU2T
-#undef CLB_SU2T1
-}
-
 void sweep(clb_handle *h, int nk, bool rf, bool rp, const Kick &kc)
 {
   SU2Sector *u = h->su2;
   if (u->tangent) {
     if (u->fp32)
-      sweep_tan_t<float>(h, nk, rf, rp, kc);
+      su2_sweep_tan<float>(h, nk, rf, rp, kc);
     else
-      sweep_tan_t<double>(h, nk, rf, rp, kc);
+      su2_sweep_tan<double>(h, nk, rf, rp, kc);
   } else if (u->fp32) {
-    sweep_t<float>(h, nk, rf, rp, kc);
+    su2_sweep<float>(h, nk, rf, rp, kc);
   } else {
-    sweep_t<double>(h, nk, rf, rp, kc);
+    su2_sweep<double>(h, nk, rf, rp, kc);
   }
 }
 

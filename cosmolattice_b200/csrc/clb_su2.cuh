@@ -41,6 +41,9 @@ struct Params {
   int N;
   size_t n3;
   double dx, dx2, inv_dx2, inv_dx;
+  DivBy ddx, ddx2;          // divisions by dx and dx^2
+  double ngrad;             // (1/dx)^3 / gS (su2kernels.h:44), in the form's arithmetic below
+  float ngrad_f;
   double qG, qH, gC, gD, gS, c4;
   double rfo2, rof2; // (fStar/omegaStar)^2 and its inverse
   double alpha, fm2, dt, inv_n3;

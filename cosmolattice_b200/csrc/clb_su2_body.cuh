@@ -55,8 +55,8 @@ template <class T> __device__ __forceinline__ D2<T> isig(int b, const D2<T> &d)
   return D2<T>{cmul(I, d.u), cmul(C2<T>{0, -1}, d.v)};
 }
 // Divisions of the kernels: the FP64 form keeps the reference's rounding (a / b); the FP32 form,
-// bound to no rounding order, multiplies by the reciprocal (formed once per site for dx, dx^2 and
-// the field norms); the tangent-linear types divide as Tan does.
+// bound to no rounding order, multiplies by the reciprocal; the tangent-linear types divide as Tan
+// does.
 template <class T> __device__ __forceinline__ T kdiv(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ float kdiv<float>(float a, float b) { return a * (1.0f / b); }
 // the FP32 tangent-linear form: the value part as kdiv<float> forms it (bitwise the plain form)
@@ -65,6 +65,23 @@ template <> __device__ __forceinline__ Tan<float> kdiv<Tan<float>>(Tan<float> a,
   const float r = 1.0f / b.v, q = a.v * r;
   return Tan<float>(q, (a.d - q * b.d) * r);
 }
+
+// x / dx and x / dx^2 (DivBy) of a tangent pair: the bits of kdiv by the spacing
+__device__ __forceinline__ Tan<double> div_by(Tan<double> a, const DivBy &d)
+{
+  return Tan<double>(clb::div_by(a.v, d), clb::div_by(a.d, d));
+}
+__device__ __forceinline__ Tan<float> div_by(Tan<float> a, const DivBy &d) { return Tan<float>(a.v * d.rf, a.d * d.rf); }
+using clb::div_by;
+// 1 / y of such a divisor
+template <class T> __device__ __forceinline__ T recip(const DivBy &d)
+{
+  if constexpr (sizeof(typename TanTraits<T>::base) == 4)
+    return T(d.rf);
+  else
+    return T(d.rh);
+}
+template <> __device__ __forceinline__ Tan<float> recip<Tan<float>>(const DivBy &d) { return Tan<float>(d.rf, 0.0f); }
 
 template <class T> __device__ __forceinline__ T ipw(T x, int n)
 {
@@ -150,9 +167,9 @@ template <class S, class T> struct Site {
     const T c = F(comp, s);
     T t[3];
     for (int d = 0; d < 3; ++d) t[d] = (F(comp, pl(d)) + F(comp, mi(d))) - 2 * c;
-    return kdiv(T(1), dx * dx) * ((t[0] + t[1]) + t[2]);
+    return recip<T>(a->ddx2) * ((t[0] + t[1]) + t[2]);
   }
-  __device__ __forceinline__ T fd(int comp, size_t t0, size_t t1) const { return kdiv(F(comp, t1) - F(comp, t0), dx); }
+  __device__ __forceinline__ T fd(int comp, size_t t0, size_t t1) const { return div_by(F(comp, t1) - F(comp, t0), a->ddx); }
   __device__ __forceinline__ Q4<T> plaq(int i, int j) const
   {
     return qmul(qmul(qmul(link(i, s), link(j, pl(i))), qdag(link(i, pl(j)))), qdag(link(j, s)));
@@ -219,13 +236,14 @@ __device__ __forceinline__ Site<S, Tan<S>> make_site_tan(const S *f, const S *df
 template <class S, class T> __device__ __forceinline__ T cgrad_term(const Site<S, T> &v, const C2<T> &w, const C2<T> &c)
 {
   const C2<T> d0 = csub(w, c);
-  const C2<T> d{kdiv(d0.re, v.dx), kdiv(d0.im, v.dx)};
+  const C2<T> d{div_by(d0.re, v.a->ddx), div_by(d0.im, v.a->ddx)};
   return d.re * d.re + d.im * d.im;
 }
 template <class S, class T> __device__ __forceinline__ T dgrad_term(const Site<S, T> &v, const D2<T> &w, const D2<T> &c)
 {
   const C2<T> du0 = csub(w.u, c.u), dv0 = csub(w.v, c.v);
-  const C2<T> du{kdiv(du0.re, v.dx), kdiv(du0.im, v.dx)}, dv{kdiv(dv0.re, v.dx), kdiv(dv0.im, v.dx)};
+  const DivBy &dd = v.a->ddx;
+  const C2<T> du{div_by(du0.re, dd), div_by(du0.im, dd)}, dv{div_by(dv0.re, dd), div_by(dv0.im, dd)};
   return (du.re * du.re + du.im * du.im) + (dv.re * dv.re + dv.im * dv.im);
 }
 
@@ -243,9 +261,9 @@ template <class S, class T> __device__ __forceinline__ C2<T> covLapC(const Site<
     plus = d == 0 ? w : cadd(plus, w);
     minus = d == 0 ? m : cadd(minus, m);
   }
-  const T dx2 = v.dx * v.dx;
+  const DivBy &dx2 = v.a->ddx2;
   const C2<T> c = v.cs(v.s);
-  return C2<T>{kdiv((plus.re + minus.re) - 6 * c.re, dx2), kdiv((plus.im + minus.im) - 6 * c.im, dx2)};
+  return C2<T>{div_by((plus.re + minus.re) - 6 * c.re, dx2), div_by((plus.im + minus.im) - 6 * c.im, dx2)};
 }
 
 template <class S, class T> __device__ __forceinline__ void covLapD(const Site<S, T> &v, T out[4], T *g2 = nullptr)
@@ -267,12 +285,12 @@ template <class S, class T> __device__ __forceinline__ void covLapD(const Site<S
       minus = D2<T>{cadd(minus.u, m.u), cadd(minus.v, m.v)};
     }
   }
-  const T dx2 = v.dx * v.dx;
+  const DivBy &dx2 = v.a->ddx2;
   const D2<T> c = v.dbl(v.s);
-  out[0] = kdiv((plus.u.re + minus.u.re) - 6 * c.u.re, dx2);
-  out[1] = kdiv((plus.u.im + minus.u.im) - 6 * c.u.im, dx2);
-  out[2] = kdiv((plus.v.re + minus.v.re) - 6 * c.v.re, dx2);
-  out[3] = kdiv((plus.v.im + minus.v.im) - 6 * c.v.im, dx2);
+  out[0] = div_by((plus.u.re + minus.u.re) - 6 * c.u.re, dx2);
+  out[1] = div_by((plus.u.im + minus.u.im) - 6 * c.u.im, dx2);
+  out[2] = div_by((plus.v.re + minus.v.re) - 6 * c.v.re, dx2);
+  out[3] = div_by((plus.v.im + minus.v.im) - 6 * c.v.im, dx2);
 }
 
 // Kick coefficients pow(aI, 1+alpha), pow(aI, 3+alpha), its half and pow(aI, -1+alpha).
@@ -353,20 +371,27 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
         const T g0 = v.fd(7 + j, s, v.pl(i));
         g0s[i][j] = g0;
         const T g1 = v.fd(7 + j, v.mi(j), v.plmi(i, j));
-        const T t = kdiv(g0 - g1, v.dx);
+        const T t = div_by(g0 - g1, a.ddx);
         grad = j == 0 ? t : grad + t;
       }
       const T Jc = v.gC * cmul(conj_(v.wC(i)), C0).im;
       const T Jd = v.gD * sprod(v.wD(i), D0).im;
-      const T J = kdiv(T(2.0), v.dx) * rfo2 * (Jc + Jd);
+      const T J = 2 * recip<T>(a.ddx) * rfo2 * (Jc + Jd);
       K[7 + i] = G * (lap - grad) - A * J;
     }
     if constexpr (AVG) av->b2A = aB2(v, g0s);
   }
   if constexpr (sect_su2(SECT)) {
     const D2<T> Dg = v.dbl(s);
-    const T normGrad = kdiv(ipw(kdiv(T(1), v.dx), 3), v.gS) * G;
-    const T normSrc = kdiv(T(1), v.dx) * A;
+    T ngrad; // (1/dx)^3 / gS; the tangent form's gS can carry a derivative
+    if constexpr (std::is_same<T, double>::value)
+      ngrad = a.ngrad;
+    else if constexpr (std::is_same<T, float>::value)
+      ngrad = a.ngrad_f;
+    else
+      ngrad = kdiv(ipw(recip<T>(a.ddx), 3), v.gS);
+    const T normGrad = ngrad * G;
+    const T normSrc = recip<T>(a.ddx) * A;
     T pw[3]; // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
     for (int i = 0; i < 3; ++i) {
       T gr[3] = {0, 0, 0}, gb[3] = {0, 0, 0};
@@ -720,13 +745,13 @@ __global__ void __launch_bounds__(128)
     {
       double l[3];
       for (int i = 0; i < 3; ++i) l[i] = q[7 + i] - (double)p[(size_t)(7 + i) * n3 + v.mi(i)];
-      const double LHS = ((l[0] + l[1]) + l[2]) / dx;
+      const double LHS = div_by((l[0] + l[1]) + l[2], a.ddx);
       const double nrm = 2 / dx * a.rfo2;
       const double imc = cmul(conj_(C2<double>{q[1], q[2]}), v.cs(s)).im;
       const double imd = sprod(D2<double>{C2<double>{q[3], q[4]}, C2<double>{q[5], q[6]}}, v.dbl(s)).im;
       const double rho = nrm * a.gC * imc + nrm * a.gD * imd;
       const double RHS = -dx * rho;
-      const double L1 = l[0] / dx, L2 = l[1] / dx, L3 = l[2] / dx;
+      const double L1 = div_by(l[0], a.ddx), L2 = div_by(l[1], a.ddx), L3 = div_by(l[2], a.ddx);
       const double diff = LHS - (RHS + 0.0), sum = L1 * L1 + L2 * L2 + L3 * L3 + (RHS + 0.0) * (RHS + 0.0);
       acc[42] += sqrt(diff * diff);
       acc[43] += sqrt(sum * sum);

@@ -1,0 +1,114 @@
+// clb_su2_sweep_impl.cuh - the kick sweeps' launches (clb_su2_sweep.cuh).
+#pragma once
+
+#include "clb_su2_sweep.cuh"
+
+namespace clb {
+
+template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const Kick &kc)
+{
+  SU2Sector *u = h->su2;
+  const int kind = nk == 0 ? K_U1_REDUCE : K_U1_KICK;
+  const S *f = static_cast<const S *>(u->f);
+  S *p = static_cast<S *>(u->p);
+  // kick sweeps run as two halves (sectors S, phi, Phi, A; then SU(2)) or three parts (S, phi, Phi;
+  // A; SU(2)), which hold fewer registers than one sweep over every sector; reduction-only sweeps
+  // run whole
+#define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
+  CLB_LAUNCH(h, kind, k_kick<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(                                  \
+                          f, p, u->prm, kc, u->d_st, u->d_part, static_cast<const S *>(u->ph)))
+#define CLB_SU2K(NK, RF, RP)                                                                                            \
+  do {                                                                                                                 \
+    if (NK > 0 && u->split == 3) {                                                                                     \
+      CLB_SU2K1(NK, RF, RP, 5);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 6);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
+    } else if (NK > 0 && u->split == 2) {                                                                              \
+      CLB_SU2K1(NK, RF, RP, 3);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
+    } else if (NK > 0 && u->split) {                                                                                   \
+      CLB_SU2K1(NK, RF, RP, 1);                                                                                        \
+      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
+    } else {                                                                                                           \
+      CLB_SU2K1(NK, RF, RP, 0);                                                                                        \
+    }                                                                                                                  \
+  } while (0)
+  if (nk == 0) {
+    if (rf && rp)
+      CLB_SU2K(0, true, true);
+    else if (rf)
+      CLB_SU2K(0, true, false);
+    else
+      CLB_SU2K(0, false, true);
+  } else if (nk == 1) {
+    if (rf && rp)
+      CLB_SU2K(1, true, true);
+    else if (rp)
+      CLB_SU2K(1, false, true);
+    else
+      CLB_SU2K(1, false, false);
+  } else {
+    if (rf && rp)
+      CLB_SU2K(2, true, true);
+    else
+      CLB_SU2K(2, false, false);
+  }
+#undef CLB_SU2K
+#undef CLB_SU2K1
+}
+
+template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, const Kick &kc)
+{
+  SU2Sector *u = h->su2;
+  const int kind = nk == 0 ? K_U1_REDUCE : K_U1_KICK;
+  const S *f = static_cast<const S *>(u->f), *df = static_cast<const S *>(u->df);
+  S *p = static_cast<S *>(u->p), *dp = static_cast<S *>(u->dp);
+#define CLB_SU2T1(NK, RF, RP, SECT)                                                                                     \
+  CLB_LAUNCH(h, kind,                                                                                                   \
+             k_kick_tan<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(f, df, p, dp, u->prm, kc, u->d_tst,    \
+                                                                                  u->tan_cd, u->d_tpart))
+#define CLB_SU2T(NK, RF, RP)                                                                                            \
+  do {                                                                                                                 \
+    if (NK > 0 && u->tan_split == 3) {                                                                                 \
+      CLB_SU2T1(NK, RF, RP, 5);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 6);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
+    } else if (NK > 0 && u->tan_split == 2) {                                                                          \
+      CLB_SU2T1(NK, RF, RP, 3);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
+    } else if (NK > 0 && u->tan_split) {                                                                               \
+      CLB_SU2T1(NK, RF, RP, 1);                                                                                        \
+      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
+    } else {                                                                                                           \
+      CLB_SU2T1(NK, RF, RP, 0);                                                                                        \
+    }                                                                                                                  \
+  } while (0)
+  if (nk == 0) {
+    if (rf && rp)
+      CLB_SU2T(0, true, true);
+    else if (rf)
+      CLB_SU2T(0, true, false);
+    else
+      CLB_SU2T(0, false, true);
+  } else if (nk == 1) {
+    if (rf && rp)
+      CLB_SU2T(1, true, true);
+    else if (rp)
+      CLB_SU2T(1, false, true);
+    else
+      CLB_SU2T(1, false, false);
+  } else {
+    if (rf && rp)
+      CLB_SU2T(2, true, true);
+    else
+      CLB_SU2T(2, false, false);
+  }
+#undef CLB_SU2T
+#undef CLB_SU2T1
+}
+
+} // namespace clb

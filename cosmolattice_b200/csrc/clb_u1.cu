@@ -90,6 +90,8 @@ U1Params make_params(const clb_handle *h)
   a.dx = c.dx;
   a.dx2 = c.dx * c.dx;
   a.inv_dx2 = 1.0 / (c.dx * c.dx);
+  a.ddx = make_div(a.dx, (float)a.dx);
+  a.ddx2 = make_div(a.dx2, (float)a.dx2);
   a.gQ = m.couplings[1];
   a.c4 = m.couplings[0];
   a.ndxg = -c.dx * a.gQ;

@@ -46,6 +46,7 @@ struct U1Params {
   int N;
   size_t n3;
   double dx, dx2, inv_dx2;
+  DivBy ddx, ddx2; // divisions by dx and dx^2
   double ndxg;  // (-dx) gQ: link phase per unit A
   double gQ, c4;
   double J0;    // 2/dx (fStar/omegaStar)^2            (mattercurrents.h:29, 70)
@@ -64,12 +65,12 @@ __device__ __forceinline__ double u1_m(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double u1_a(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double u1_s(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double u1_d(double a, double b) { return __ddiv_rn(a, b); }
-// FP32 form: plain single-precision arithmetic (contraction allowed; a division by dx, dx^2 or
-// |phi| is a multiply by the reciprocal)
+// FP32 form: plain single-precision arithmetic (contraction allowed; a division by |phi| is a
+// multiply by the reciprocal, as div_by is for dx and dx^2)
 __device__ __forceinline__ float u1_m(float a, float b) { return a * b; }
 __device__ __forceinline__ float u1_a(float a, float b) { return a + b; }
 __device__ __forceinline__ float u1_s(float a, float b) { return a - b; }
-__device__ __forceinline__ float u1_d(float a, float b) { return a * (1.0f / b); } // reciprocal formed once per site
+__device__ __forceinline__ float u1_d(float a, float b) { return a * (1.0f / b); }
 __device__ __forceinline__ void u1_sincos(double x, double *sn, double *cs) { sincos(x, sn, cs); }
 __device__ __forceinline__ void u1_sincos(float x, float *sn, float *cs) { sincosf(x, sn, cs); }
 
@@ -88,6 +89,7 @@ __device__ __forceinline__ FD u1_s(FD a, FD b) { return FD(a.v - b.v); }
 __device__ __forceinline__ FD u1_d(FD a, FD b) { return FD(a.v * (1.0 / b.v)); }
 __device__ __forceinline__ FD operator-(FD a) { return FD(-a.v); }
 __device__ __forceinline__ FD sqrt(FD a) { return FD(::sqrt(a.v)); }
+__device__ __forceinline__ FD div_by(FD a, const DivBy &d) { return FD(a.v * d.rh); }
 __device__ __forceinline__ void u1_sincos(FD x, FD *sn, FD *cs) { sincos(x.v, &sn->v, &cs->v); }
 
 // Per-site kernel values in arithmetic type T.  Fields f (storage S): [Re phi, Im phi, A_x, A_y,
@@ -109,7 +111,7 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
   const size_t n3 = a.n3;
   const S *phr = f, *phi = f + n3;
   const S *A[3] = {f + 2 * n3, f + 3 * n3, f + 4 * n3};
-  const T ndxg = (T)a.ndxg, dx = (T)a.dx, dx2 = (T)a.dx2, inv_dx2 = (T)a.inv_dx2, c4 = (T)a.c4;
+  const T ndxg = (T)a.ndxg, inv_dx2 = (T)a.inv_dx2, c4 = (T)a.c4;
   const T J0 = (T)a.J0, gQ = (T)a.gQ;
   o.fr = (T)phr[s];
   o.fi = (T)phi[s];
@@ -146,12 +148,12 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) o.g0[i][j] = u1_d(u1_s((T)A[j][s + op[i]], (T)A[j][s]), dx);
+    for (int j = 0; j < 3; ++j) o.g0[i][j] = div_by(u1_s((T)A[j][s + op[i]], (T)A[j][s]), a.ddx);
   o.nrm = sqrt(u1_a(u1_m(o.fr, o.fr), u1_m(o.fi, o.fi)));
   if (!KERNEL) return;
   // complex scalar: a^{1+alpha} covLap(phi) - a^{3+alpha}/2 (dV/d|phi|)/|phi| phi
-  const T clr = u1_d(u1_s(u1_a(pr, mr), u1_m(T(6.0), o.fr)), dx2);
-  const T cli = u1_d(u1_s(u1_a(pim, mim), u1_m(T(6.0), o.fi)), dx2);
+  const T clr = div_by(u1_s(u1_a(pr, mr), u1_m(T(6.0), o.fr)), a.ddx2);
+  const T cli = div_by(u1_s(u1_a(pim, mim), u1_m(T(6.0), o.fi)), a.ddx2);
   const T nd = u1_m(c4, u1_m(T(4.0), u1_m(u1_m(o.nrm, o.nrm), o.nrm)));
   const T q = u1_d(nd, o.nrm);
   o.Kr = u1_s(u1_m(kA, clr), u1_m(kB2, u1_m(q, o.fr)));
@@ -169,8 +171,8 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
     for (int j = 0; j < 3; ++j) {
       const size_t sj = s + om[j];
       const size_t sij = i == j ? s : s + op[i] + om[j]; // x + i - j
-      const T g1 = u1_d(u1_s((T)A[j][sij], (T)A[j][sj]), dx);
-      const T tj = u1_d(u1_s(o.g0[i][j], g1), dx);
+      const T g1 = div_by(u1_s((T)A[j][sij], (T)A[j][sj]), a.ddx);
+      const T tj = div_by(u1_s(o.g0[i][j], g1), a.ddx);
       grad = j == 0 ? tj : u1_a(grad, tj);
     }
     const T im = u1_s(u1_m(o.wr[i], o.fi), u1_m(o.wi[i], o.fr));
@@ -180,12 +182,12 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
 }
 
 // sum_j |D+_j phi|^2 (fieldfunctionals.h:80-84) from the site's covariant neighbours
-template <class T> __device__ __forceinline__ T u1_cs_grad2(const U1Site<T> &o, T dx)
+template <class T> __device__ __forceinline__ T u1_cs_grad2(const U1Site<T> &o, const DivBy &ddx)
 {
   T acc = 0;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    const T dr = u1_d(u1_s(o.wr[j], o.fr), dx), di = u1_d(u1_s(o.wi[j], o.fi), dx);
+    const T dr = div_by(u1_s(o.wr[j], o.fr), ddx), di = div_by(u1_s(o.wi[j], o.fi), ddx);
     const T n2 = u1_a(u1_m(dr, dr), u1_m(di, di));
     acc = j == 0 ? n2 : u1_a(acc, n2);
   }
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
     U1Site<T> o;
     u1_site<(NK > 0)>(f, a, s, op, om, kA, kB2, kG, o);
     if (RF) {
-      acc[2] += (double)u1_cs_grad2(o, (T)a.dx);
+      acc[2] += (double)u1_cs_grad2(o, a.ddx);
       acc[3] += (double)u1_b2(o);
       acc[4] += (double)u1_pot(o, (T)a.c4);
     }
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
         U1Site<T> o;
         u1_site<(NK > 0)>(ring, av, t, op, om, kA, kB2, kG, o);
         if (RF) {
-          acc[2] += (double)u1_cs_grad2(o, (T)a.dx);
+          acc[2] += (double)u1_cs_grad2(o, a.ddx);
           acc[3] += (double)u1_b2(o);
           acc[4] += (double)u1_pot(o, (T)a.c4);
         }
@@ -652,7 +654,7 @@ __global__ void __launch_bounds__(256)
     const double up2 = u1_a(u1_a(u1_m(q[0], q[0]), u1_m(q[1], q[1])), u1_m(q[2], q[2]));
     const double b2 = u1_b2(o);
     acc[0] += cp2;
-    acc[1] += u1_cs_grad2(o, a.dx);
+    acc[1] += u1_cs_grad2(o, a.ddx);
     acc[2] += up2;
     acc[3] += b2;
     acc[4] += u1_pot(o, a.c4);
@@ -676,10 +678,10 @@ __global__ void __launch_bounds__(256)
       acc[18] += sqrt(u1_a(u1_a(u1_m(b1, b1), u1_m(bb, bb)), u1_m(b3, b3)));
     }
     // Gauss: LHS = sum_i (pi_i(x) - pi_i(x - i)) / dx, RHS = -dx rho, rho = (J0 gQ) Im(conj(pi_phi) phi)
-    const double LHS = u1_d(u1_a(u1_a(l[0], l[1]), l[2]), a.dx);
+    const double LHS = div_by(u1_a(u1_a(l[0], l[1]), l[2]), a.ddx);
     const double im = u1_s(u1_m(pr, o.fi), u1_m(pi, o.fr));
     const double RHS = u1_m(-a.dx, u1_m(gnorm, im));
-    const double L1 = u1_d(l[0], a.dx), L2 = u1_d(l[1], a.dx), L3 = u1_d(l[2], a.dx);
+    const double L1 = div_by(l[0], a.ddx), L2 = div_by(l[1], a.ddx), L3 = div_by(l[2], a.ddx);
     const double diff = u1_s(LHS, RHS);
     const double sum = u1_a(u1_a(u1_a(u1_m(L1, L1), u1_m(L2, L2)), u1_m(L3, L3)), u1_m(RHS, RHS));
     acc[19] += fabs(diff);
