@@ -92,24 +92,6 @@ __attribute__((visibility("hidden"))) void set_global_error(const std::string &m
 namespace {
 
 
-// Launch with the programmatic-stream-serialization attribute: the kernel may start while the
-// previous kernel in the stream drains; it waits (griddep_wait) before touching dependent data.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
-{
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // Sweep geometry: bz x by (z, y) sites per block; the x direction is split so the grid holds about
 // two waves of resident blocks.
 void setup_geometry(clb_handle *h, int blocks_per_sm)

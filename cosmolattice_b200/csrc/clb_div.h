@@ -42,6 +42,13 @@ CLB_DIV_FN double div_by(double x, const DivBy &d)
   return std::fma(std::fma(-q, d.y, x), d.rh, q);
 #endif
 }
-CLB_DIV_FN float div_by(float x, const DivBy &d) { return x * d.rf; }
+CLB_DIV_FN float div_by(float x, const DivBy &d)
+{
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(x, d.rf); // never contracted: every instantiation of a kernel rounds alike
+#else
+  return x * d.rf;
+#endif
+}
 
 } // namespace clb

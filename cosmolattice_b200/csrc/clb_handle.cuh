@@ -131,6 +131,24 @@ const char *const kKindNames[K_NKINDS] = {"scalar_fused_sweep", "scalar_kick_swe
                                           "gauge_reduce",       "u1_adjoint_sweep",  "initial_conditions",
                                           "gw_sweep"};
 
+// Launch with the programmatic-stream-serialization attribute: the kernel may start while the
+// previous kernel in the stream drains; it waits (griddep_wait) before touching dependent data.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 cudaEvent_t take_event(clb_handle *h)
 {
   if (!h->ev_pool.empty()) {

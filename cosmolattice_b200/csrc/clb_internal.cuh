@@ -162,6 +162,49 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV], double *smem /* [N
   }
 }
 
+// Fixed-order sums of the NV columns of a sweep's partial rows (nrows x NV), in G groups of rows
+// (b, b + G, ...): a thread takes column t % NVP of its groups, so a warp's loads are contiguous,
+// and one warp per column adds the group sums.  The block has a multiple of NVP threads (NVP >= NV
+// a power of two), G is a multiple of 32; every thread gets the sums, whose
+// order depends on G alone.
+template <int NV, int NVP, int G>
+__device__ __forceinline__ void rows_reduce(const double *__restrict__ rows, int nrows, double *smem /* NV (G + 1) */,
+                                            double (&v)[NV])
+{
+  constexpr int U = 8; // rows in flight per thread
+  const int k = threadIdx.x % NVP;
+  if (k < NV) {
+    for (int g = threadIdx.x / NVP; g < G; g += blockDim.x / NVP) {
+      double s[U] = {};
+      int b = g;
+      for (; b + (U - 1) * G < nrows; b += U * G)
+#pragma unroll
+        for (int u = 0; u < U; ++u) s[u] += rows[(size_t)(b + u * G) * NV + k];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b + u * G < nrows) s[u] += rows[(size_t)(b + u * G) * NV + k];
+      smem[k * G + g] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+    }
+  }
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = w; c < NV; c += blockDim.x >> 5) {
+    double s = 0;
+#pragma unroll
+    for (int i = 0; i < G; i += 32) s += smem[c * G + i + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) smem[NV * G + c] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = smem[NV * G + j];
+}
+
+// x^e of the tails' coefficients, one per lane: lane l < n forms pow(base, e) with its own base and
+// exponent, so the warp takes one pow's latency for all of them; bcast(r, l) hands out lane l's.
+__device__ __forceinline__ double bcast(double r, int l) { return __shfl_sync(0xffffffffu, r, l); }
+
 // Periodic neighbour offsets of site s = (x N + y) N + z: op[d] to x + d, om[d] to x - d.
 __device__ __forceinline__ void u1_offsets(int N, size_t s, long long (&op)[3], long long (&om)[3])
 {

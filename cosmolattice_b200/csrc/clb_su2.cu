@@ -86,6 +86,7 @@ template <class T> void coefs(StateT<T> &s, double al)
   s.kB = pow(s.aI, 3 + al);
   s.kB2 = pow(s.aI, 3 + al) / 2;
   s.kG = pow(s.aI, -1 + al);
+  s.kS = pow(s.aI, 2 * al + 1);
   s.p3 = pow(s.aSI, al - 3);
   s.p1 = pow(s.aSI, al - 1);
 }
@@ -129,9 +130,9 @@ template <class S> void drift_tan_t(clb_handle *h, double w, bool lf)
 {
   SU2Sector *u = h->su2;
   CLB_LAUNCH(h, K_U1_DRIFT,
-             k_drift_tan<S><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<S *>(u->f), static_cast<S *>(u->df),
-                                                               static_cast<const S *>(u->p), static_cast<const S *>(u->dp),
-                                                               u->prm, w, lf ? 1 : 0, u->d_tst, u->tan_cd));
+             launch_pdl(k_drift_tan<S>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<S *>(u->f),
+                        static_cast<S *>(u->df), static_cast<const S *>(u->p), static_cast<const S *>(u->dp), u->prm, w,
+                        lf ? 1 : 0, (const TState *)u->d_tst, u->tan_cd));
 }
 
 void drift(clb_handle *h, double w, bool lf, double dtd = -1.0)
@@ -146,15 +147,15 @@ void drift(clb_handle *h, double w, bool lf, double dtd = -1.0)
     return;
   }
   if (u->fp32)
-    CLB_LAUNCH(h, K_U1_DRIFT, k_drift<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<float *>(u->f),
-                                                                                 static_cast<const float *>(u->p),
-                                                                                 u->prm, w, lf ? 1 : 0, u->d_st,
-                                                                                 static_cast<float *>(u->ph), dtd));
+    CLB_LAUNCH(h, K_U1_DRIFT,
+               launch_pdl(su2d::k_drift<float>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<float *>(u->f),
+                          static_cast<const float *>(u->p), u->prm, w, lf ? 1 : 0, (const State *)u->d_st,
+                          static_cast<float *>(u->ph), dtd));
   else
-    CLB_LAUNCH(h, K_U1_DRIFT, k_drift<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<double *>(u->f),
-                                                                                  static_cast<const double *>(u->p),
-                                                                                  u->prm, w, lf ? 1 : 0, u->d_st,
-                                                                                  static_cast<double *>(u->ph), dtd));
+    CLB_LAUNCH(h, K_U1_DRIFT,
+               launch_pdl(su2d::k_drift<double>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<double *>(u->f),
+                          static_cast<const double *>(u->p), u->prm, w, lf ? 1 : 0, (const State *)u->d_st,
+                          static_cast<double *>(u->ph), dtd));
 }
 
 // FP32 form: after the drift of every kUnitarizeEvery-th step the links are projected back to
@@ -178,9 +179,11 @@ void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 =
   SU2Sector *u = h->su2;
   TailOp op{flags, reduced ? kSU2Blocks : 0, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
   if (u->tangent)
-    CLB_LAUNCH(h, K_TAIL, su2d::k_tail<Tan<double>><<<1, 256, 0, h->stream>>>(u->d_tpart, op, u->d_tst, u->prm));
+    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<Tan<double>>, dim3(1), dim3(su2d::kTailThreads), 0, h->stream,
+                                     (const double *)u->d_tpart, op, u->d_tst, u->prm));
   else
-    CLB_LAUNCH(h, K_TAIL, su2d::k_tail<double><<<1, 256, 0, h->stream>>>(u->d_part, op, u->d_st, u->prm));
+    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<double>, dim3(1), dim3(su2d::kTailThreads), 0, h->stream,
+                                     (const double *)u->d_part, op, u->d_st, u->prm));
 }
 
 // Value part of the tangent-form scalar state.

@@ -58,6 +58,7 @@ template <class T> struct StateT {
   T g2S, g2C, g2D, b2A, b2G, potI;
   T g2S_SI, g2C_SI, g2D_SI, b2A_SI, b2G_SI, potSI; // position Verlet: half-step field averages
   T kA, kB, kB2, kG; // pow(aI, 1+alpha), pow(aI, 3+alpha), /2, pow(aI, -1+alpha)
+  T kS;              // pow(aI, 2 alpha + 1)
   T p3, p1;          // pow(aSI, alpha-3), pow(aSI, alpha-1); position Verlet: of aI
   int32_t status, pad;
 };
@@ -94,6 +95,7 @@ template <class A, class B, class Fn> inline void zip_state(StateT<A> &x, const 
   fn(x.kB, y.kB);
   fn(x.kB2, y.kB2);
   fn(x.kG, y.kG);
+  fn(x.kS, y.kS);
   fn(x.p3, y.p3);
   fn(x.p1, y.p1);
 }
@@ -125,7 +127,7 @@ template <class T> __device__ __forceinline__ T sf_kernel(const StateT<T> &s, co
 {
   const double al = p.alpha;
   const EnT<T> E = energies_of(s, p);
-  return pow(s.aI, 2 * al + 1) / 3.0 * p.fm2 *
+  return s.kS / 3.0 * p.fm2 *
          ((((al - 2) * ((E.ks + E.kc) + E.kd) + al * ((E.gs + E.gc) + E.gd)) +
            (al - 1) * ((1.0 * (E.ea + E.ba) + E.eg) + E.bg)) +
           (al + 1) * s.potI);
@@ -136,22 +138,26 @@ template <class T> __device__ __host__ inline T rho_of(const StateT<T> &s, const
   return ((((((((((E.ks + E.kc) + E.kd) + E.gs) + E.gc) + E.gd) + E.ea) + E.ba) + E.eg) + E.bg) + 0.0) + s.potI;
 }
 
-// One-thread tail.  T = double: partials [block][kRed]; T = Tan<double>: [block][2 kRed], the
-// values then their tangents.
+// Tail.  T = double: partials [block][kRed]; T = Tan<double>: [block][2 kRed], the values then their
+// tangents.  The sums' grouping is the same in both, so the value part of a tangent run follows
+// the plain run.  After the sums one warp holds the state in every lane, and the powers of a are
+// formed side by side, one per lane.
+constexpr int kTailGroups = 32, kTailThreads = 512;
+__device__ __forceinline__ double bcast_t(double r, int l) { return bcast(r, l); }
+__device__ __forceinline__ Tan<double> bcast_t(Tan<double> r, int l) { return Tan<double>(bcast(r.v, l), bcast(r.d, l)); }
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kTailThreads)
     k_tail(const double *__restrict__ partials, TailOp op, StateT<T> *__restrict__ stp, Params p)
 {
   constexpr int W = TanTraits<T>::is ? 2 : 1;
-  __shared__ double smem[(256 / 32) * kRed * W];
+  __shared__ double smem[kRed * W * (kTailGroups + 1)];
+  griddep_wait();
+  griddep_launch();
   double r[kRed * W];
   for (int k = 0; k < kRed * W; ++k) r[k] = 0;
-  if (op.nblocks > 0) {
-    for (int b = threadIdx.x; b < op.nblocks; b += blockDim.x)
-      for (int k = 0; k < kRed * W; ++k) r[k] += partials[(size_t)b * kRed * W + k];
-    block_reduce<kRed * W, 256>(r, smem);
-  }
-  if (threadIdx.x != 0) return;
+  if (op.nblocks > 0) rows_reduce<kRed * W, kRed * W, kTailGroups>(partials, op.nblocks, smem, r);
+  if (threadIdx.x >= 32) return;
+  const int lane = (int)threadIdx.x;
   StateT<T> s = *stp;
   T v[kRed];
   for (int k = 0; k < kRed; ++k) {
@@ -183,7 +189,7 @@ __global__ void __launch_bounds__(256)
     h[3] = val(s.g2D);
     h[4] = val(s.potI);
   };
-  const bool hist = op.hist != nullptr && op.hist_row >= 0;
+  const bool hist = op.hist != nullptr && op.hist_row >= 0 && lane == 0;
   if (fl & T_STORE_FIELDS) store_fields();
   if (hist && (fl & T_HIST_EARLY)) write_hist();
   if (fl & T_STORE_PI2_I)
@@ -263,17 +269,22 @@ __global__ void __launch_bounds__(256)
     s.aSI = s.aI;
   }
   if (fl & T_FB_ADOT) s.aDotI = T(op.fb);
-  s.kA = pow(s.aI, 1 + p.alpha);
-  s.kB = pow(s.aI, 3 + p.alpha);
-  s.kB2 = pow(s.aI, 3 + p.alpha) / 2;
-  s.kG = pow(s.aI, -1 + p.alpha);
   const T ad = (fl & T_PV_MODE) ? ((fl & (T_PV_DRIFT_A1 | T_FB_PV_HALF)) ? s.aIM : s.aI) : s.aSI;
-  s.p3 = pow(ad, p.alpha - 3);
-  s.p1 = pow(ad, p.alpha - 1);
+  const double al = p.alpha;
+  const double e = lane == 0 ? 1 + al : lane == 1 ? 3 + al : lane == 2 ? -1 + al : lane == 3 ? al - 3
+                                                                : lane == 4 ? al - 1 : 2 * al + 1;
+  const T pw = pow(lane == 3 || lane == 4 ? ad : s.aI, e);
+  s.kA = bcast_t(pw, 0);
+  s.kB = bcast_t(pw, 1);
+  s.kB2 = s.kB / 2;
+  s.kG = bcast_t(pw, 2);
+  s.p3 = bcast_t(pw, 3);
+  s.p1 = bcast_t(pw, 4);
+  s.kS = bcast_t(pw, 5);
   bool ok = finite_(s.aI) && finite_(s.aDotI) && finite_(s.aDotSI) && finite_(s.potI);
   for (int g = 0; g < 5; ++g) ok = ok && finite_(s.pi2[g]);
   if (!ok) s.status = 1;
-  *stp = s;
+  if (lane == 0) *stp = s;
 }
 
 } // namespace su2d

@@ -564,6 +564,8 @@ __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_K
   constexpr int G0 = sect_g0(SECT), G1 = sect_g1(SECT);                   // sectors [G0, G1)
   constexpr int C0 = sector_c0(G0), C1 = sector_c0(G1);                    // momentum components [C0, C1)
   __shared__ double smem[(128 / 32) * kRed];
+  griddep_wait();
+  griddep_launch();
   const State st = *stp;
   double acc[kRed];
   for (int k = 0; k < kRed; ++k) acc[k] = 0;
@@ -644,6 +646,8 @@ __global__ void __launch_bounds__(256)
             S *__restrict__ ph, double dtd)
 {
   // dtd: the time step of this drift (the position Verlet's half drifts pass dt/2)
+  griddep_wait();
+  griddep_launch();
   const double dt = dtd, p3 = stp->p3, p1 = stp->p1;
   const double cC = lf ? p3 * dt : p3 * dt * w;
   const double cA = lf ? p1 * dt : p1 * w * dt;
@@ -835,6 +839,8 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4 ? CLB_SU2_TAN_MINB_F32 : C
   constexpr int G0 = sect_g0(SECT), G1 = sect_g1(SECT);                   // sectors [G0, G1)
   constexpr int C0 = sector_c0(G0), C1 = sector_c0(G1);                    // momentum components [C0, C1)
   __shared__ double smem[(128 / 32) * 2 * kRed];
+  griddep_wait();
+  griddep_launch();
   const Coef<T> C{T(stp->kA), T(stp->kB), T(stp->kB2), T(stp->kG)};
   double acc[2 * kRed];
   for (int k = 0; k < 2 * kRed; ++k) acc[k] = 0;
@@ -926,6 +932,8 @@ __global__ void __launch_bounds__(256)
     k_drift_tan(S *__restrict__ f, S *__restrict__ df, const S *__restrict__ p, const S *__restrict__ dp, Params a,
                 double w, int lf, const TState *__restrict__ stp, CoupDot cd)
 {
+  griddep_wait();
+  griddep_launch();
   using T = Tan<double>;
   const double dt = a.dt;
   const T p3 = stp->p3, p1 = stp->p1;

@@ -15,8 +15,9 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
   // A; SU(2)), which hold fewer registers than one sweep over every sector; reduction-only sweeps
   // run whole
 #define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
-  CLB_LAUNCH(h, kind, k_kick<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(                                  \
-                          f, p, u->prm, kc, u->d_st, u->d_part, static_cast<const S *>(u->ph)))
+  CLB_LAUNCH(h, kind,                                                                                                   \
+             launch_pdl(k_kick<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, p, u->prm, kc,       \
+                        (const State *)u->d_st, u->d_part, static_cast<const S *>(u->ph)))
 #define CLB_SU2K(NK, RF, RP)                                                                                            \
   do {                                                                                                                 \
     if (NK > 0 && u->split == 3) {                                                                                     \
@@ -67,8 +68,8 @@ template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, c
   S *p = static_cast<S *>(u->p), *dp = static_cast<S *>(u->dp);
 #define CLB_SU2T1(NK, RF, RP, SECT)                                                                                     \
   CLB_LAUNCH(h, kind,                                                                                                   \
-             k_kick_tan<S, NK, RF, RP, SECT><<<kSU2Blocks, 128, 0, h->stream>>>(f, df, p, dp, u->prm, kc, u->d_tst,    \
-                                                                                  u->tan_cd, u->d_tpart))
+             launch_pdl(k_kick_tan<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, df, p, dp,       \
+                        u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart))
 #define CLB_SU2T(NK, RF, RP)                                                                                            \
   do {                                                                                                                 \
     if (NK > 0 && u->tan_split == 3) {                                                                                 \

@@ -114,6 +114,7 @@ void set_coefs(U1State &s, double alpha)
   s.kA = std::pow(s.aI, 1 + alpha);
   s.kB2 = std::pow(s.aI, 3 + alpha) / 2;
   s.kG = std::pow(s.aI, -1 + alpha);
+  s.kS = std::pow(s.aI, 2 * alpha + 1);
 }
 
 // Kick factors: complex scalar (dt/2) w and U(1) (dt w)/2 on the VV; (w dt) for both on the leapfrog.
@@ -135,14 +136,15 @@ template <int NK, bool RF, bool RP, class S> void kick_t(clb_handle *h, int kind
       attr = true;
     }
     CLB_LAUNCH(h, kind,
-               k_u1_kick_tile<NK, RF, RP, S><<<kU1Blocks, 256, U1Ring<S>::BYTES, h->stream>>>(
-                   static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc, u->d_st, u->d_part, u->tile_lx));
+               launch_pdl(k_u1_kick_tile<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), U1Ring<S>::BYTES, h->stream,
+                          static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc, (const U1State *)u->d_st,
+                          u->d_part, u->tile_lx, (S *)nullptr, (S *)nullptr));
     return;
   }
   CLB_LAUNCH(h, kind,
-             k_u1_kick<NK, RF, RP, S><<<kU1Blocks, 256, 0, h->stream>>>(static_cast<const S *>(u->f),
-                                                                         static_cast<S *>(u->p), u->prm, kc, u->d_st,
-                                                                         u->d_part));
+             launch_pdl(k_u1_kick<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), 0, h->stream, static_cast<const S *>(u->f),
+                        static_cast<S *>(u->p), u->prm, kc, (const U1State *)u->d_st, u->d_part, (S *)nullptr,
+                        (S *)nullptr));
 }
 template <int NK, bool RF, bool RP> void kick(clb_handle *h, int kind, const U1Kick &kc)
 {
@@ -154,8 +156,8 @@ template <class S> void drift_t(clb_handle *h, double w, double dtd)
 {
   U1Sector *u = h->u1;
   CLB_LAUNCH(h, K_U1_DRIFT,
-             k_u1_drift<S><<<kU1Blocks, 256, 0, h->stream>>>(static_cast<S *>(u->f), static_cast<const S *>(u->p),
-                                                              h->n3, w, dtd, u->d_st));
+             launch_pdl(k_u1_drift<S>, dim3(kU1Blocks), dim3(256), 0, h->stream, static_cast<S *>(u->f),
+                        static_cast<const S *>(u->p), h->n3, w, dtd, (const U1State *)u->d_st));
 }
 // field drifts of weight w over dt (the position Verlet's half drifts pass dt/2: halving is exact,
 // so ((pow dt)/2) w and ((pow w) dt)/2 of positionverlet.h:182-197 are the same numbers)
@@ -184,7 +186,8 @@ void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 =
 {
   U1Sector *u = h->u1;
   TailOp op{flags, reduced ? kU1Blocks : 0, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
-  CLB_LAUNCH(h, K_TAIL, k_u1_tail<<<1, 256, 0, h->stream>>>(u->d_part, op, u->d_st, u->prm));
+  CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail, dim3(1), dim3(kU1TailThreads), 0, h->stream, (const double *)u->d_part, op,
+                                   u->d_st, u->prm));
 }
 
 // Kick-sweep variants by (number of kicks, field reductions, momentum reductions).
@@ -233,9 +236,10 @@ template <int NK, bool RED, class S> void kick_save_t(clb_handle *h, const U1Kic
       attr = true;
     }
     CLB_LAUNCH(h, K_U1_KICK,
-               k_u1_kick_tile<NK, RED, RED, S, true, true><<<kU1Blocks, 256, U1Ring<S>::BYTES, h->stream>>>(
-                   static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc, u->d_st, u->d_part, u->tile_lx,
-                   reinterpret_cast<S *>(slot), reinterpret_cast<S *>(slot + half)));
+               launch_pdl(k_u1_kick_tile<NK, RED, RED, S, true, true>, dim3(kU1Blocks), dim3(256), U1Ring<S>::BYTES,
+                          h->stream, static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc,
+                          (const U1State *)u->d_st, u->d_part, u->tile_lx, reinterpret_cast<S *>(slot),
+                          reinterpret_cast<S *>(slot + half)));
     return;
   }
   CLB_LAUNCH(h, K_U1_KICK,
@@ -296,7 +300,8 @@ void vv_run(clb_handle *h, int64_t nsteps, const SegSave *sv, bool hist = true, 
         U1Sector *u = h->u1;
         const TailOp a{T_STORE_FIELDS | T_STORE_PI2_I | T_VV_KICK_ONE, kU1Blocks, w, 0.0, nullptr, -1};
         const TailOp b{more ? (uint32_t)(T_VV_KICK_HALF | T_STORE_PI2_B | T_VV_DRIFT) : 0u, kU1Blocks, w, wn, nullptr, -1};
-        CLB_LAUNCH(h, K_TAIL, k_u1_tail_split<<<1, 256, 0, h->stream>>>(u->d_part, a, b, u->d_st, u->prm, sv->rec, k + 1));
+        CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail_split, dim3(1), dim3(kU1TailThreads), 0, h->stream,
+                                         (const double *)u->d_part, a, b, u->d_st, u->prm, sv->rec, k + 1));
       } else {
         k_u1_record<<<1, 1, 0, h->stream>>>(h->u1->d_st, sv->rec, k + 1);
       }

@@ -39,6 +39,7 @@ struct U1State {
   double kA;       // pow(aI, 1 + alpha)         (complexscalarkernels.h:33, u1kernels.h:45)
   double kB2;      // pow(aI, 3 + alpha) / 2     (complexscalarkernels.h:34)
   double kG;       // pow(aI, -1 + alpha)        (u1kernels.h:46)
+  double kS;       // pow(aI, 2 alpha + 1)       (scalefactorkernels.h:75)
   int32_t status, pad;
 };
 
@@ -226,6 +227,8 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
               double *__restrict__ partials, S *__restrict__ save_f = nullptr, S *__restrict__ save_p = nullptr)
 {
   __shared__ double smem[(256 / 32) * kU1Red];
+  griddep_wait();
+  griddep_launch();
   using T = typename std::conditional<FAST && sizeof(S) == 8, FD, S>::type;
   const size_t n3 = a.n3;
   const T kA = (T)st->kA, kB2 = (T)st->kB2, kG = (T)st->kG;
@@ -319,6 +322,8 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
   const size_t n3 = a.n3;
   U1Params av = a;
   av.n3 = (size_t)RG::CS; // u1_site reads component c of ring index t at ring[c * CS + t]
+  griddep_wait();
+  griddep_launch();
   const T kA = (T)st->kA, kB2 = (T)st->kB2, kG = (T)st->kG;
   const int tz = threadIdx.x % BZ, ty = threadIdx.x / BZ;
   const int gz = (N + BZ - 1) / BZ, gy = (N + BY - 1) / BY, gxr = (N + LX - 1) / LX;
@@ -420,6 +425,8 @@ __global__ void __launch_bounds__(256)
     k_u1_drift(S *__restrict__ f, const S *__restrict__ p, size_t n3, double w, double dt,
                const U1State *__restrict__ st)
 {
+  griddep_wait();
+  griddep_launch();
   const double cc = u1_m(u1_m(st->cs_drift, dt), w);
   const double cu = u1_m(u1_m(st->u1_drift, w), dt);
   const size_t n = 5 * n3, n2 = 2 * n3;
@@ -438,7 +445,7 @@ __device__ __forceinline__ double u1_sf_kernel(const U1State &s, const U1Params 
   const double Eel = u1_m(e4, s.u1Pi2I), Emag = u1_m(e4, s.u1Mag2I);
   const double br = u1_a(u1_a(u1_a(u1_m(al - 2, Ekcs), u1_m(al, Egcs)), u1_m(al - 1, u1_a(Eel, Emag))),
                          u1_m(al + 1, s.potI));
-  return u1_m(u1_m(pow(s.aI, 2 * al + 1) / 3.0, p.fm2), br);
+  return u1_m(u1_m(s.kS / 3.0, p.fm2), br);
 }
 
 
@@ -453,28 +460,15 @@ __device__ __forceinline__ double u1_sf_kernel_si(const U1State &s, const U1Para
   const double Eel = u1_m(e4, s.u1Pi2SI), Emag = u1_m(e4, s.u1Mag2SI);
   const double br = u1_a(u1_a(u1_a(u1_m(al - 2, Ekcs), u1_m(al, Egcs)), u1_m(al - 1, u1_a(Eel, Emag))),
                          u1_m(al + 1, s.potSI));
-  return u1_m(u1_m(pow(s.aI, 2 * al + 1) / 3.0, p.fm2), br);
+  return u1_m(u1_m(s.kS / 3.0, p.fm2), br);
 }
 
-// One-thread tail: fixed-order sum of the kick-sweep partials and the scale-factor update, in
-// the order of the VelocityVerlet and LeapFrog schedules (same flags as the scalar tail).
-// Fixed-order sum of the kick-sweep partial rows (all threads of one 256-thread block; the
-// totals are valid in thread 0).
-__device__ __forceinline__ void u1_reduce_partials(const double *__restrict__ partials, int nblocks,
-                                                   double (&v)[kU1Red], double *smem)
-{
-#pragma unroll
-  for (int k = 0; k < kU1Red; ++k) v[k] = 0;
-  if (nblocks <= 0) return;
-#pragma unroll 5
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < kU1Red; ++k) v[k] += partials[(size_t)b * kU1Red + k];
-  }
-  block_reduce<kU1Red, 256>(v, smem);
-}
+// Tail: fixed-order sum of the kick-sweep partials and the scale-factor update, in the order of the
+// VelocityVerlet and LeapFrog schedules (same flags as the scalar tail).
+constexpr int kU1TailGroups = 64, kU1TailThreads = 8 * kU1TailGroups;
 
-// The scale-factor update of one tail on the state s from the reduced sums v.
+// The scale-factor update of one tail on the state s from the reduced sums v, by the 32 lanes of
+// one warp alike (each holds the state); lane 0 writes the history row.
 __device__ __forceinline__ void u1_tail_apply(U1State &s, const double (&v)[kU1Red], const TailOp &op, const U1Params &p)
 {
   const double csP = v[0] * p.inv_n3, u1P = v[1] * p.inv_n3, csG = v[2] * p.inv_n3, u1B = v[3] * p.inv_n3;
@@ -496,7 +490,7 @@ __device__ __forceinline__ void u1_tail_apply(U1State &s, const double (&v)[kU1R
     r[3] = s.csGrad2I;
     r[4] = s.potI;
   };
-  const bool hist = op.hist != nullptr && op.hist_row >= 0;
+  const bool hist = op.hist != nullptr && op.hist_row >= 0 && (threadIdx.x & 31) == 0;
   if (fl & T_STORE_FIELDS) {
     s.csGrad2I = csG;
     s.u1Mag2I = u1B;
@@ -582,45 +576,56 @@ __device__ __forceinline__ void u1_tail_apply(U1State &s, const double (&v)[kU1R
   }
   if (fl & T_FB_ADOT) s.aDotI = op.fb;
   const double ad = (fl & T_PV_MODE) ? ((fl & (T_PV_DRIFT_A1 | T_FB_PV_HALF)) ? s.aIM : s.aI) : s.aSI;
-  s.cs_drift = pow(ad, p.alpha - 3);
-  s.u1_drift = pow(ad, p.alpha - 1);
-  s.kA = pow(s.aI, 1 + p.alpha);
-  s.kB2 = pow(s.aI, 3 + p.alpha) / 2;
-  s.kG = pow(s.aI, -1 + p.alpha);
+  // the six powers side by side, one per lane (as six in turn they were most of the tail)
+  const int lane = threadIdx.x & 31;
+  const double al = p.alpha;
+  const double e = lane == 0 ? al - 3 : lane == 1 ? al - 1 : lane == 2 ? 1 + al : lane == 3 ? 3 + al
+                                                                : lane == 4 ? -1 + al : 2 * al + 1;
+  const double r = pow(lane < 2 ? ad : s.aI, e);
+  s.cs_drift = bcast(r, 0);
+  s.u1_drift = bcast(r, 1);
+  s.kA = bcast(r, 2);
+  s.kB2 = bcast(r, 3) / 2;
+  s.kG = bcast(r, 4);
+  s.kS = bcast(r, 5);
   if (!isfinite(s.aI) || !isfinite(s.aDotI) || !isfinite(s.aDotSI) || !isfinite(s.csPi2I) || !isfinite(s.u1Pi2I) ||
       !isfinite(s.csGrad2I) || !isfinite(s.u1Mag2I) || !isfinite(s.potI))
     s.status = 1;
 }
 
-static __global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(kU1TailThreads)
     k_u1_tail(const double *__restrict__ partials, TailOp op, U1State *__restrict__ st, U1Params p)
 {
-  __shared__ double smem[(256 / 32) * kU1Red];
-  double v[kU1Red];
-  u1_reduce_partials(partials, op.nblocks, v, smem);
-  if (threadIdx.x != 0) return;
+  __shared__ double smem[kU1Red * (kU1TailGroups + 1)];
+  griddep_wait();
+  griddep_launch();
   U1State s = *st;
+  double v[kU1Red] = {};
+  if (op.nblocks > 0) rows_reduce<kU1Red, 8, kU1TailGroups>(partials, op.nblocks, smem, v);
+  if (threadIdx.x >= 32) return;
   u1_tail_apply(s, v, op, p);
-  *st = s;
+  if (threadIdx.x == 0) *st = s;
 }
 
 // A stage boundary of the adjoint's segment recompute in one launch: the tail of the merged
 // sweep's first kick (a), the boundary's record row, then the tail of its second kick (b, if
 // b.flags), both from one reduction of the partials; the same values as k_u1_tail(a),
 // k_u1_record, k_u1_tail(b).
-static __global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(kU1TailThreads)
     k_u1_tail_split(const double *__restrict__ partials, TailOp a, TailOp b, U1State *__restrict__ st, U1Params p,
                     U1State *__restrict__ rec, int64_t row)
 {
-  __shared__ double smem[(256 / 32) * kU1Red];
-  double v[kU1Red];
-  u1_reduce_partials(partials, a.nblocks, v, smem);
-  if (threadIdx.x != 0) return;
+  __shared__ double smem[kU1Red * (kU1TailGroups + 1)];
+  griddep_wait();
+  griddep_launch();
   U1State s = *st;
+  double v[kU1Red] = {};
+  if (a.nblocks > 0) rows_reduce<kU1Red, 8, kU1TailGroups>(partials, a.nblocks, smem, v);
+  if (threadIdx.x >= 32) return;
   u1_tail_apply(s, v, a, p);
-  rec[row] = s;
+  if (threadIdx.x == 0) rec[row] = s;
   if (b.flags) u1_tail_apply(s, v, b, p);
-  *st = s;
+  if (threadIdx.x == 0) *st = s;
 }
 
 // Measurement sums (one sweep): [0] |pi_phi|^2, [1] sum |D phi|^2, [2] sum pi_A^2, [3] B^2, [4] V,
