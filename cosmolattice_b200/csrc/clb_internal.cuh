@@ -221,23 +221,28 @@ __device__ __forceinline__ void u1_offsets(int N, size_t s, long long (&op)[3], 
   }
 }
 
-// Site order of the gauge-model sweeps.
-//   order 0: a grid-stride loop over s = (x N + y) N + z.
-//   order 1 (bricks): the block's threads cover a 32 (z) x blockDim.x/32 (y) tile of one x-plane and
-//     march it along x over runs of kBrickRun planes; the (tile, run) items go to the blocks in turn.
+// Site order of the gauge-model sweeps (the order argument of for_sites).
+//   0: a grid-stride loop over s = (x N + y) N + z.
+//   R > 0 (bricks): the block's threads cover a 32 (z) x blockDim.x/32 (y) tile of one x-plane and
+//     march it along x over runs of R planes; the (tile, run) items go to the blocks in turn.
 //     The plane a thread reads as its x + 1 neighbours is the plane of its next site, so those
 //     values, and the y neighbours inside the tile, are re-read from L1 rather than from L2.
 // Either order visits every site once; the per-site arithmetic is the same, and only the grouping
 // of the volume sums into block partials differs.
-constexpr int kBrickRun = 32;
-// Bricks where they measured faster: lattices of at least 32 sites a side (a smaller one fills
-// too little of a tile) and a sweep that gains from them (bricks = true; at 192^3 the lphi4SU2U1
-// kicks 1.11x FP64 and 1.06x FP32, the FP32 lphi4U1 kick 1.04x, while the FP64 lphi4U1 kick lost
-// 1.22x).  CLB_GAUGE_ORDER=0 or 1 forces the order.
+// Bricks pay where a few planes of the state no longer stay in L2 between a plane's visits (from N of
+// about 160), and cost idle blocks and partial tiles below.  lphi4SU2U1 (us per step, linear / runs
+// of 4 / 16 / 32): 95^3 FP32 414 / 420 / 489 / 799, 80^3 tangent FP64 908 / 1076 / 1290 / 2180,
+// 128^3 FP64 1286 / 1410 / 1476 / 1506, 192^3 FP64 4637 / 4631 / 4481 / 4527.
+// bricks: whether the sweep takes them (the FP64 lphi4U1 site-by-site kick loses at every size).
+// CLB_GAUGE_ORDER overrides: 0 linear, 1 bricks, R > 1 bricks with runs of R planes.
+constexpr int kBrickRun = 16;
 inline int gauge_site_order(int N, bool bricks)
 {
-  if (const char *env = std::getenv("CLB_GAUGE_ORDER")) return std::atoi(env) != 0 ? 1 : 0;
-  return bricks && N >= 32 ? 1 : 0;
+  if (const char *env = std::getenv("CLB_GAUGE_ORDER")) {
+    const int v = std::atoi(env);
+    return v == 1 ? kBrickRun : v < 0 ? 0 : v;
+  }
+  return bricks && N >= 160 ? kBrickRun : 0;
 }
 template <class Fn> __device__ __forceinline__ void for_sites(int N, size_t n3, int order, Fn &&fn)
 {
@@ -247,7 +252,7 @@ template <class Fn> __device__ __forceinline__ void for_sites(int N, size_t n3, 
   }
   const int TY = (int)(blockDim.x >> 5);
   const int tz = (int)(threadIdx.x & 31), ty = (int)(threadIdx.x >> 5);
-  const int ntz = (N + 31) >> 5, nty = (N + TY - 1) / TY, nxr = (N + kBrickRun - 1) / kBrickRun;
+  const int ntz = (N + 31) >> 5, nty = (N + TY - 1) / TY, nxr = (N + order - 1) / order;
   const long long items = (long long)ntz * nty * nxr;
   const size_t plane = (size_t)N * N;
   for (long long it = blockIdx.x; it < items; it += gridDim.x) {
@@ -256,7 +261,7 @@ template <class Fn> __device__ __forceinline__ void for_sites(int N, size_t n3, 
     const int yt = (int)(r % nty), xr = (int)(r / nty);
     const int z = zt * 32 + tz, y = yt * TY + ty;
     if (z >= N || y >= N) continue;
-    const int xa = xr * kBrickRun, xb = min(N, xa + kBrickRun);
+    const int xa = xr * order, xb = min(N, xa + order);
     size_t s = (size_t)xa * plane + (size_t)y * N + z;
     for (int x = xa; x < xb; ++x, s += plane) fn(s);
   }
