@@ -50,7 +50,7 @@ using TD = Tan<double>;
 __device__ __forceinline__ void sincos_t(TD t, TD &s, TD &c)
 {
   double sv, cv;
-  sincos(t.v, &sv, &cv);
+  sincos_link(t.v, &sv, &cv);
   s = TD(sv, cv * t.d);
   c = TD(cv, -sv * t.d);
 }

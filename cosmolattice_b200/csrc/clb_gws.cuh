@@ -117,7 +117,8 @@ __device__ __forceinline__ void gw_gauge_tensor(const R *__restrict__ phr, const
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const R th = A::mul(ndxg, Ax[(size_t)i * n3 + s]);
-    const R ur = cos(th), ui = sin(th);
+    R ur, ui;
+    sincos_link(th, &ui, &ur);
     const R pr = phr[nb[i]], pm = phi[nb[i]];
     const R wr = A::sub(A::mul(ur, pr), A::mul(ui, pm)), wi = A::add(A::mul(ur, pm), A::mul(ui, pr));
     dr[i] = A::sub(wr, fr) / dx;

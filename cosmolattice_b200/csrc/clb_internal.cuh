@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "clb_div.h"
+#include "clb_trig.h"
 
 namespace clb {
 

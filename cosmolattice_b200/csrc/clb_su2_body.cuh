@@ -135,7 +135,9 @@ template <class S, class T> struct Site {
   __device__ __forceinline__ C2<T> phase(T g, int i, size_t t) const
   {
     const T th = (-dx * g) * F(7 + i, t);
-    return C2<T>{cos(th), sin(th)};
+    C2<T> r;
+    sincos_link(th, &r.im, &r.re);
+    return r;
   }
   __device__ __forceinline__ T normD(size_t t) const
   {
@@ -613,13 +615,22 @@ __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_K
 }
 
 // Drifts (velocityverlet.h:181-222; the leapfrog's forms leapfrog.h:203-236 have lf = 1), in FP64
-// and rounded to the storage type once.
-__device__ __forceinline__ Q4<double> qexp(double p1, double p2, double p3)
+// and rounded to the storage type once.  The link step's exponential from n = |p|, as the reference
+// forms it (FP64 storage); rounded to FP32 afterwards it comes from n^2 directly where that is
+// small, without the square root and the division.
+template <class S> __device__ __forceinline__ Q4<double> qexp(double p1, double p2, double p3)
 {
-  const double n = sqrt(p1 * p1 + p2 * p2 + p3 * p3);
+  const double n2 = p1 * p1 + p2 * p2 + p3 * p3;
+  if (sizeof(S) == 4 && n2 <= kSmallPhase * kSmallPhase) {
+    const double sn = __fma_rn(n2, sinc_poly(n2), 1.0);
+    return Q4<double>{__fma_rn(n2, cosm_poly(n2), 1.0), sn * p1, sn * p2, sn * p3};
+  }
+  const double n = sqrt(n2);
   if (n == 0) return Q4<double>{1, 0, 0, 0};
-  const double sn = sin(n) / n;
-  return Q4<double>{cos(n), sn * p1, sn * p2, sn * p3};
+  double s, c;
+  sincos_link(n, &s, &c);
+  const double sn = s / n;
+  return Q4<double>{c, sn * p1, sn * p2, sn * p3};
 }
 // The U(1) link phases of A_i(x) for both couplings, exactly as Site::phase forms them, into the
 // phase arrays the kick reads.
@@ -630,8 +641,10 @@ template <class S> __device__ __forceinline__ void put_phases(S *__restrict__ ph
   for (int which = 0; which < 2; ++which) {
     const S th = (-(S)a.dx * (S)(which == 0 ? a.gC : a.gD)) * A;
     const size_t b = (size_t)(4 * i + 2 * which) * n3 + s;
-    ph[b] = cos(th);
-    ph[b + n3] = sin(th);
+    S c, sn;
+    sincos_link(th, &sn, &c);
+    ph[b] = c;
+    ph[b + n3] = sn;
   }
 }
 template <class S> __global__ void __launch_bounds__(256) k_phases(const S *__restrict__ f, S *__restrict__ ph, Params a)
@@ -664,7 +677,7 @@ __global__ void __launch_bounds__(256)
     }
     for (int i = 0; i < 3; ++i) {
       const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = (size_t)(10 + 4 * i) * n3 + s;
-      const Q4<double> E = qexp(cG * (double)p[pb], cG * (double)p[pb + n3], cG * (double)p[pb + 2 * n3]);
+      const Q4<double> E = qexp<S>(cG * (double)p[pb], cG * (double)p[pb + n3], cG * (double)p[pb + 2 * n3]);
       const Q4<double> U = qmul(E, Q4<double>{(double)f[fb], (double)f[fb + n3], (double)f[fb + 2 * n3], (double)f[fb + 3 * n3]});
       f[fb] = (S)U.w;
       f[fb + n3] = (S)U.x;
@@ -906,22 +919,33 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4 ? CLB_SU2_TAN_MINB_F32 : C
 // exp of an algebra element with its tangent; the value is qexp's.  d(sin n / n)/dn =
 // (n cos n - sin n) / n^2 is taken from its Taylor series below n = 0.1, where the closed form
 // cancels.
-__device__ __forceinline__ Q4<Tan<double>> qexp_tan(Tan<double> p1, Tan<double> p2, Tan<double> p3)
+template <class S> __device__ __forceinline__ Q4<Tan<double>> qexp_tan(Tan<double> p1, Tan<double> p2, Tan<double> p3)
 {
   using T = Tan<double>;
-  const double n = sqrt(p1.v * p1.v + p2.v * p2.v + p3.v * p3.v);
+  const double n2 = p1.v * p1.v + p2.v * p2.v + p3.v * p3.v;
+  if (sizeof(S) == 4 && n2 <= kSmallPhase * kSmallPhase) {
+    // d(sin n / n) = ds n dn and d(cos n) = -(sin n / n) n dn, with n dn = p . dp
+    const double sn = __fma_rn(n2, sinc_poly(n2), 1.0), cn = __fma_rn(n2, cosm_poly(n2), 1.0);
+    const double ndn = (p1.v * p1.d + p2.v * p2.d) + p3.v * p3.d;
+    const double sd = -(1.0 / 3 - n2 * (1.0 / 30 - n2 * (1.0 / 840 - n2 * (1.0 / 45360)))) * ndn;
+    return Q4<T>{T(cn, -sn * ndn), T(sn * p1.v, sd * p1.v + sn * p1.d), T(sn * p2.v, sd * p2.v + sn * p2.d),
+                 T(sn * p3.v, sd * p3.v + sn * p3.d)};
+  }
+  const double n = sqrt(n2);
   if (n == 0) return Q4<T>{T(1.0), T(0.0, p1.d), T(0.0, p2.d), T(0.0, p3.d)};
-  const double sn = sin(n) / n, cn = cos(n);
+  double s1, cn;
+  sincos_link(n, &s1, &cn);
+  const double sn = s1 / n;
   const double dn = ((p1.v * p1.d + p2.v * p2.d) + p3.v * p3.d) / n;
   double ds;
   if (n < 0.1) {
     const double x = n * n;
     ds = -n * (1.0 / 3 - x * (1.0 / 30 - x * (1.0 / 840 - x / 45360)));
   } else {
-    ds = (n * cn - sin(n)) / (n * n);
+    ds = (n * cn - s1) / (n * n);
   }
   const double sd = ds * dn;
-  return Q4<T>{T(cn, -sin(n) * dn), T(sn * p1.v, sd * p1.v + sn * p1.d), T(sn * p2.v, sd * p2.v + sn * p2.d),
+  return Q4<T>{T(cn, -s1 * dn), T(sn * p1.v, sd * p1.v + sn * p1.d), T(sn * p2.v, sd * p2.v + sn * p2.d),
                T(sn * p3.v, sd * p3.v + sn * p3.d)};
 }
 
@@ -955,7 +979,7 @@ __global__ void __launch_bounds__(256)
       put(f, df, (7 + i) * n3 + s, ld(f, df, (7 + i) * n3 + s) + cA * ld(p, dp, (7 + i) * n3 + s) * 1.0);
     for (int i = 0; i < 3; ++i) {
       const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = (size_t)(10 + 4 * i) * n3 + s;
-      const Q4<T> E = qexp_tan(cG * ld(p, dp, pb), cG * ld(p, dp, pb + n3), cG * ld(p, dp, pb + 2 * n3));
+      const Q4<T> E = qexp_tan<S>(cG * ld(p, dp, pb), cG * ld(p, dp, pb + n3), cG * ld(p, dp, pb + 2 * n3));
       const Q4<T> U = qmul(E, Q4<T>{ld(f, df, fb), ld(f, df, fb + n3), ld(f, df, fb + 2 * n3), ld(f, df, fb + 3 * n3)});
       put(f, df, fb, U.w);
       put(f, df, fb + n3, U.x);

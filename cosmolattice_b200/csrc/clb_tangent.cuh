@@ -109,6 +109,14 @@ template <class T> __host__ __device__ __forceinline__ Tan<T> cos(Tan<T> a)
 {
   return Tan<T>(::cos(a.v), -::sin(a.v) * a.d);
 }
+// sine and cosine of a link phase, the value part as the plain forms take it
+template <class T> __device__ __forceinline__ void sincos_link(Tan<T> a, Tan<T> *s, Tan<T> *c)
+{
+  T sv, cv;
+  sincos_link(a.v, &sv, &cv);
+  *s = Tan<T>(sv, cv * a.d);
+  *c = Tan<T>(cv, -sv * a.d);
+}
 template <class T> __host__ __device__ __forceinline__ Tan<T> pow(Tan<T> a, typename Id<T>::type e)
 {
   return Tan<T>(::pow(a.v, e), e * ::pow(a.v, e - 1) * a.d);

@@ -72,8 +72,8 @@ __device__ __forceinline__ float u1_m(float a, float b) { return a * b; }
 __device__ __forceinline__ float u1_a(float a, float b) { return a + b; }
 __device__ __forceinline__ float u1_s(float a, float b) { return a - b; }
 __device__ __forceinline__ float u1_d(float a, float b) { return a * (1.0f / b); }
-__device__ __forceinline__ void u1_sincos(double x, double *sn, double *cs) { sincos(x, sn, cs); }
-__device__ __forceinline__ void u1_sincos(float x, float *sn, float *cs) { sincosf(x, sn, cs); }
+__device__ __forceinline__ void u1_sincos(double x, double *sn, double *cs) { sincos_link(x, sn, cs); }
+__device__ __forceinline__ void u1_sincos(float x, float *sn, float *cs) { sincos_link(x, sn, cs); }
 
 // FP64 arithmetic of the adjoint's segment recompute, which is not bound to the reference's
 // rounding order: products and sums may contract into FMAs, and a division becomes a multiply by
@@ -91,7 +91,7 @@ __device__ __forceinline__ FD u1_d(FD a, FD b) { return FD(a.v * (1.0 / b.v)); }
 __device__ __forceinline__ FD operator-(FD a) { return FD(-a.v); }
 __device__ __forceinline__ FD sqrt(FD a) { return FD(::sqrt(a.v)); }
 __device__ __forceinline__ FD div_by(FD a, const DivBy &d) { return FD(a.v * d.rh); }
-__device__ __forceinline__ void u1_sincos(FD x, FD *sn, FD *cs) { sincos(x.v, &sn->v, &cs->v); }
+__device__ __forceinline__ void u1_sincos(FD x, FD *sn, FD *cs) { sincos_link(x.v, &sn->v, &cs->v); }
 
 // Per-site kernel values in arithmetic type T.  Fields f (storage S): [Re phi, Im phi, A_x, A_y,
 // A_z] x n3.  The FP64 form (S = T = double) pins every rounding; the FP32 form computes in float.
