@@ -80,6 +80,7 @@ const double *su2_component(clb_handle *h, int which, int comp, bool *gauge);
 // gravitational waves of the scalar singlets (clb_gws.cu)
 void gw_kick_step(clb_handle *h);
 void gw_drift(clb_handle *h);
+void gw_between_steps(clb_handle *h, bool more);
 void gw_sync(clb_handle *h);
 void gw_set_synced(clb_handle *h, bool s);
 void gw_destroy(clb_handle *h);
@@ -380,8 +381,7 @@ template <class R, int NS> struct EvolveVV {
         const double wn = more ? wof((size_t)((k + 1) % (int64_t)S)) : 0.0;
         fb_tail(h, T_FB_AIM | T_FB_AI, h->fb_a(tc + w * dt));
         L::fused(h, dt * w, w * dt / 2, more ? wn * dt / 2 : 0.0, false);
-        if (h->gw && i + 1 == S) gw_drift(h);
-        if (h->gw && i + 1 == S && more) gw_kick_step(h);
+        if (h->gw && i + 1 == S) gw_between_steps(h, more);
         tc += dt * w;
         if (i + 1 == S) {
           h->fb_t += dt;
@@ -425,8 +425,7 @@ template <class R, int NS> struct EvolveVV {
       const bool more = k + 1 < total;
       const double wn = more ? wof((size_t)((k + 1) % (int64_t)S)) : 0.0;
       L::fused(h, dt * w, w * dt / 2, more ? wn * dt / 2 : 0.0, ex);
-      if (h->gw && i + 1 == S) gw_drift(h);
-      if (h->gw && i + 1 == S && more) gw_kick_step(h); // a_I of the step's end, before the tail drifts a
+      if (h->gw && i + 1 == S) gw_between_steps(h, more); // a_I of the step's end, before the tail drifts a
       if (ex) {
         uint32_t fl = T_STORE_PI2_I | T_STORE_FIELDS | T_VV_KICK_ONE;
         if (more) fl |= T_VV_KICK_HALF | T_VV_DRIFT;
@@ -551,10 +550,7 @@ template <class R, int NS> struct EvolvePV {
         }
         if (last) {
           L::drift_fields(h, dt / 2 * w, ex);
-          if (h->gw) {
-            gw_drift(h);
-            if (s + 1 < nsteps) gw_kick_step(h);
-          }
+          if (h->gw) gw_between_steps(h, s + 1 < nsteps);
           if (ex) tail(h, T_PV_MODE | T_STORE_FIELDS | (s + 1 < nsteps ? T_PV_DRIFT_A1 : 0u), h->sweep_blocks, 0, w0, s);
         }
       }
@@ -594,10 +590,7 @@ template <class R, int NS> struct EvolveLF {
       for (int64_t s = 1; s < nsteps; ++s) {
         h->fb_t += dt;
         L::fused(h, dt, dt, 0.0, false);
-        if (h->gw) {
-          gw_drift(h);
-          gw_kick_step(h);
-        }
+        if (h->gw) gw_between_steps(h, true);
         a_drift();
       }
       L::drift_fields(h, dt, false);
@@ -628,10 +621,7 @@ template <class R, int NS> struct EvolveLF {
     if (ex) tail(h, T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, L::reduce_pi2(h));
     for (int64_t s = 1; s < nsteps; ++s) {
       L::fused(h, dt, dt, 0.0, ex);
-      if (h->gw) {
-        gw_drift(h);
-        gw_kick_step(h);
-      }
+      if (h->gw) gw_between_steps(h, true);
       if (ex)
         tail(h, T_STORE_FIELDS | T_HIST_EARLY | T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, h->sweep_blocks, 0, 0, s - 1);
     }

@@ -35,6 +35,7 @@
 #include "clb_vv.h"
 
 #include <cmath>
+#include <type_traits>
 #include <string>
 #include <vector>
 
@@ -47,7 +48,7 @@ constexpr int kGWSpecBlocks = 148 * 2;
 template <class R, int NS> struct ScalarGWSource {
   const R *fld;
   Pad pd;
-  R dx;
+  DivBy ddx;
   __device__ __forceinline__ void operator()(size_t, int x, int y, int z, int xp, int yp, int zp, R (&P)[6]) const
   {
     using A = Ar<R>;
@@ -55,8 +56,8 @@ template <class R, int NS> struct ScalarGWSource {
     for (int f = 0; f < NS; ++f) {
       const R *F = fld + (size_t)f * pd.comp;
       const R c = F[pd.at(x, y, z)];
-      const R g0 = A::sub(F[pd.at(xp, y, z)], c) / dx, g1 = A::sub(F[pd.at(x, yp, z)], c) / dx,
-              g2 = A::sub(F[pd.at(x, y, zp)], c) / dx;
+      const R g0 = gw_div(A::sub(F[pd.at(xp, y, z)], c), ddx), g1 = gw_div(A::sub(F[pd.at(x, yp, z)], c), ddx),
+              g2 = gw_div(A::sub(F[pd.at(x, y, zp)], c), ddx);
       const R t[6] = {A::mul(g0, g0), A::mul(g0, g1), A::mul(g0, g2), A::mul(g1, g1), A::mul(g1, g2), A::mul(g2, g2)};
 #pragma unroll
       for (int k = 0; k < 6; ++k) P[k] = f == 0 ? t[k] : A::add(P[k], t[k]);
@@ -181,33 +182,33 @@ bool gw_ok(const clb_handle *h) { return h->gw != nullptr; }
 namespace clb {
 
 // The gauge models' GW kick and drift (clb_u1.cu, clb_su2.cu).
-void u1_gw_kick(clb_handle *h, double w);
+void u1_gw_kick(clb_handle *h, double w, bool drift);
 void u1_gw_drift(clb_handle *h);
-void su2_gw_kick(clb_handle *h, double w);
+void su2_gw_kick(clb_handle *h, double w, bool drift);
 void su2_gw_drift(clb_handle *h);
 bool su2_tangent_active(const clb_handle *h);
 
-// Runs one GW kick (weight w of dt) at the handle's current fields and a_I.
-__attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w)
+// Runs one GW kick (weight w of dt) at the handle's current fields and a_I, with drift after the drift
+// of the step just taken in the same sweep.
+__attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w, bool drift)
 {
   GWSector *g = h->gw;
   g->synced = false;
-  if (h->u1) return u1_gw_kick(h, w);
-  if (h->su2) return su2_gw_kick(h, w);
-  const double inv_dx2 = 1.0 / (h->cfg.dx * h->cfg.dx);
-  const double hd = w * h->cfg.dt;
-#define CLB_GWK(R, NS)                                                                                                 \
-  CLB_LAUNCH(h, K_GW, (k_gw_kick<R, ScalarGWSource<R, NS>><<<kGWBlocks, 256, 0, h->stream>>>(                        \
-                          static_cast<const R *>(g->u), static_cast<R *>(g->pi), h->N, inv_dx2, hd, &h->d_st->kick_A, \
-                          ScalarGWSource<R, NS>{static_cast<const R *>(h->fld[h->cf]), h->pd, (R)h->cfg.dx})))
-  if (h->fp32) {
-    if (h->NS == 1) CLB_GWK(float, 1);
-    else CLB_GWK(float, 2);
-  } else {
-    if (h->NS == 1) CLB_GWK(double, 1);
-    else CLB_GWK(double, 2);
-  }
-#undef CLB_GWK
+  if (h->u1) return u1_gw_kick(h, w, drift);
+  if (h->su2) return su2_gw_kick(h, w, drift);
+  auto go = [&](auto zero, auto ns) {
+    using R = decltype(zero);
+    using Src = ScalarGWSource<R, decltype(ns)::value>;
+    const Src src{static_cast<const R *>(h->fld[h->cf]), h->pd, make_div(h->cfg.dx, (float)h->cfg.dx)};
+    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, Src>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &h->d_st->kick_A, &h->d_st->drift_p,
+                                                &h->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
+  };
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  if (h->fp32)
+    h->NS == 1 ? go(0.0f, One{}) : go(0.0f, Two{});
+  else
+    h->NS == 1 ? go(0.0, One{}) : go(0.0, Two{});
 }
 
 // Runs one GW drift with the a_SI of the matter step just taken.
@@ -229,12 +230,21 @@ __attribute__((visibility("hidden"))) void gw_drift(clb_handle *h)
 }
 
 // The GW kick before a matter step (evolver.h:104-107): half a step after a sync, else a whole one.
-__attribute__((visibility("hidden"))) void gw_kick_step(clb_handle *h) { gw_kick(h, h->gw->synced ? 0.5 : 1.0); }
+__attribute__((visibility("hidden"))) void gw_kick_step(clb_handle *h) { gw_kick(h, h->gw->synced ? 0.5 : 1.0, false); }
+
+// The GW drift after a matter step and, with more to come in the call, the next step's GW kick: nothing
+// that either reads changes in between.
+__attribute__((visibility("hidden"))) void gw_between_steps(clb_handle *h, bool more)
+{
+  if (more && h->gw->u2) return gw_kick(h, 1.0, true);
+  gw_drift(h);
+  if (more) gw_kick_step(h);
+}
 
 // Evolver::sync (evolver.h:132-138): the half kick to integer time, if the momenta are unsynced.
 __attribute__((visibility("hidden"))) void gw_sync(clb_handle *h)
 {
-  if (!h->gw->synced) gw_kick(h, 0.5);
+  if (!h->gw->synced) gw_kick(h, 0.5, false);
   h->gw->synced = true;
 }
 
@@ -243,8 +253,8 @@ __attribute__((visibility("hidden"))) void gw_set_synced(clb_handle *h, bool s) 
 __attribute__((visibility("hidden"))) void gw_destroy(clb_handle *h)
 {
   if (!h->gw) return;
-  if (h->gw->u) cudaFree(h->gw->u);
-  if (h->gw->pi) cudaFree(h->gw->pi);
+  for (void *p : {h->gw->u, h->gw->pi, h->gw->u2, h->gw->pi2})
+    if (p) cudaFree(p);
   if (h->gw->d_fk) cudaFree(h->gw->d_fk);
   delete h->gw;
   h->gw = nullptr;
@@ -274,6 +284,12 @@ int clb_gws_enable(clb_handle *h)
   if (e != cudaSuccess) {
     gw_destroy(h);
     return h->fail(CLB_ENOMEM, std::string("clb_gws_enable: ") + cudaGetErrorString(e));
+  }
+  // without room for the second pair the drift and the kick run as two sweeps
+  if (cudaMalloc(&g->u2, bytes) != cudaSuccess || cudaMalloc(&g->pi2, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    if (g->u2) cudaFree(g->u2);
+    g->u2 = g->pi2 = nullptr;
   }
   return CLB_OK;
 }

@@ -27,7 +27,8 @@ template <class R> struct SU2GWSource {
   const R *f, *p;
   size_t n3;
   int N;
-  R dx, ndxg, rfo2;
+  DivBy ddx;
+  R ndxg, rfo2;
   const double *aI;
   __device__ __forceinline__ void operator()(size_t s, int x, int y, int z, int xp, int yp, int zp, R (&P)[6]) const
   {
@@ -36,10 +37,10 @@ template <class R> struct SU2GWSource {
     const R c = f[s];
     R g[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) g[i] = A::sub(f[nb[i]], c) / dx;
+    for (int i = 0; i < 3; ++i) g[i] = gw_div(A::sub(f[nb[i]], c), ddx);
 #pragma unroll
     for (int k = 0; k < 6; ++k) P[k] = A::mul(g[gw_pair_i(k)], g[gw_pair_j(k)]);
-    gw_gauge_tensor<R>(f + n3, f + 2 * n3, f + 7 * n3, p + 7 * n3, n3, nb, s, dx, ndxg, (R)*aI, rfo2, false, P);
+    gw_gauge_tensor<R>(f + n3, f + 2 * n3, f + 7 * n3, p + 7 * n3, n3, nb, s, ddx, ndxg, (R)*aI, rfo2, false, P);
   }
 };
 } // namespace
@@ -369,25 +370,24 @@ __attribute__((visibility("hidden"))) int su2_initialize(clb_handle *h, int32_t 
 }
 
 void gw_kick_step(clb_handle *h);
-void gw_drift(clb_handle *h);
+void gw_between_steps(clb_handle *h, bool more);
 void gw_sync(clb_handle *h);
 
 __attribute__((visibility("hidden"))) bool su2_tangent_active(const clb_handle *h) { return h->su2->tangent; }
 
 // The GW kick (weight w of dt) with the lphi4SU2U1 source, at the current fields, momenta and a_I.
-__attribute__((visibility("hidden"))) void su2_gw_kick(clb_handle *h, double w)
+__attribute__((visibility("hidden"))) void su2_gw_kick(clb_handle *h, double w, bool drift)
 {
   SU2Sector *u = h->su2;
   GWSector *g = h->gw;
   const double r = h->md.fStar / h->md.omegaStar; // pow<2>(fStar / omegaStar)
-  const double inv_dx2 = 1.0 / (h->cfg.dx * h->cfg.dx), hd = w * h->cfg.dt;
   const double ndxg = -u->prm.dx * u->prm.gC;     // the phase of Site::phaseC
   auto go = [&](auto zero) {
     using R = decltype(zero);
-    const SU2GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, (R)h->cfg.dx,
+    const SU2GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, u->prm.ddx,
                              (R)ndxg, (R)(r * r), &u->d_st->aI};
-    CLB_LAUNCH(h, K_GW, (k_gw_kick<R, SU2GWSource<R>><<<kGWBlocks, 256, 0, h->stream>>>(
-                            static_cast<const R *>(g->u), static_cast<R *>(g->pi), h->N, inv_dx2, hd, &u->d_st->kA, src)));
+    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, SU2GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &u->d_st->kA, &u->d_st->p3,
+                                                        &u->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
   };
   if (u->fp32) go(0.0f);
   else go(0.0);
@@ -456,12 +456,12 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
     auto wof = [&](size_t i) { return ws[i < P ? i : S - i - 1]; };
     if (h->cfg.evolver == CLB_LF) {
       for (int64_t s = 0; s < nsteps; ++s) {
-        if (h->gw) gw_kick_step(h); // evolver.h:102-124, as in the self-consistent leapfrog
+        if (h->gw && s == 0) gw_kick_step(h); // evolver.h:102-124, as in the self-consistent leapfrog
         sweep(h, 1, false, false, lf_kick(dt, h->synced ? 0.5 : 1.0));
         const double tm = h->fb_t - t0;
         tail(h, T_FB_AIM | T_FB_AI | T_FB_ASI, false, 0, 0, -1, h->fb_a(tm + dt), h->fb_a(tm + dt / 2.0));
         drift(h, 1.0, true);
-        if (h->gw) gw_drift(h);
+        if (h->gw) gw_between_steps(h, s + 1 < nsteps);
         step_done(h);
         h->fb_t += dt;
         h->synced = false;
@@ -469,7 +469,7 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
     } else if (is_pv(h->cfg.evolver)) {
       tail(h, T_PV_MODE, false);
       for (int64_t s = 0; s < nsteps; ++s) {
-        if (h->gw) gw_kick_step(h); // evolver.h:102-124
+        if (h->gw && s == 0) gw_kick_step(h); // evolver.h:102-124
         double tc = h->fb_t - t0;
         for (size_t i = 0; i < S; ++i) {
           const double w = wof(i);
@@ -480,7 +480,7 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
           drift(h, w, false, dt / 2);
           tc += dt * w;
         }
-        if (h->gw) gw_drift(h);
+        if (h->gw) gw_between_steps(h, s + 1 < nsteps);
         step_done(h);
         h->fb_t += dt;
       }
@@ -507,10 +507,10 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
       };
       if (h->gw) {
         // one step at a time, as in the self-consistent VV with GWs
+        gw_kick_step(h);
         for (int64_t s = 0; s < nsteps; ++s) {
-          gw_kick_step(h);
           vv_fb(1);
-          gw_drift(h);
+          gw_between_steps(h, s + 1 < nsteps);
         }
       } else {
         vv_fb(nsteps);
@@ -524,10 +524,9 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
     if (ex) tail(h, T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, true);
     for (int64_t s = 0; s < nsteps; ++s) {
       drift(h, 1.0, true);
-      if (h->gw) gw_drift(h);
+      if (h->gw) gw_between_steps(h, s + 1 < nsteps);
       step_done(h);
       if (s + 1 < nsteps) {
-        if (h->gw) gw_kick_step(h);
         sweep(h, 1, ex, ex, lf_kick(dt, 1.0));
         if (ex) tail(h, T_STORE_FIELDS | T_HIST_EARLY | T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, true, 0, 0, s);
       } else if (ex) {
@@ -560,8 +559,7 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
                true, w, last ? 0.0 : wof(i + 1));
         drift(h, w, false, dt / 2);
         if (last && h->gw) {
-          gw_drift(h);
-          if (s + 1 < nsteps) gw_kick_step(h);
+          gw_between_steps(h, s + 1 < nsteps);
         }
         if (last) {
           step_done(h);
@@ -575,10 +573,10 @@ __attribute__((visibility("hidden"))) int su2_evolve(clb_handle *h, int64_t nste
     // the GW leapfrog around each matter step (evolver.h:102-124): its kick reads the gauge
     // momenta at integer time, which the merged sweep between two steps never stores, so the steps
     // run one by one (the schedule of one-step clb_evolve calls)
+    gw_kick_step(h);
     for (int64_t s = 0; s < nsteps; ++s) {
-      gw_kick_step(h);
       vv_steps(h, 1, s);
-      gw_drift(h);
+      gw_between_steps(h, s + 1 < nsteps);
     }
   } else {
     vv_steps(h, nsteps, 0);

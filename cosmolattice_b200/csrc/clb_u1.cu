@@ -30,12 +30,13 @@ template <class R> struct U1GWSource {
   const R *f, *p;
   size_t n3;
   int N;
-  R dx, ndxg, rfo2;
+  DivBy ddx;
+  R ndxg, rfo2;
   const double *aI;
   __device__ __forceinline__ void operator()(size_t s, int x, int y, int z, int xp, int yp, int zp, R (&P)[6]) const
   {
     const size_t nb[3] = {((size_t)xp * N + y) * N + z, ((size_t)x * N + yp) * N + z, ((size_t)x * N + y) * N + zp};
-    gw_gauge_tensor<R>(f, f + n3, f + 2 * n3, p + 2 * n3, n3, nb, s, dx, ndxg, (R)*aI, rfo2, true, P);
+    gw_gauge_tensor<R>(f, f + n3, f + 2 * n3, p + 2 * n3, n3, nb, s, ddx, ndxg, (R)*aI, rfo2, true, P);
   }
 };
 } // namespace
@@ -358,22 +359,21 @@ int check(clb_handle *h, const char *where)
 } // namespace
 
 void gw_kick_step(clb_handle *h);
-void gw_drift(clb_handle *h);
+void gw_between_steps(clb_handle *h, bool more);
 void gw_sync(clb_handle *h);
 
 // The GW kick (weight w of dt) with the lphi4U1 source, at the current fields, momenta and a_I.
-__attribute__((visibility("hidden"))) void u1_gw_kick(clb_handle *h, double w)
+__attribute__((visibility("hidden"))) void u1_gw_kick(clb_handle *h, double w, bool drift)
 {
   U1Sector *u = h->u1;
   GWSector *g = h->gw;
   const double r = h->md.fStar / h->md.omegaStar; // pow<2>(fStar / omegaStar)
-  const double inv_dx2 = 1.0 / (h->cfg.dx * h->cfg.dx), hd = w * h->cfg.dt;
   auto go = [&](auto zero) {
     using R = decltype(zero);
-    const U1GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, (R)h->cfg.dx,
+    const U1GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, u->prm.ddx,
                             (R)u->prm.ndxg, (R)(r * r), &u->d_st->aI};
-    CLB_LAUNCH(h, K_GW, (k_gw_kick<R, U1GWSource<R>><<<kGWBlocks, 256, 0, h->stream>>>(
-                            static_cast<const R *>(g->u), static_cast<R *>(g->pi), h->N, inv_dx2, hd, &u->d_st->kA, src)));
+    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, U1GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &u->d_st->kA, &u->d_st->cs_drift,
+                                                        &u->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
   };
   if (u->fp32) go(0.0f);
   else go(0.0);
@@ -572,19 +572,19 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
     auto wof = [&](size_t i) { return ws[i < P ? i : S - i - 1]; };
     if (h->cfg.evolver == CLB_LF) {
       for (int64_t s = 0; s < nsteps; ++s) {
-        if (h->gw) gw_kick_step(h); // evolver.h:102-124, as in the self-consistent leapfrog
+        if (h->gw && s == 0) gw_kick_step(h); // evolver.h:102-124, as in the self-consistent leapfrog
         kick_sweep(h, 1, false, false, lf_kick(dt, h->synced ? 0.5 : 1.0));
         const double tm = h->fb_t - t0;
         tail(h, T_FB_AIM | T_FB_AI | T_FB_ASI, false, 0, 0, -1, h->fb_a(tm + dt), h->fb_a(tm + dt / 2.0));
         drift(h, 1.0);
-        if (h->gw) gw_drift(h);
+        if (h->gw) gw_between_steps(h, s + 1 < nsteps);
         h->fb_t += dt;
         h->synced = false;
       }
     } else if (is_pv(h->cfg.evolver)) {
       tail(h, T_PV_MODE, false);
       for (int64_t s = 0; s < nsteps; ++s) {
-        if (h->gw) gw_kick_step(h); // evolver.h:102-124
+        if (h->gw && s == 0) gw_kick_step(h); // evolver.h:102-124
         double tc = h->fb_t - t0;
         for (size_t i = 0; i < S; ++i) {
           const double w = wof(i);
@@ -595,7 +595,7 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
           drift(h, w, dt / 2);
           tc += dt * w;
         }
-        if (h->gw) gw_drift(h);
+        if (h->gw) gw_between_steps(h, s + 1 < nsteps);
         h->fb_t += dt;
       }
     } else {
@@ -620,10 +620,10 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
       };
       if (h->gw) {
         // one step at a time, as in the self-consistent VV with GWs
+        gw_kick_step(h);
         for (int64_t s = 0; s < nsteps; ++s) {
-          gw_kick_step(h);
           vv_fb(1);
-          gw_drift(h);
+          gw_between_steps(h, s + 1 < nsteps);
         }
       } else {
         vv_fb(nsteps);
@@ -639,9 +639,8 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
     if (ex) tail(h, T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, true);
     for (int64_t s = 0; s < nsteps; ++s) {
       drift(h, 1.0);
-      if (h->gw) gw_drift(h);
+      if (h->gw) gw_between_steps(h, s + 1 < nsteps);
       if (s + 1 < nsteps) {
-        if (h->gw) gw_kick_step(h);
         kick_sweep(h, 1, ex, ex, lf_kick(dt, 1.0));
         if (ex) tail(h, T_STORE_FIELDS | T_HIST_EARLY | T_STORE_PI2_LF | T_LF_KICK | T_LF_DRIFT, true, 0, 0, s);
       } else {
@@ -678,8 +677,7 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
                true, w, last ? 0.0 : wof(i + 1));
         drift(h, w, dt / 2);
         if (last && h->gw) {
-          gw_drift(h);
-          if (s + 1 < nsteps) gw_kick_step(h);
+          gw_between_steps(h, s + 1 < nsteps);
         }
         if (last && ex) {
           kick_sweep(h, 0, true, false, U1Kick{});
@@ -690,10 +688,10 @@ __attribute__((visibility("hidden"))) int u1_evolve(clb_handle *h, int64_t nstep
     // the GW leapfrog around each matter step (evolver.h:102-124): its kick reads the gauge
     // momenta at integer time, which the merged sweep between two steps never stores, so the steps
     // run one by one (the schedule of one-step clb_evolve calls)
+    gw_kick_step(h);
     for (int64_t s = 0; s < nsteps; ++s) {
-      gw_kick_step(h);
       vv_run(h, 1, nullptr, true, s);
-      gw_drift(h);
+      gw_between_steps(h, s + 1 < nsteps);
     }
   } else {
     vv_run(h, nsteps, nullptr);
