@@ -72,7 +72,7 @@ int su2_tangent_get_state(clb_handle *h, double *fields_dot, double *momenta_dot
 int su2_tangent_observable(clb_handle *h, const double *w, int32_t nw, double *obs, double *dobs);
 int su2_tangent_end(clb_handle *h);
 int su2_tangent_energies(clb_handle *h, double *E, double *dE);
-const void *su2_tangent_component(clb_handle *h, int which, int comp, bool *f32, double *aI, double *daI);
+const double *su2_tangent_component(clb_handle *h, int which, int comp, double *aI, double *daI);
 
 const double *u1_component(clb_handle *h, int which, int comp, bool *gauge);
 const double *su2_component(clb_handle *h, int which, int comp, bool *gauge);
@@ -1502,10 +1502,9 @@ int clb_tangent_spectrum(clb_handle *h, int32_t which, int32_t comp, int32_t ps_
   if (!h) return CLB_EINVAL;
   if (!h->su2) return h->fail(CLB_EUNSUPPORTED, "clb_tangent_spectrum: the tangent-linear form covers lphi4SU2U1");
   if (!d_value_out) return h->fail(CLB_EINVAL, "clb_tangent_spectrum: null output");
-  bool f32 = false;
   double aI = 1, daI = 0;
-  const void *tsrc = nullptr;
-  if (which == 0 || which == 1) tsrc = su2_tangent_component(h, which, comp, &f32, &aI, &daI);
+  const double *tsrc = nullptr;
+  if (which == 0 || which == 1) tsrc = su2_tangent_component(h, which, comp, &aI, &daI);
   if (!tsrc && (which == 0 || which == 1) && comp >= 0 && comp < (which == 0 ? 22 : 19))
     return h->fail(CLB_ESTATE, "clb_tangent_spectrum: call clb_tangent_begin first");
   std::vector<double> sums;
@@ -1520,10 +1519,7 @@ int clb_tangent_spectrum(clb_handle *h, int32_t which, int32_t comp, int32_t ps_
   cudaError_t e = cudaSuccess;
   if (!h->d_spec2 && (e = cudaMalloc(&h->d_spec2, spec_n * sizeof(double))) != cudaSuccess)
     return h->fail(CLB_ENOMEM, std::string("clb_tangent_spectrum: ") + cudaGetErrorString(e));
-  if (f32)
-    CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<float><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const float *>(tsrc), h->d_spec2, N));
-  else
-    CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<double><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const double *>(tsrc), h->d_spec2, N));
+  CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<double><<<kElemBlocks, 256, 0, h->stream>>>(tsrc, h->d_spec2, N));
   if (cufftExecD2Z(h->plan, h->d_spec2, reinterpret_cast<cufftDoubleComplex *>(h->d_spec2)) != CUFFT_SUCCESS)
     return h->fail(CLB_ECUDA, "clb_tangent_spectrum: cufftExecD2Z failed");
   const size_t smem = (size_t)nbins * sizeof(double);

@@ -21,7 +21,7 @@ namespace clb {
 
 namespace {
 // PITensor.h's GW source for lphi4SU2U1: the singlet S (component 0), the complex scalar phi
-// (1, 2) and the U(1) field (7..9, momenta 7..9), in the order scalarSinglet + complexScalar +
+// (1, 2) and the U(1) field (7..9, the arrays 3..5; momenta 7..9), in the order scalarSinglet + complexScalar +
 // electricU1 + magneticU1; the doublet and the SU(2) field source none.
 template <class R> struct SU2GWSource {
   const R *f, *p;
@@ -40,7 +40,7 @@ template <class R> struct SU2GWSource {
     for (int i = 0; i < 3; ++i) g[i] = gw_div(A::sub(f[nb[i]], c), ddx);
 #pragma unroll
     for (int k = 0; k < 6; ++k) P[k] = A::mul(g[gw_pair_i(k)], g[gw_pair_j(k)]);
-    gw_gauge_tensor<R>(f + n3, f + 2 * n3, f + 7 * n3, p + 7 * n3, n3, nb, s, ddx, ndxg, (R)*aI, rfo2, false, P);
+    gw_gauge_tensor<R>(f + n3, f + 2 * n3, f + 3 * n3, p + 7 * n3, n3, nb, s, ddx, ndxg, (R)*aI, rfo2, false, P);
   }
 };
 } // namespace
@@ -78,6 +78,8 @@ Params su2_params(const clb_handle *h)
   a.dt = c.dt;
   a.inv_n3 = 1.0 / (double)h->n3;
   a.order = gauge_site_order(c.N, true);
+  a.divN = make_fast_div((uint32_t)c.N);
+  field_offsets(a.n3, a.oD, a.oU);
   return a;
 }
 
@@ -169,9 +171,9 @@ void step_done(clb_handle *h)
   u->steps_since_unitarize = 0;
   if (u->tangent)
     CLB_LAUNCH(h, K_U1_DRIFT, k_unitarize_tan<float><<<kSU2Blocks, 256, 0, h->stream>>>(
-                                  static_cast<float *>(u->f), static_cast<float *>(u->df), h->n3));
+                                  static_cast<float *>(u->f), static_cast<float *>(u->df), u->prm));
   else
-    CLB_LAUNCH(h, K_U1_DRIFT, k_unitarize<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<float *>(u->f), h->n3));
+    CLB_LAUNCH(h, K_U1_DRIFT, k_unitarize<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<float *>(u->f), u->prm));
 }
 
 void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 = 0, int64_t hist_row = -1,
@@ -236,12 +238,14 @@ __attribute__((visibility("hidden"))) int su2_create(clb_handle *h)
     u->tan_split = u->split;
   }
   bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
-  ok = ok && cudaMalloc(&u->f, NF * h->n3 * u->esz) == cudaSuccess;
+  size_t oD, oU;
+  u->nf = field_offsets(h->n3, oD, oU);
+  ok = ok && cudaMalloc(&u->f, u->nf * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->p, NP * h->n3 * u->esz) == cudaSuccess;
-  ok = ok && cudaMemset(u->f, 0, NF * h->n3 * u->esz) == cudaSuccess;
+  ok = ok && cudaMemset(u->f, 0, u->nf * u->esz) == cudaSuccess;
   ok = ok && cudaMemset(u->p, 0, NP * h->n3 * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->ph, 12 * h->n3 * u->esz) == cudaSuccess;
-  if (u->fp32) ok = ok && cudaMalloc(&u->d_stage, h->n3 * sizeof(double)) == cudaSuccess;
+  ok = ok && cudaMalloc(&u->d_stage, h->n3 * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_st, sizeof(State)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_part, (size_t)kSU2Blocks * kMeas * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_sums, kMeas * sizeof(double)) == cudaSuccess;
@@ -277,25 +281,64 @@ __attribute__((visibility("hidden"))) void su2_destroy(clb_handle *h)
   h->su2 = nullptr;
 }
 
+namespace {
+// Component c of a field (fidx) or momentum buffer: its first element and the distance to the next.
+template <class S> S *comp_at(const clb_handle *h, void *buf, bool field, int c, int &stride)
+{
+  stride = field && ((c >= 3 && c < 7) || c >= 10) ? 4 : 1;
+  return static_cast<S *>(buf) + (field ? fidx(h->su2->prm, c, 0) : (size_t)c * h->n3);
+}
+// The component from / to an FP64 array on the host or the device, through the staging buffer where
+// the device holds it in FP32 or among others; ordered on the handle's stream.
+cudaError_t set_comp(clb_handle *h, void *buf, bool field, int c, const double *src)
+{
+  SU2Sector *u = h->su2;
+  int st;
+  const size_t bytes = h->n3 * sizeof(double);
+  if (!u->fp32) {
+    double *dst = comp_at<double>(h, buf, field, c, st);
+    if (st == 1) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, h->stream);
+    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src, bytes, cudaMemcpyDefault, h->stream);
+    if (e != cudaSuccess) return e;
+    k_comp_set<double><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, dst, st, h->n3);
+  } else {
+    float *dst = comp_at<float>(h, buf, field, c, st);
+    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src, bytes, cudaMemcpyDefault, h->stream);
+    if (e != cudaSuccess) return e;
+    k_comp_set<float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, dst, st, h->n3);
+  }
+  return cudaGetLastError();
+}
+// The component in FP64 as one array: its own place on the device or tmp (N^3).
+const double *flat_comp(clb_handle *h, void *buf, bool field, int c, double *tmp)
+{
+  int st;
+  if (!h->su2->fp32) {
+    const double *src = comp_at<double>(h, buf, field, c, st);
+    if (st == 1) return src;
+    k_comp_get<double><<<kSU2Blocks, 256, 0, h->stream>>>(src, st, tmp, h->n3);
+  } else {
+    const float *src = comp_at<float>(h, buf, field, c, st);
+    k_comp_get<float><<<kSU2Blocks, 256, 0, h->stream>>>(src, st, tmp, h->n3);
+  }
+  return tmp;
+}
+cudaError_t get_comp(clb_handle *h, void *buf, bool field, int c, double *dst)
+{
+  const double *src = flat_comp(h, buf, field, c, h->su2->d_stage);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaMemcpyAsync(dst, src, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+}
+} // namespace
+
 __attribute__((visibility("hidden"))) int su2_set_state(clb_handle *h, const double *fields, const double *momenta,
                                                         const clb_scalefactor *sf)
 {
   SU2Sector *u = h->su2;
   cudaError_t e = cudaStreamSynchronize(h->stream);
   free_tangent(u); // a new state ends the tangent-linear form
-  if (!u->fp32) {
-    if (e == cudaSuccess) e = cudaMemcpyAsync(u->f, fields, NF * h->n3 * sizeof(double), cudaMemcpyDefault, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(u->p, momenta, NP * h->n3 * sizeof(double), cudaMemcpyDefault, h->stream);
-  } else {
-    // one component at a time through the FP64 staging buffer
-    for (int c = 0; c < NF + NP && e == cudaSuccess; ++c) {
-      const double *src = c < NF ? fields + (size_t)c * h->n3 : momenta + (size_t)(c - NF) * h->n3;
-      float *dst = static_cast<float *>(c < NF ? u->f : u->p) + (size_t)(c < NF ? c : c - NF) * h->n3;
-      e = cudaMemcpyAsync(u->d_stage, src, h->n3 * sizeof(double), cudaMemcpyDefault, h->stream);
-      if (e == cudaSuccess) k_convert<double, float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, dst, h->n3);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    }
-  }
+  for (int c = 0; c < NF && e == cudaSuccess; ++c) e = set_comp(h, u->f, true, c, fields + (size_t)c * h->n3);
+  for (int c = 0; c < NP && e == cudaSuccess; ++c) e = set_comp(h, u->p, false, c, momenta + (size_t)c * h->n3);
   if (e == cudaSuccess) {
     // the link phases of the new A
     if (u->fp32)
@@ -331,19 +374,8 @@ __attribute__((visibility("hidden"))) int su2_get_state(clb_handle *h, double *f
   SU2Sector *u = h->su2;
   State s;
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  if (!u->fp32) {
-    if (e == cudaSuccess && fields) e = cudaMemcpyAsync(fields, u->f, NF * h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess && momenta) e = cudaMemcpyAsync(momenta, u->p, NP * h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  } else {
-    for (int c = 0; c < NF + NP && e == cudaSuccess; ++c) {
-      double *dst = c < NF ? (fields ? fields + (size_t)c * h->n3 : nullptr) : (momenta ? momenta + (size_t)(c - NF) * h->n3 : nullptr);
-      if (!dst) continue;
-      const float *src = static_cast<const float *>(c < NF ? u->f : u->p) + (size_t)(c < NF ? c : c - NF) * h->n3;
-      k_convert<float, double><<<kSU2Blocks, 256, 0, h->stream>>>(src, u->d_stage, h->n3);
-      e = cudaMemcpyAsync(dst, u->d_stage, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    }
-  }
+  for (int c = 0; c < NF && e == cudaSuccess && fields; ++c) e = get_comp(h, u->f, true, c, fields + (size_t)c * h->n3);
+  for (int c = 0; c < NP && e == cudaSuccess && momenta; ++c) e = get_comp(h, u->p, false, c, momenta + (size_t)c * h->n3);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&s, u->d_st, sizeof(s), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
@@ -704,49 +736,11 @@ __attribute__((visibility("hidden"))) const double *su2_component(clb_handle *h,
   SU2Sector *u = h->su2;
   if (comp < 0 || comp >= (which == 0 ? NF : NP)) return nullptr;
   *gauge = comp >= 7;
-  if (!u->fp32) return static_cast<const double *>(which == 0 ? u->f : u->p) + (size_t)comp * h->n3;
-  // FP32 form: the component in FP64 in the staging buffer (ordered on the handle's stream)
-  const float *src = static_cast<const float *>(which == 0 ? u->f : u->p) + (size_t)comp * h->n3;
-  k_convert<float, double><<<kSU2Blocks, 256, 0, h->stream>>>(src, u->d_stage, h->n3);
-  return u->d_stage;
+  // in FP64 as one array (in the staging buffer, ordered on the handle's stream, unless it is one)
+  return flat_comp(h, which == 0 ? u->f : u->p, which == 0, comp, u->d_stage);
 }
 
 // ---- tangent-linear form -------------------------------------------------------------------------
-namespace {
-// n components of N^3 FP64 host values into device storage of either form (and back).
-cudaError_t upload_comps(clb_handle *h, void *dst, const double *src, int n)
-{
-  SU2Sector *u = h->su2;
-  cudaError_t e = cudaSuccess;
-  if (!u->fp32) {
-    if (src) return cudaMemcpyAsync(dst, src, n * h->n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    return cudaMemsetAsync(dst, 0, n * h->n3 * sizeof(double), h->stream);
-  }
-  if (!src) return cudaMemsetAsync(dst, 0, n * h->n3 * sizeof(float), h->stream);
-  for (int c = 0; c < n && e == cudaSuccess; ++c) {
-    e = cudaMemcpyAsync(u->d_stage, src + (size_t)c * h->n3, h->n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess)
-      k_convert<double, float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, static_cast<float *>(dst) + (size_t)c * h->n3, h->n3);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  }
-  return e;
-}
-cudaError_t download_comps(clb_handle *h, double *dst, const void *src, int n)
-{
-  SU2Sector *u = h->su2;
-  cudaError_t e = cudaSuccess;
-  if (!dst) return e;
-  if (!u->fp32) return cudaMemcpyAsync(dst, src, n * h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  for (int c = 0; c < n && e == cudaSuccess; ++c) {
-    k_convert<float, double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(src) + (size_t)c * h->n3,
-                                                                 u->d_stage, h->n3);
-    e = cudaMemcpyAsync(dst + (size_t)c * h->n3, u->d_stage, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  }
-  return e;
-}
-} // namespace
-
 // Starts the tangent-linear form: from here clb_initialize, clb_evolve and clb_sync also advance
 // the derivative of the state along couplings_dot (the six couplings' derivatives), starting from
 // the given start-state tangent (null: zero).
@@ -764,7 +758,7 @@ __attribute__((visibility("hidden"))) int su2_tangent_begin(clb_handle *h, const
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_tangent_begin");
   free_tangent(u);
-  bool ok = cudaMalloc(&u->df, NF * h->n3 * u->esz) == cudaSuccess && cudaMalloc(&u->dp, NP * h->n3 * u->esz) == cudaSuccess;
+  bool ok = cudaMalloc(&u->df, u->nf * u->esz) == cudaSuccess && cudaMalloc(&u->dp, NP * h->n3 * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_tst, sizeof(TState)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_tpart, (size_t)kSU2Blocks * 2 * kRed * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_tsums, 2 * kRed * sizeof(double)) == cudaSuccess;
@@ -772,7 +766,12 @@ __attribute__((visibility("hidden"))) int su2_tangent_begin(clb_handle *h, const
     free_tangent(u);
     return h->fail(CLB_ENOMEM, "clb_tangent_begin: tangent storage does not fit");
   }
-  if ((e = upload_comps(h, u->df, fields_dot, NF)) != cudaSuccess || (e = upload_comps(h, u->dp, momenta_dot, NP)) != cudaSuccess) {
+  e = cudaMemsetAsync(u->df, 0, u->nf * u->esz, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(u->dp, 0, NP * h->n3 * u->esz, h->stream);
+  for (int c = 0; c < NF && e == cudaSuccess && fields_dot; ++c) e = set_comp(h, u->df, true, c, fields_dot + (size_t)c * h->n3);
+  for (int c = 0; c < NP && e == cudaSuccess && momenta_dot; ++c) e = set_comp(h, u->dp, false, c, momenta_dot + (size_t)c * h->n3);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream); // the caller's arrays are read
+  if (e != cudaSuccess) {
     free_tangent(u);
     return h->cuda_fail(e, "clb_tangent_begin");
   }
@@ -808,8 +807,8 @@ __attribute__((visibility("hidden"))) int su2_tangent_get_state(clb_handle *h, d
   SU2Sector *u = h->su2;
   if (!u->tangent) return h->fail(CLB_ESTATE, "clb_tangent_get_state: call clb_tangent_begin first");
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess) e = download_comps(h, fields_dot, u->df, NF);
-  if (e == cudaSuccess) e = download_comps(h, momenta_dot, u->dp, NP);
+  for (int c = 0; c < NF && e == cudaSuccess && fields_dot; ++c) e = get_comp(h, u->df, true, c, fields_dot + (size_t)c * h->n3);
+  for (int c = 0; c < NP && e == cudaSuccess && momenta_dot; ++c) e = get_comp(h, u->dp, false, c, momenta_dot + (size_t)c * h->n3);
   TState t;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&t, u->d_tst, sizeof(t), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -903,10 +902,10 @@ __attribute__((visibility("hidden"))) int su2_tangent_end(clb_handle *h)
   return e == cudaSuccess ? CLB_OK : h->cuda_fail(e, "clb_tangent_end");
 }
 
-// Tangent of one state component (clb_tangent_spectrum): raw storage (float in the FP32 form) and
-// the scale factor with its tangent.
-__attribute__((visibility("hidden"))) const void *su2_tangent_component(clb_handle *h, int which, int comp, bool *f32,
-                                                                        double *aI, double *daI)
+// Tangent of one state component (clb_tangent_spectrum) as one FP64 array, and the scale factor with
+// its tangent.  The link-phase buffer, which the tangent form does not use, stages it.
+__attribute__((visibility("hidden"))) const double *su2_tangent_component(clb_handle *h, int which, int comp, double *aI,
+                                                                          double *daI)
 {
   SU2Sector *u = h->su2;
   if (!u->tangent || comp < 0 || comp >= (which == 0 ? NF : NP)) return nullptr;
@@ -914,9 +913,7 @@ __attribute__((visibility("hidden"))) const void *su2_tangent_component(clb_hand
   if (cudaMemcpy(&t, u->d_tst, sizeof(t), cudaMemcpyDeviceToHost) != cudaSuccess) return nullptr;
   *aI = t.aI.v;
   *daI = t.aI.d;
-  *f32 = u->fp32;
-  const char *base = static_cast<const char *>(which == 0 ? u->df : u->dp);
-  return base + (size_t)comp * h->n3 * u->esz;
+  return flat_comp(h, which == 0 ? u->df : u->dp, which == 0, comp, static_cast<double *>(u->ph));
 }
 
 } // namespace clb

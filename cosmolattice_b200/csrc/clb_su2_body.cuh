@@ -97,55 +97,78 @@ template <class S, class T> struct Site {
   const S *f;
   const S *df;
   // U(1) link phases exp(-i dx g A_i) for g = gQ of phi (C) and of Phi (D), kept by the drift:
-  // [4 i + 2 (0 C, 1 D) + (0 cos, 1 sin)] x n3; null: formed from A here
+  // [i][0 C, 1 D][site][cos, sin]; null: formed from A here
   const S *ph;
   const Params *a;
-  size_t s;
-  long long op[3], om[3];
+  uint32_t s, op[3], om[3]; // the site and its neighbours' offsets, modulo 2^32 (a state of more sites fits no GPU)
   T dx, gC, gD, gS, qG, qH, c4;
-  __device__ __forceinline__ T F(int c, size_t t) const
+  __device__ __forceinline__ T F(int c, uint32_t t) const
   {
-    const size_t i = (size_t)c * a->n3 + t;
+    const size_t i = fidx(*a, c, t);
     if constexpr (TanTraits<T>::is)
       return T((typename TanTraits<T>::base)f[i], (typename TanTraits<T>::base)df[i]);
     else
       return (T)f[i];
   }
-  __device__ __forceinline__ Q4<T> link(int i, size_t t) const
+  // the quadruple at index i of the field buffer
+  __device__ __forceinline__ V4<T> quad(size_t i) const
   {
-    const int b = 10 + 4 * i;
-    return Q4<T>{F(b, t), F(b + 1, t), F(b + 2, t), F(b + 3, t)};
+    const V4<S> v = ld4c(f + i);
+    V4<T> r;
+    if constexpr (TanTraits<T>::is) {
+      using B = typename TanTraits<T>::base;
+      const V4<S> d = ld4c(df + i);
+      for (int k = 0; k < 4; ++k) r.v[k] = T((B)v.v[k], (B)d.v[k]);
+    } else {
+      for (int k = 0; k < 4; ++k) r.v[k] = (T)v.v[k];
+    }
+    return r;
   }
-  __device__ __forceinline__ D2<T> dbl(size_t t) const { return D2<T>{C2<T>{F(3, t), F(4, t)}, C2<T>{F(5, t), F(6, t)}}; }
-  __device__ __forceinline__ C2<T> cs(size_t t) const { return C2<T>{F(1, t), F(2, t)}; }
+  __device__ __forceinline__ Q4<T> link(int i, uint32_t t) const
+  {
+    const V4<T> q = quad(fidx(*a, 10 + 4 * i, t));
+    return Q4<T>{q.v[0], q.v[1], q.v[2], q.v[3]};
+  }
+  __device__ __forceinline__ D2<T> dbl(uint32_t t) const
+  {
+    const V4<T> q = quad(fidx(*a, 3, t));
+    return D2<T>{C2<T>{q.v[0], q.v[1]}, C2<T>{q.v[2], q.v[3]}};
+  }
+  __device__ __forceinline__ C2<T> cs(uint32_t t) const { return C2<T>{F(1, t), F(2, t)}; }
   // the stored phases when the arithmetic type is the storage type (the same cos and sin of the
   // same argument, formed by the drift), else formed here
-  __device__ __forceinline__ C2<T> phaseCD(int which, int i, size_t t) const
+  __device__ __forceinline__ C2<T> phaseCD(int which, int i, uint32_t t) const
   {
     if constexpr (std::is_same<S, T>::value) {
       if (ph) {
-        const size_t b = (size_t)(4 * i + 2 * which) * a->n3 + t;
-        return C2<T>{ph[b], ph[b + a->n3]};
+        if constexpr (sizeof(S) == 8) {
+          const double2 q = __ldg(reinterpret_cast<const double2 *>(ph + ((size_t)(2 * i + which) * a->n3 + t) * 2));
+          return C2<T>{q.x, q.y};
+        } else {
+          const float2 q = __ldg(reinterpret_cast<const float2 *>(ph + ((size_t)(2 * i + which) * a->n3 + t) * 2));
+          return C2<T>{q.x, q.y};
+        }
       }
     }
     return phase(which == 0 ? gC : gD, i, t);
   }
-  __device__ __forceinline__ C2<T> phaseC(int i, size_t t) const { return phaseCD(0, i, t); }
-  __device__ __forceinline__ C2<T> phaseD(int i, size_t t) const { return phaseCD(1, i, t); }
-  __device__ __forceinline__ C2<T> phase(T g, int i, size_t t) const
+  __device__ __forceinline__ C2<T> phaseC(int i, uint32_t t) const { return phaseCD(0, i, t); }
+  __device__ __forceinline__ C2<T> phaseD(int i, uint32_t t) const { return phaseCD(1, i, t); }
+  __device__ __forceinline__ C2<T> phase(T g, int i, uint32_t t) const
   {
     const T th = (-dx * g) * F(7 + i, t);
     C2<T> r;
     sincos_link(th, &r.im, &r.re);
     return r;
   }
-  __device__ __forceinline__ T normD(size_t t) const
+  __device__ __forceinline__ T normD(uint32_t t) const
   {
+    const V4<T> d = quad(fidx(*a, 3, t));
     T q = 0;
-    for (int c = 0; c < 4; ++c) q = c == 0 ? F(3, t) * F(3, t) : q + F(3 + c, t) * F(3 + c, t);
+    for (int c = 0; c < 4; ++c) q = c == 0 ? d.v[0] * d.v[0] : q + d.v[c] * d.v[c];
     return sqrt(q);
   }
-  __device__ __forceinline__ T normC(size_t t) const { return sqrt(F(1, t) * F(1, t) + F(2, t) * F(2, t)); }
+  __device__ __forceinline__ T normC(uint32_t t) const { return sqrt(F(1, t) * F(1, t) + F(2, t) * F(2, t)); }
   __device__ __forceinline__ T potTerm(int k) const
   {
     const T nD = normD(s);
@@ -159,9 +182,9 @@ template <class S, class T> struct Site {
   {
     return (c4 * ipw(nD, 4) + qG * ipw(nD * Sv, 2)) + 2 * qH * ipw(nD * nC, 2);
   }
-  __device__ __forceinline__ size_t pl(int i) const { return s + op[i]; }
-  __device__ __forceinline__ size_t mi(int i) const { return s + om[i]; }
-  __device__ __forceinline__ size_t plmi(int i, int j) const { return i == j ? s : s + op[i] + om[j]; }
+  __device__ __forceinline__ uint32_t pl(int i) const { return s + op[i]; }
+  __device__ __forceinline__ uint32_t mi(int i) const { return s + om[i]; }
+  __device__ __forceinline__ uint32_t plmi(int i, int j) const { return i == j ? s : s + op[i] + om[j]; }
   __device__ __forceinline__ D2<T> wD(int i) const { return dscale(phaseD(i, s), qapply(link(i, s), dbl(pl(i)))); }
   __device__ __forceinline__ C2<T> wC(int i) const { return cmul(phaseC(i, s), cs(pl(i))); }
   __device__ __forceinline__ T lapl(int comp) const
@@ -171,19 +194,19 @@ template <class S, class T> struct Site {
     for (int d = 0; d < 3; ++d) t[d] = (F(comp, pl(d)) + F(comp, mi(d))) - 2 * c;
     return recip<T>(a->ddx2) * ((t[0] + t[1]) + t[2]);
   }
-  __device__ __forceinline__ T fd(int comp, size_t t0, size_t t1) const { return div_by(F(comp, t1) - F(comp, t0), a->ddx); }
+  __device__ __forceinline__ T fd(int comp, uint32_t t0, uint32_t t1) const { return div_by(F(comp, t1) - F(comp, t0), a->ddx); }
   __device__ __forceinline__ Q4<T> plaq(int i, int j) const
   {
     return qmul(qmul(qmul(link(i, s), link(j, pl(i))), qdag(link(i, pl(j)))), qdag(link(j, s)));
   }
   __device__ __forceinline__ Q4<T> plaqBack(int i, int j) const
   {
-    const size_t sm = mi(j);
+    const uint32_t sm = mi(j);
     return qdag(qmul(qmul(qmul(link(i, s), qdag(link(j, plmi(i, j)))), qdag(link(i, sm))), link(j, sm)));
   }
 };
 
-template <class S, class T> __device__ __forceinline__ Site<S, T> make_site(const S *f, const Params &a, size_t s)
+template <class S, class T> __device__ __forceinline__ Site<S, T> make_site(const S *f, const Params &a, uint32_t s)
 {
   Site<S, T> v;
   v.f = f;
@@ -198,7 +221,7 @@ template <class S, class T> __device__ __forceinline__ Site<S, T> make_site(cons
   v.qG = (T)a.qG;
   v.qH = (T)a.qH;
   v.c4 = (T)a.c4;
-  u1_offsets(a.N, s, v.op, v.om);
+  site_offsets(a.divN, s, v.op, v.om);
   return v;
 }
 
@@ -210,7 +233,7 @@ struct CoupDot {
 
 // Tangent-linear view: the state f with its tangent df, and the couplings with their tangents.
 template <class S>
-__device__ __forceinline__ Site<S, Tan<S>> make_site_tan(const S *f, const S *df, const Params &a, size_t s,
+__device__ __forceinline__ Site<S, Tan<S>> make_site_tan(const S *f, const S *df, const Params &a, uint32_t s,
                                                         const CoupDot &cd)
 {
   using T = Tan<S>;
@@ -228,7 +251,7 @@ __device__ __forceinline__ Site<S, Tan<S>> make_site_tan(const S *f, const S *df
   v.gD = cp(a.gD, 3);
   v.gS = cp(a.gS, 4);
   v.c4 = cp(a.c4, 5);
-  u1_offsets(a.N, s, v.op, v.om);
+  site_offsets(a.divN, s, v.op, v.om);
   return v;
 }
 
@@ -277,7 +300,7 @@ template <class S, class T> __device__ __forceinline__ void covLapD(const Site<S
       const T n2 = dgrad_term(v, w, v.dbl(v.s));
       *g2 = d == 0 ? n2 : *g2 + n2;
     }
-    const size_t sm = v.mi(d);
+    const uint32_t sm = v.mi(d);
     const D2<T> m = qapply(qdag(v.link(d, sm)), dscale(conj_(v.phaseD(d, sm)), v.dbl(sm)));
     if (d == 0) {
       plus = w;
@@ -339,7 +362,7 @@ template <int SECT = 0, bool AVG = false, class S, class T>
 __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T K[NP], SiteAvg<T> *av = nullptr)
 {
   const Params &a = *v.a;
-  const size_t s = v.s;
+  const uint32_t s = v.s;
   const T A = C.A, B = C.B, B2 = C.B2, G = C.G;
   const T qG = v.qG, qH = v.qH, c4 = v.c4, rfo2 = (T)a.rfo2;
   if constexpr (sect_scalars(SECT)) {
@@ -355,7 +378,8 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
       T dl[4];
       covLapD(v, dl, AVG ? &av->g2D : nullptr);
       const T ndD = c4 * (4 * ipw(nD, 3)) + nD * (2 * qG * ipw(Sv, 2) + 4 * qH * ipw(nC, 2));
-      for (int c = 0; c < 4; ++c) K[3 + c] = A * dl[c] - B2 * (kdiv(ndD, nD) * v.F(3 + c, s));
+      const V4<T> d = v.quad(fidx(a, 3, s));
+      for (int c = 0; c < 4; ++c) K[3 + c] = A * dl[c] - B2 * (kdiv(ndD, nD) * d.v[c]);
     }
     if constexpr (AVG && sect_sphi(SECT)) {
       av->g2S = sGrad2(v);
@@ -571,7 +595,7 @@ __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_K
   const State st = *stp;
   double acc[kRed];
   for (int k = 0; k < kRed; ++k) acc[k] = 0;
-  for_sites(a.N, a.n3, a.order, [&](size_t s) {
+  for_sites(a.N, a.n3, a.order, [&](uint32_t s) {
     Site<S, S> v = make_site<S, S>(f, a, s);
     v.ph = ph;
     S q[NP];
@@ -636,21 +660,22 @@ template <class S> __device__ __forceinline__ Q4<double> qexp(double p1, double 
 // phase arrays the kick reads.
 template <class S> __device__ __forceinline__ void put_phases(S *__restrict__ ph, const Params &a, int i, size_t s, S A)
 {
-  const size_t n3 = a.n3;
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
     const S th = (-(S)a.dx * (S)(which == 0 ? a.gC : a.gD)) * A;
-    const size_t b = (size_t)(4 * i + 2 * which) * n3 + s;
     S c, sn;
     sincos_link(th, &sn, &c);
-    ph[b] = c;
-    ph[b + n3] = sn;
+    S *q = ph + ((size_t)(2 * i + which) * a.n3 + s) * 2;
+    if constexpr (sizeof(S) == 8)
+      *reinterpret_cast<double2 *>(q) = double2{c, sn};
+    else
+      *reinterpret_cast<float2 *>(q) = float2{c, sn};
   }
 }
 template <class S> __global__ void __launch_bounds__(256) k_phases(const S *__restrict__ f, S *__restrict__ ph, Params a)
 {
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < a.n3; s += (size_t)gridDim.x * blockDim.x)
-    for (int i = 0; i < 3; ++i) put_phases(ph, a, i, s, f[(size_t)(7 + i) * a.n3 + s]);
+    for (int i = 0; i < 3; ++i) put_phases(ph, a, i, s, f[fidx(a, 7 + i, s)]);
 }
 
 template <class S>
@@ -669,35 +694,40 @@ __global__ void __launch_bounds__(256)
   const size_t n3 = a.n3;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
     f[s] = (S)((double)f[s] + p3 * (dtw * (double)p[s]));
-    for (int c = 1; c < 7; ++c) f[c * n3 + s] = (S)((double)f[c * n3 + s] + cC * (double)p[c * n3 + s]);
+    for (int c = 1; c < 3; ++c) f[c * n3 + s] = (S)((double)f[c * n3 + s] + cC * (double)p[c * n3 + s]);
+    {
+      S *fd = f + fidx(a, 3, s);
+      V4<S> d = ld4(fd);
+      for (int c = 0; c < 4; ++c) d.v[c] = (S)((double)d.v[c] + cC * (double)p[(3 + c) * n3 + s]);
+      st4(fd, d.v[0], d.v[1], d.v[2], d.v[3]);
+    }
     for (int i = 0; i < 3; ++i) {
-      const S A = (S)((double)f[(7 + i) * n3 + s] + cA * (double)p[(7 + i) * n3 + s] * 1.0);
-      f[(7 + i) * n3 + s] = A;
+      S *fa = f + fidx(a, 7 + i, s);
+      const S A = (S)((double)*fa + cA * (double)p[(7 + i) * n3 + s] * 1.0);
+      *fa = A;
       put_phases(ph, a, i, s, A);
     }
     for (int i = 0; i < 3; ++i) {
-      const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = (size_t)(10 + 4 * i) * n3 + s;
+      const size_t pb = (size_t)(10 + 3 * i) * n3 + s;
+      S *fu = f + fidx(a, 10 + 4 * i, s);
+      const V4<S> q = ld4(fu);
       const Q4<double> E = qexp<S>(cG * (double)p[pb], cG * (double)p[pb + n3], cG * (double)p[pb + 2 * n3]);
-      const Q4<double> U = qmul(E, Q4<double>{(double)f[fb], (double)f[fb + n3], (double)f[fb + 2 * n3], (double)f[fb + 3 * n3]});
-      f[fb] = (S)U.w;
-      f[fb + n3] = (S)U.x;
-      f[fb + 2 * n3] = (S)U.y;
-      f[fb + 3 * n3] = (S)U.z;
+      const Q4<double> U = qmul(E, Q4<double>{(double)q.v[0], (double)q.v[1], (double)q.v[2], (double)q.v[3]});
+      st4(fu, (S)U.w, (S)U.x, (S)U.y, (S)U.z);
     }
   }
 }
 
 // Re-unitarisation of the stored links (FP32 form): U <- U / |U| in FP64.
-template <class S> __global__ void __launch_bounds__(256) k_unitarize(S *__restrict__ f, size_t n3)
+template <class S> __global__ void __launch_bounds__(256) k_unitarize(S *__restrict__ f, Params a)
 {
+  const size_t n3 = a.n3;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < 3 * n3; s += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = s / n3, t = s - i * n3, fb = (size_t)(10 + 4 * i) * n3 + t;
-    const double w = f[fb], x = f[fb + n3], y = f[fb + 2 * n3], z = f[fb + 3 * n3];
+    S *fu = f + a.oU + 4 * s;
+    const V4<S> q = ld4(fu);
+    const double w = q.v[0], x = q.v[1], y = q.v[2], z = q.v[3];
     const double r = 1.0 / sqrt(((w * w + x * x) + y * y) + z * z);
-    f[fb] = (S)(w * r);
-    f[fb + n3] = (S)(x * r);
-    f[fb + 2 * n3] = (S)(y * r);
-    f[fb + 3 * n3] = (S)(z * r);
+    st4(fu, (S)(w * r), (S)(x * r), (S)(y * r), (S)(z * r));
   }
 }
 
@@ -716,7 +746,7 @@ __global__ void __launch_bounds__(128)
   const size_t n3 = a.n3;
   const double dx = a.dx;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
-    const Site<S, double> v = make_site<S, double>(f, a, s);
+    const Site<S, double> v = make_site<S, double>(f, a, (uint32_t)s);
     double q[NP];
     for (int c = 0; c < NP; ++c) q[c] = (double)p[(size_t)c * n3 + s];
     double t[5];
@@ -779,7 +809,7 @@ __global__ void __launch_bounds__(128)
     {
       double L[3];
       for (int i = 0; i < 3; ++i) {
-        const size_t sm = v.mi(i);
+        const uint32_t sm = v.mi(i);
         const Q4<double> Ui = v.link(i, sm);
         const size_t pb = (size_t)(10 + 3 * i) * n3 + sm;
         const Q4<double> r =
@@ -834,17 +864,23 @@ template <int G0 = 0, int G1 = 5, class R> __device__ __forceinline__ void pi2s_
 // Tangent kick sweep: k_kick on (p, dp) with kernels and field sums in Tan<S>; partials
 // [block][2 kRed]: the kRed sums of k_kick, then their tangents.
 // SECT as k_kick: 0 whole; 1 and 2 the halves, or 3, 4 and 2 the three parts, of a split sweep.
-// Resident blocks per SM of the tangent kick parts: three in FP64, four in FP32, timed at 256^3 VV2
-// (ms per tangent step, 1 / 2 / 3 / 4 blocks): FP64 39.2, 39.3, 37.9, 39.3; FP32 23.2, 23.3, 21.9,
-// 21.4.  The value part stays the plain evolution's bitwise either way.
+// Resident blocks per SM of the tangent kick parts: four in FP32, in FP64 three, and four for the S
+// and phi part and the Phi part.  80^3, us per launch at 2 / 3 / 4 blocks: FP64 S and phi 84 / 77 /
+// 58, Phi 122 / 109 / 104, A 142 / 127 / 132, SU(2) 366 / 374 / 371; FP32 tangent step 567 / 509 /
+// 569 at 3 / 4 / 5.  The value part stays the plain evolution's bitwise either way.
 #ifndef CLB_SU2_TAN_MINB_F64
 #define CLB_SU2_TAN_MINB_F64 3
+#endif
+#ifndef CLB_SU2_TAN_P56_MINB_F64
+#define CLB_SU2_TAN_P56_MINB_F64 4
 #endif
 #ifndef CLB_SU2_TAN_MINB_F32
 #define CLB_SU2_TAN_MINB_F32 4
 #endif
 template <class S, int NK, bool RF, bool RP, int SECT = 0>
-__global__ void __launch_bounds__(128, sizeof(S) == 4 ? CLB_SU2_TAN_MINB_F32 : CLB_SU2_TAN_MINB_F64)
+__global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_MINB_F32
+                                       : SECT == 5 || SECT == 6 ? CLB_SU2_TAN_P56_MINB_F64
+                                                                : CLB_SU2_TAN_MINB_F64)
     k_kick_tan(const S *__restrict__ f, const S *__restrict__ df, S *__restrict__ p, S *__restrict__ dp, Params a,
                Kick kc, const TState *__restrict__ stp, CoupDot cd, double *__restrict__ partials)
 {
@@ -857,7 +893,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4 ? CLB_SU2_TAN_MINB_F32 : C
   const Coef<T> C{T(stp->kA), T(stp->kB), T(stp->kB2), T(stp->kG)};
   double acc[2 * kRed];
   for (int k = 0; k < 2 * kRed; ++k) acc[k] = 0;
-  for_sites(a.N, a.n3, a.order, [&](size_t s) {
+  for_sites(a.N, a.n3, a.order, [&](uint32_t s) {
     const Site<S, T> v = make_site_tan<S>(f, df, a, s, cd);
     S q[NP], dq[NP];
     for (int c = C0; c < C1; ++c) {
@@ -972,38 +1008,66 @@ __global__ void __launch_bounds__(256)
     x[i] = (S)r.v;
     dx[i] = (S)r.d;
   };
+  auto ld4t = [&](size_t i) {
+    const V4<S> v = ld4(f + i), d = ld4(df + i);
+    V4<T> r;
+    for (int k = 0; k < 4; ++k) r.v[k] = T((double)v.v[k], (double)d.v[k]);
+    return r;
+  };
+  auto put4 = [&](size_t i, T x, T y, T z, T w) {
+    st4(f + i, (S)x.v, (S)y.v, (S)z.v, (S)w.v);
+    st4(df + i, (S)x.d, (S)y.d, (S)z.d, (S)w.d);
+  };
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
     put(f, df, s, ld(f, df, s) + p3 * (dtw * ld(p, dp, s)));
-    for (int c = 1; c < 7; ++c) put(f, df, c * n3 + s, ld(f, df, c * n3 + s) + cC * ld(p, dp, c * n3 + s));
-    for (int i = 0; i < 3; ++i)
-      put(f, df, (7 + i) * n3 + s, ld(f, df, (7 + i) * n3 + s) + cA * ld(p, dp, (7 + i) * n3 + s) * 1.0);
+    for (int c = 1; c < 3; ++c) put(f, df, c * n3 + s, ld(f, df, c * n3 + s) + cC * ld(p, dp, c * n3 + s));
+    {
+      const size_t fb = fidx(a, 3, s);
+      V4<T> d = ld4t(fb);
+      for (int c = 0; c < 4; ++c) d.v[c] = d.v[c] + cC * ld(p, dp, (3 + c) * n3 + s);
+      put4(fb, d.v[0], d.v[1], d.v[2], d.v[3]);
+    }
     for (int i = 0; i < 3; ++i) {
-      const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = (size_t)(10 + 4 * i) * n3 + s;
+      const size_t fa = fidx(a, 7 + i, s);
+      put(f, df, fa, ld(f, df, fa) + cA * ld(p, dp, (7 + i) * n3 + s) * 1.0);
+    }
+    for (int i = 0; i < 3; ++i) {
+      const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = fidx(a, 10 + 4 * i, s);
+      const V4<T> q = ld4t(fb);
       const Q4<T> E = qexp_tan<S>(cG * ld(p, dp, pb), cG * ld(p, dp, pb + n3), cG * ld(p, dp, pb + 2 * n3));
-      const Q4<T> U = qmul(E, Q4<T>{ld(f, df, fb), ld(f, df, fb + n3), ld(f, df, fb + 2 * n3), ld(f, df, fb + 3 * n3)});
-      put(f, df, fb, U.w);
-      put(f, df, fb + n3, U.x);
-      put(f, df, fb + 2 * n3, U.y);
-      put(f, df, fb + 3 * n3, U.z);
+      const Q4<T> U = qmul(E, Q4<T>{q.v[0], q.v[1], q.v[2], q.v[3]});
+      put4(fb, U.w, U.x, U.y, U.z);
     }
   }
 }
 
 // Tangent re-unitarisation (FP32 form): U <- U / |U| on (f, df).
-template <class S> __global__ void __launch_bounds__(256) k_unitarize_tan(S *__restrict__ f, S *__restrict__ df, size_t n3)
+template <class S> __global__ void __launch_bounds__(256) k_unitarize_tan(S *__restrict__ f, S *__restrict__ df, Params a)
 {
   using T = Tan<double>;
+  const size_t n3 = a.n3;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < 3 * n3; s += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = s / n3, t = s - i * n3, fb = (size_t)(10 + 4 * i) * n3 + t;
-    T q[4];
-    for (int c = 0; c < 4; ++c) q[c] = T((double)f[fb + c * n3], (double)df[fb + c * n3]);
+    const V4<S> v = ld4(f + a.oU + 4 * s), d = ld4(df + a.oU + 4 * s);
+    T q[4], u[4];
+    for (int c = 0; c < 4; ++c) q[c] = T((double)v.v[c], (double)d.v[c]);
     const T r = 1.0 / sqrt(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
-    for (int c = 0; c < 4; ++c) {
-      const T u = q[c] * r;
-      f[fb + c * n3] = (S)u.v;
-      df[fb + c * n3] = (S)u.d;
-    }
+    for (int c = 0; c < 4; ++c) u[c] = q[c] * r;
+    st4(f + a.oU + 4 * s, (S)u[0].v, (S)u[1].v, (S)u[2].v, (S)u[3].v);
+    st4(df + a.oU + 4 * s, (S)u[0].d, (S)u[1].d, (S)u[2].d, (S)u[3].d);
   }
+}
+
+// One field or momentum component between its place on the device (the elements base + stride s) and
+// an FP64 array.
+template <class S> __global__ void __launch_bounds__(256) k_comp_get(const S *__restrict__ src, int stride, double *__restrict__ dst, size_t n)
+{
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    dst[i] = (double)src[i * stride];
+}
+template <class S> __global__ void __launch_bounds__(256) k_comp_set(const double *__restrict__ src, S *__restrict__ dst, int stride, size_t n)
+{
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    dst[i * stride] = (S)src[i];
 }
 
 } // namespace su2d

@@ -13,13 +13,14 @@ using namespace su2d;
 constexpr int kSU2Blocks = 148 * 8; // 128-thread grid-stride sweeps
 
 struct SU2Sector {
-  void *f = nullptr, *p = nullptr; // 22 and 19 x N^3 of double (FP64) or float (FP32 form)
+  void *f = nullptr, *p = nullptr; // fields (nf elements, fidx) and 19 x N^3 momenta, double (FP64) or float (FP32 form)
+  size_t nf = 0;
   bool fp32 = false;
   size_t esz = 8;
   State *d_st = nullptr;
   double *d_part = nullptr, *d_sums = nullptr;
-  double *d_stage = nullptr; // one FP64 component, for FP32 conversions
-  void *ph = nullptr;        // U(1) link phases (12 x N^3, storage type), kept by the drifts
+  double *d_stage = nullptr; // one FP64 component, for conversions
+  void *ph = nullptr;        // U(1) link phases (6 x N^3 pairs, storage type), kept by the drifts
   // kick sweeps: 0 one sweep, 1 two halves, 2 three parts, 3 four parts (S and phi; Phi; A; SU(2))
   // (CLB_SU2_SPLIT sets both forms).  su2_create takes four parts in FP64 and three in FP32, by
   // timing at 384^3 VV2 since the kick forms the field averages from its own products (ms per
