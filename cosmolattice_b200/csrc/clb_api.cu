@@ -129,6 +129,7 @@ void sweep_sh(clb_handle *h, int kind, int fb, int pb, int fo, int po, double dt
                          160 * 1024);
     attr_set = true;
   }
+  h->rb_valid = false;
   SweepArgs a = h->sw;
   a.dtw = dtw;
   a.h1 = h1;
@@ -203,6 +204,7 @@ template <class R, int NS> struct Launch {
   // elementwise in-place drift over the whole padded arrays (ghosts stay periodic copies)
   static void drift(clb_handle *h, double dtw)
   {
+    h->rb_valid = false;
     CLB_LAUNCH(h, K_DRIFT,
                k_drift<R><<<kElemBlocks, 256, 0, h->stream>>>(F<R>(h, h->cf), P<R>(h, h->cp),
                                                                (size_t)NS * (size_t)h->pd.comp, dtw, h->d_st, h->rs,
@@ -259,6 +261,7 @@ cudaError_t upload(clb_handle *h, const double *src, void *dst, CompOffsets off)
   return cudaGetLastError();
 }
 
+// (ordered on the handle's stream: the caller waits for it)
 cudaError_t download(clb_handle *h, const void *src, double *dst, CompOffsets off)
 {
   const long long planes = (long long)h->NS * h->N, per = (long long)h->N * h->N;
@@ -275,7 +278,7 @@ cudaError_t download(clb_handle *h, const void *src, double *dst, CompOffsets of
                                     cudaMemcpyDeviceToHost, h->stream);
     if (r != cudaSuccess) return r;
   }
-  return cudaStreamSynchronize(h->stream);
+  return cudaGetLastError();
 }
 
 // 3-D tensor map over the stacked padded components: dims {Zp, Yp, NS N}, box = one plane tile.
@@ -311,6 +314,7 @@ bool encode_map(clb_handle *h, void *base, CUtensorMap *map, std::string &why)
 void tail(clb_handle *h, uint32_t flags, int nblocks, double w = 0, double w2 = 0, int64_t hist_row = -1,
           double fa = 0, double fb = 0)
 {
+  h->rb_valid = false;
   TailOp op{flags, nblocks, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
   if (h->pdl_now)
     CLB_LAUNCH(h, K_TAIL, launch_pdl(k_tail, dim3(1), dim3(kTailThreads), 0, h->stream, (const double *)h->d_part, op,
@@ -659,21 +663,24 @@ template <class R, int NS> struct Measure {
   static void run(clb_handle *h, double am) { Launch<R, NS>::measure(h, am); }
 };
 
+// The device's scalar state and error flag in h->rb, with the stream idle.
+cudaError_t read_back(clb_handle *h)
+{
+  if (h->rb_valid) return cudaSuccess;
+  cudaError_t e = cudaMemcpyAsync(h->rb, h->d_st, sizeof(Readback), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  h->rb_valid = e == cudaSuccess;
+  return e;
+}
+
 int sync_and_check(clb_handle *h, const char *where)
 {
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return h->cuda_fail(e, where);
-  e = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, where);
   collect_profile(h);
-  DevState s;
-  e = cudaMemcpy(&s, h->d_st, sizeof(s), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return h->cuda_fail(e, where);
-  int terr = 0;
-  e = cudaMemcpy(&terr, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return h->cuda_fail(e, where);
-  if (terr != 0) return h->fail(CLB_ETIMEOUT, std::string(where) + ": a sweep's bounded wait for its tile loads gave up");
-  if (s.status != 0) return h->fail(CLB_ENONFINITE, std::string(where) + ": a volume average or a(t) is not finite");
+  if (h->rb->err != 0) return h->fail(CLB_ETIMEOUT, std::string(where) + ": a sweep's bounded wait for its tile loads gave up");
+  if (h->rb->st.status != 0) return h->fail(CLB_ENONFINITE, std::string(where) + ": a volume average or a(t) is not finite");
   return CLB_OK;
 }
 
@@ -821,10 +828,11 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
     ok = cudaMalloc(&h->fld[b], bytes) == cudaSuccess && cudaMalloc(&h->pi[b], bytes) == cudaSuccess;
     if (ok) ok = cudaMemset(h->fld[b], 0, bytes) == cudaSuccess && cudaMemset(h->pi[b], 0, bytes) == cudaSuccess;
   }
-  ok = ok && cudaMalloc(&h->d_st, sizeof(DevState)) == cudaSuccess;
+  ok = ok && cudaMalloc(&h->d_st, sizeof(Readback)) == cudaSuccess && cudaMemset(h->d_st, 0, sizeof(Readback)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&h->rb, sizeof(Readback)) == cudaSuccess;
+  if (ok) h->d_err = &reinterpret_cast<Readback *>(h->d_st)->err;
   ok = ok && cudaMalloc(&h->d_part, h->part_rows * kMeasSlots * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_sums, kMeasSlots * sizeof(double)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_err, sizeof(int)) == cudaSuccess && cudaMemset(h->d_err, 0, sizeof(int)) == cudaSuccess;
   ok = ok && cudaEventCreate(&h->ev_call[0]) == cudaSuccess && cudaEventCreate(&h->ev_call[1]) == cudaSuccess;
   if (ok) {
     h->stage_n = std::max<size_t>(kStageMin, (size_t)h->N * h->N);
@@ -869,7 +877,7 @@ void clb_destroy(clb_handle *h)
   if (h->d_st) cudaFree(h->d_st);
   if (h->d_part) cudaFree(h->d_part);
   if (h->d_sums) cudaFree(h->d_sums);
-  if (h->d_err) cudaFree(h->d_err);
+  if (h->rb) cudaFreeHost(h->rb);
   if (h->d_hist) cudaFree(h->d_hist);
   if (h->d_stage) cudaFree(h->d_stage);
   if (h->plan_ok) cufftDestroy(h->plan);
@@ -959,6 +967,7 @@ __attribute__((visibility("hidden"))) int clb::scalar_set_state(clb_handle *h, c
     s.ref_phi[0][f] = s.ref_phi[1][f] = fo.v[f];
     s.ref_pi[0][f] = s.ref_pi[1][f] = po.v[f];
   }
+  h->rb_valid = false;
   e = cudaMemcpy(h->d_st, &s, sizeof(s), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_set_state");
   h->has_state = true;
@@ -974,11 +983,9 @@ int clb_get_state(clb_handle *h, double *fields, double *momenta, clb_scalefacto
   if (!h) return CLB_EINVAL;
   if (h->u1) return u1_get_state(h, fields, momenta, sf);
   if (h->su2) return su2_get_state(h, fields, momenta, sf);
-  cudaError_t e = cudaStreamSynchronize(h->stream);
+  cudaError_t e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
-  DevState cur;
-  e = cudaMemcpy(&cur, h->d_st, sizeof(cur), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
+  const DevState cur = h->rb->st;
   CompOffsets fo{{0.0, 0.0}}, po{{0.0, 0.0}};
   if (h->fp32)
     for (int f = 0; f < h->NS; ++f) {
@@ -990,17 +997,15 @@ int clb_get_state(clb_handle *h, double *fields, double *momenta, clb_scalefacto
   };
   e = fetch(h->fld[h->cf], fields, fo);
   if (e == cudaSuccess) e = fetch(h->pi[h->cp], momenta, po);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
   if (sf) {
-    DevState s;
-    e = cudaMemcpy(&s, h->d_st, sizeof(s), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
-    sf->aI = s.aI;
-    sf->aSI = s.aSI;
-    sf->aIM = s.aIM;
-    sf->aDotI = s.aDotI;
-    sf->aDotSI = s.aDotSI;
-    sf->aDotSIM = s.aDotSIM;
+    sf->aI = cur.aI;
+    sf->aSI = cur.aSI;
+    sf->aIM = cur.aIM;
+    sf->aDotI = cur.aDotI;
+    sf->aDotSI = cur.aDotSI;
+    sf->aDotSIM = cur.aDotSIM;
   }
   return CLB_OK;
 }
@@ -1147,10 +1152,9 @@ int clb_measure(clb_handle *h, double e0, clb_measurement *m)
   if (!h->initialized) return h->fail(CLB_ESTATE, "clb_measure: call clb_initialize first");
   if (h->u1) return u1_measure(h, e0, m);
   if (h->su2) return su2_measure(h, e0, m);
-  DevState s;
-  cudaError_t e = cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess) e = cudaMemcpy(&s, h->d_st, sizeof(s), cudaMemcpyDeviceToHost);
+  cudaError_t e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_measure");
+  DevState s = h->rb->st;
   const double al = h->md.alpha;
   const double am = std::pow(s.aI, al - 3);
   dispatch<Measure>(h, am);
@@ -1201,7 +1205,8 @@ int clb_measure(clb_handle *h, double e0, clb_measurement *m)
     m->friedmann[0] = (LHS - RHS) / (LHS + RHS);
     m->friedmann[1] = LHS;
     m->friedmann[2] = RHS;
-    e = cudaMemcpy(h->d_st, &s, sizeof(s), cudaMemcpyHostToDevice);
+    h->rb->st = s; // the stream is idle: no copy into or out of rb is in flight
+    e = cudaMemcpyAsync(h->d_st, &h->rb->st, sizeof(s), cudaMemcpyHostToDevice, h->stream);
     if (e != cudaSuccess) return h->cuda_fail(e, "clb_measure");
   } else {
     m->friedmann[0] = std::fabs(1.0 - Etot / e0);
@@ -1367,8 +1372,8 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
     const size_t comp_off = (size_t)comp * (size_t)h->pd.comp;
     double ref = 0.0;
     if (h->fp32) {
-      DevState cur;
-      if ((e = cudaMemcpy(&cur, h->d_st, sizeof(cur), cudaMemcpyDeviceToHost)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
+      if ((e = read_back(h)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
+      const DevState &cur = h->rb->st;
       ref = which == 0 ? cur.ref_phi[h->rs][comp] : cur.ref_pi[h->rs][comp];
       CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather<float><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const float *>(src) + comp_off, h->d_spec, h->pd, ref));
     } else {
@@ -1406,9 +1411,8 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
     if (r != CLB_OK) return r;
     aI = sf.aI;
   } else {
-    DevState s;
-    if ((e = cudaMemcpy(&s, h->d_st, sizeof(s), cudaMemcpyDeviceToHost)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
-    aI = s.aI;
+    if ((e = read_back(h)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
+    aI = h->rb->st.aI;
   }
   const double kIR = 2 * 3.14159265358979323846 / (N * h->cfg.dx);
   // momenta: a^{2 alpha - 6} for matter (scalarsingletmeasurer.h:80), a^{2 alpha - 2} for gauge

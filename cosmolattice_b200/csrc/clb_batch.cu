@@ -74,6 +74,7 @@ struct clb_batch {
   int *d_blk = nullptr;
   DevState *d_st = nullptr;
   double *d_part = nullptr, *d_sums = nullptr, *d_stage = nullptr;
+  DevState *rb = nullptr; // pinned: one member's state on its way to the host
   size_t stage_n = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -648,6 +649,7 @@ void clb_batch_destroy(clb_batch *b)
   for (void *q : {(void *)b->d_lat, (void *)b->d_blk, (void *)b->d_st, (void *)b->d_part, (void *)b->d_sums,
                   (void *)b->d_stage, (void *)b->d_plat, (void *)b->d_members, (void *)b->d_offsets})
     if (q) cudaFree(q);
+  if (b->rb) cudaFreeHost(b->rb);
   for (auto e : b->ev)
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -739,6 +741,7 @@ int clb_batch_create(const clb_config *cfgs, const clb_model_desc *mds, int32_t 
   ok = ok && cudaMalloc(&b->d_offsets, (size_t)(n + 1) * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_sums, 8 * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_stage, b->stage_n * sizeof(double)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&b->rb, sizeof(DevState)) == cudaSuccess;
   ok = ok && cudaEventCreate(&b->ev[0]) == cudaSuccess && cudaEventCreate(&b->ev[1]) == cudaSuccess;
   if (ok) {
     // a configuration tuned earlier in this process for the same ensemble, else the default
@@ -831,9 +834,10 @@ int clb_batch_get_state(clb_batch *b, int32_t i, double *fields, double *momenta
   const BatchLat &L = b->lat[(size_t)i];
   const size_t n3 = (size_t)L.N * L.N * L.N;
   DevState s;
-  cudaError_t e = cudaStreamSynchronize(b->stream);
-  if (e == cudaSuccess) e = cudaMemcpy(&s, b->d_st + i, sizeof(s), cudaMemcpyDeviceToHost);
-  for (int w = 0; w < 2 && e == cudaSuccess; ++w) {
+  cudaError_t e = cudaMemcpyAsync(b->rb, b->d_st + i, sizeof(s), cudaMemcpyDeviceToHost, b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  s = *b->rb;
+  for (int w = 0; w < 2 && e == cudaSuccess; ++w) { // the two arrays in stream order, one wait
     double *dst = w == 0 ? fields : momenta;
     if (!dst) continue;
     const void *src = w == 0 ? b->f[b->cf] : b->p[b->cf];
@@ -843,8 +847,8 @@ int clb_batch_get_state(clb_batch *b, int32_t i, double *fields, double *momenta
     else
       k_batch_unpack<double><<<kPackBlocks, 256, 0, b->stream>>>(static_cast<const double *>(src) + L.off, b->d_stage, n3, 0.0);
     e = cudaMemcpyAsync(dst, b->d_stage, n3 * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "clb_batch_get_state");
   if (sf) {
     sf->aI = s.aI;

@@ -177,6 +177,16 @@ template <class S, class D> __global__ void __launch_bounds__(256) k_gw_copy(con
 
 bool gw_ok(const clb_handle *h) { return h->gw != nullptr; }
 
+// The transform buffers (5 x N x N x 2 (N/2 + 1) doubles), which also stage the FP32 form's transfers
+// (5 N^3 doubles fit), kept with the sector.
+cudaError_t gw_scratch(clb_handle *h, double **out)
+{
+  cudaError_t e = cudaSuccess;
+  if (!h->gw->d_fk) e = cudaMalloc(&h->gw->d_fk, 5 * (size_t)h->N * h->N * 2 * (h->N / 2 + 1) * sizeof(double));
+  *out = h->gw->d_fk;
+  return e;
+}
+
 } // namespace
 
 namespace clb {
@@ -194,6 +204,7 @@ __attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w, bool
 {
   GWSector *g = h->gw;
   g->synced = false;
+  h->rb_valid = false;
   if (h->u1) return u1_gw_kick(h, w, drift);
   if (h->su2) return su2_gw_kick(h, w, drift);
   auto go = [&](auto zero, auto ns) {
@@ -214,6 +225,7 @@ __attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w, bool
 // Runs one GW drift with the a_SI of the matter step just taken.
 __attribute__((visibility("hidden"))) void gw_drift(clb_handle *h)
 {
+  h->rb_valid = false;
   if (h->u1) return u1_gw_drift(h);
   if (h->su2) return su2_gw_drift(h);
   GWSector *g = h->gw;
@@ -253,7 +265,7 @@ __attribute__((visibility("hidden"))) void gw_set_synced(clb_handle *h, bool s) 
 __attribute__((visibility("hidden"))) void gw_destroy(clb_handle *h)
 {
   if (!h->gw) return;
-  for (void *p : {h->gw->u, h->gw->pi, h->gw->u2, h->gw->pi2})
+  for (void *p : {h->gw->u, h->gw->pi, h->gw->u2, h->gw->pi2, h->gw->d_bins})
     if (p) cudaFree(p);
   if (h->gw->d_fk) cudaFree(h->gw->d_fk);
   delete h->gw;
@@ -285,12 +297,7 @@ int clb_gws_enable(clb_handle *h)
     gw_destroy(h);
     return h->fail(CLB_ENOMEM, std::string("clb_gws_enable: ") + cudaGetErrorString(e));
   }
-  // without room for the second pair the drift and the kick run as two sweeps
-  if (cudaMalloc(&g->u2, bytes) != cudaSuccess || cudaMalloc(&g->pi2, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    if (g->u2) cudaFree(g->u2);
-    g->u2 = g->pi2 = nullptr;
-  }
+  alloc_pair(&g->u2, &g->pi2, bytes); // without it the drift and the kick run as two sweeps
   return CLB_OK;
 }
 
@@ -300,20 +307,17 @@ int clb_gws_set_state(clb_handle *h, const double *u, const double *pi)
   if (!gw_ok(h)) return h->fail(CLB_ESTATE, "clb_gws_set_state: call clb_gws_enable first");
   const size_t n = 5 * h->n3;
   double *tmp = nullptr;
-  cudaError_t e = cudaMalloc(&tmp, n * sizeof(double));
+  cudaError_t e = h->gw->fp32 ? gw_scratch(h, &tmp) : cudaSuccess;
   for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
     const double *src = k == 0 ? u : pi;
     void *dst = k == 0 ? h->gw->u : h->gw->pi;
     if (!src) continue;
-    e = cudaMemcpyAsync(tmp, src, n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    if (e != cudaSuccess) break;
-    if (h->gw->fp32)
+    e = cudaMemcpyAsync(h->gw->fp32 ? tmp : dst, src, n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess && h->gw->fp32)
       k_gw_copy<double, float><<<kGWBlocks, 256, 0, h->stream>>>(tmp, static_cast<float *>(dst), n);
-    else
-      e = cudaMemcpyAsync(dst, tmp, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   }
-  if (tmp) cudaFree(tmp);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_gws_set_state");
   return CLB_OK;
 }
@@ -324,19 +328,16 @@ int clb_gws_get_state(clb_handle *h, double *u, double *pi)
   if (!gw_ok(h)) return h->fail(CLB_ESTATE, "clb_gws_get_state: call clb_gws_enable first");
   const size_t n = 5 * h->n3;
   double *tmp = nullptr;
-  cudaError_t e = cudaMalloc(&tmp, n * sizeof(double));
+  cudaError_t e = h->gw->fp32 ? gw_scratch(h, &tmp) : cudaSuccess;
   for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
     double *dst = k == 0 ? u : pi;
     const void *src = k == 0 ? h->gw->u : h->gw->pi;
     if (!dst) continue;
     if (h->gw->fp32)
       k_gw_copy<float, double><<<kGWBlocks, 256, 0, h->stream>>>(static_cast<const float *>(src), tmp, n);
-    else
-      e = cudaMemcpyAsync(tmp, src, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, tmp, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    e = cudaMemcpyAsync(dst, h->gw->fp32 ? tmp : src, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
   }
-  if (tmp) cudaFree(tmp);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_gws_get_state");
   return CLB_OK;
 }
@@ -359,7 +360,8 @@ int clb_gw_spectrum(clb_handle *h, int32_t prj_type, int32_t ps_type, int32_t ps
   const size_t nzh = (size_t)(N / 2 + 1);
   const size_t comp_n = (size_t)N * N * 2 * nzh; // doubles per in-place D2Z buffer
   cudaError_t e = cudaSuccess;
-  if (!h->gw->d_fk && (e = cudaMalloc(&h->gw->d_fk, 5 * comp_n * sizeof(double))) != cudaSuccess)
+  double *fk = nullptr;
+  if ((e = gw_scratch(h, &fk)) != cudaSuccess)
     return h->fail(CLB_ENOMEM, std::string("clb_gw_spectrum: ") + cudaGetErrorString(e));
   if (!h->plan_ok) {
     if (cufftPlan3d(&h->plan, N, N, N, CUFFT_D2Z) != CUFFT_SUCCESS) return h->fail(CLB_ECUDA, "clb_gw_spectrum: cufftPlan3d failed");
@@ -377,12 +379,19 @@ int clb_gw_spectrum(clb_handle *h, int32_t prj_type, int32_t ps_type, int32_t ps
     if (cufftExecD2Z(h->plan, dst, reinterpret_cast<cufftDoubleComplex *>(dst)) != CUFFT_SUCCESS)
       return h->fail(CLB_ECUDA, "clb_gw_spectrum: cufftExecD2Z failed");
   }
-  double *part_val = nullptr, *out = nullptr;
-  unsigned long long *part_cnt = nullptr, *outc = nullptr;
-  e = cudaMalloc(&part_val, (size_t)kGWSpecBlocks * nbins * 2 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&part_cnt, (size_t)kGWSpecBlocks * nbins * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&out, (size_t)nbins * 2 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&outc, (size_t)nbins * sizeof(unsigned long long));
+  // bin partials and sums, kept for spectra of up to this many bins
+  GWSector *g = h->gw;
+  const size_t pv = (size_t)kGWSpecBlocks * nbins;
+  const size_t need = (2 * pv + 2 * (size_t)nbins) * sizeof(double) + (pv + (size_t)nbins) * sizeof(unsigned long long);
+  if (need > g->bins_bytes) {
+    if (g->d_bins) cudaFree(g->d_bins);
+    g->d_bins = nullptr;
+    g->bins_bytes = 0;
+    e = cudaMalloc(&g->d_bins, need);
+    if (e == cudaSuccess) g->bins_bytes = need;
+  }
+  double *part_val = static_cast<double *>(g->d_bins), *out = part_val + 2 * pv;
+  unsigned long long *part_cnt = reinterpret_cast<unsigned long long *>(out + 2 * (size_t)nbins), *outc = part_cnt + pv;
   std::vector<double> sums(2 * (size_t)nbins);
   std::vector<unsigned long long> cnt((size_t)nbins);
   const size_t smem = (size_t)nbins * (2 * sizeof(double) + sizeof(unsigned long long));
@@ -399,8 +408,6 @@ int clb_gw_spectrum(clb_handle *h, int32_t prj_type, int32_t ps_type, int32_t ps
   if (e == cudaSuccess) e = cudaMemcpyAsync(sums.data(), out, sums.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), outc, cnt.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  for (void *p : {(void *)part_val, (void *)part_cnt, (void *)out, (void *)outc})
-    if (p) cudaFree(p);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_gw_spectrum");
   // the PS normalisation of clb_spectrum, then (fStar/MPl)^2 / (4 a^6 rho) (powerspectrum.h:58)
   const double pi = 3.14159265358979323846;

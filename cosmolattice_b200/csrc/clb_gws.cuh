@@ -25,6 +25,8 @@ struct GWSector {
   bool fp32 = false;                 // FP32 storage and arithmetic (the handle's FP32 form)
   bool synced = true;                // momenta at integer time (after clb_initialize or a sync)
   double *d_fk = nullptr;            // five in-place D2Z buffers of the spectrum
+  void *d_bins = nullptr;            // its bin partials and sums
+  size_t bins_bytes = 0;
 };
 
 // x / dx: FP64 as the reference's rounded division, FP32 divides.

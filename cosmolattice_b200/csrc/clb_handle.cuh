@@ -24,6 +24,12 @@ using clb::U1Sector;
 using clb::SU2Sector;
 using namespace clb;
 
+// What every call of a scalar-singlet handle checks or reads at its end.
+struct Readback {
+  DevState st;
+  int err;
+};
+
 struct clb_handle {
   clb_config cfg;
   clb_model_desc md;
@@ -44,8 +50,13 @@ struct clb_handle {
   bool pdl_now = false; // set while the fused loop issues its sweeps and tails
   int bz = 64, by = 8; // sites per block tile in z and y
   size_t sweep_smem = 0;
-  int *d_err = nullptr; // set by a sweep whose bounded wait gave up
-  DevState *d_st = nullptr;
+  DevState *d_st = nullptr; // the first member of a Readback on the device
+  int *d_err = nullptr;     // its second: set by a sweep whose bounded wait gave up
+  // The last Readback in pinned memory (scalar singlets): one asynchronous copy behind a call's work
+  // takes the place of a synchronous copy per value (about 10 us each), and calls between which
+  // nothing ran read it as it is.  rb_valid: nothing that changes the device's was launched since.
+  Readback *rb = nullptr;
+  bool rb_valid = false;
   double *d_part = nullptr;
   double *d_sums = nullptr;
   size_t part_rows = 0;
@@ -147,6 +158,21 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+// Two arrays of the given size for a sweep that writes a second copy of the state, if they take no
+// more than a quarter of the free device memory (what a handle allocates later has to fit as before);
+// both null otherwise, and the handle then runs the sweeps that work in place.
+void alloc_pair(void **a, void **b, size_t bytes)
+{
+  size_t free_b = 0, total = 0;
+  *a = *b = nullptr;
+  if (cudaMemGetInfo(&free_b, &total) != cudaSuccess || 8 * bytes > free_b) return;
+  if (cudaMalloc(a, bytes) != cudaSuccess || cudaMalloc(b, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    if (*a) cudaFree(*a);
+    *a = *b = nullptr;
+  }
 }
 
 cudaEvent_t take_event(clb_handle *h)
