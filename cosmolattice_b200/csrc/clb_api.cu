@@ -232,7 +232,7 @@ template <class R, int NS> struct Launch {
                k_measure_pad<R, NS><<<kElemBlocks, 256, 0, h->stream>>>(F<R>(h, h->cf), P<R>(h, h->cp), h->pd,
                                                                         h->sa.inv_dx2, h->sa.cs.mc, am, h->d_st,
                                                                         h->rs, h->d_part));
-    CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kMeasSlots><<<1, 256, 0, h->stream>>>(h->d_part, kElemBlocks, h->d_sums));
+    CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kMeasSlots><<<1, 512, 0, h->stream>>>(h->d_part, kElemBlocks, h->d_sums));
   }
 };
 

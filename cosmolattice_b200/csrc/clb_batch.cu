@@ -973,7 +973,7 @@ int clb_batch_measure(clb_batch *b, int32_t i, double e0, clb_measurement *m)
     k_batch_measure<double><<<kMeasBlocks, 256, 0, b->stream>>>(static_cast<const double *>(b->f[b->cf]),
                                                                static_cast<const double *>(b->p[b->cf]), L, b->d_st + i,
                                                                b->rs, am, b->d_part);
-  k_sum_partials<7><<<1, 256, 0, b->stream>>>(b->d_part, kMeasBlocks, b->d_sums);
+  k_sum_partials<7><<<1, 512, 0, b->stream>>>(b->d_part, kMeasBlocks, b->d_sums);
   double v[7];
   e = cudaMemcpyAsync(v, b->d_sums, sizeof(v), cudaMemcpyDeviceToHost, b->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

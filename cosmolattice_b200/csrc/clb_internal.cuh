@@ -166,11 +166,10 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV], double *smem /* [N
 // Fixed-order sums of the NV columns of a sweep's partial rows (nrows x NV), in G groups of rows
 // (b, b + G, ...): a thread takes column t % NVP of its groups, so a warp's loads are contiguous,
 // and one warp per column adds the group sums.  The block has a multiple of NVP threads (NVP >= NV
-// a power of two), G is a multiple of 32; every thread gets the sums, whose
-// order depends on G alone.
+// a power of two), G is a multiple of 32; the sums, whose order depends on G alone, are at
+// smem[NV G] on, for every thread.
 template <int NV, int NVP, int G>
-__device__ __forceinline__ void rows_reduce(const double *__restrict__ rows, int nrows, double *smem /* NV (G + 1) */,
-                                            double (&v)[NV])
+__device__ __forceinline__ void rows_sums(const double *__restrict__ rows, int nrows, double *smem /* NV (G + 1) */)
 {
   constexpr int U = 8; // rows in flight per thread
   const int k = threadIdx.x % NVP;
@@ -198,6 +197,11 @@ __device__ __forceinline__ void rows_reduce(const double *__restrict__ rows, int
     if (lane == 0) smem[NV * G + c] = s;
   }
   __syncthreads();
+}
+template <int NV, int NVP, int G>
+__device__ __forceinline__ void rows_reduce(const double *__restrict__ rows, int nrows, double *smem, double (&v)[NV])
+{
+  rows_sums<NV, NVP, G>(rows, nrows, smem);
 #pragma unroll
   for (int j = 0; j < NV; ++j) v[j] = smem[NV * G + j];
 }

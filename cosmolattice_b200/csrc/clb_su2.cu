@@ -651,7 +651,7 @@ __attribute__((visibility("hidden"))) int su2_measure(clb_handle *h, double e0, 
   else
     CLB_LAUNCH(h, K_MEASURE, su2d::k_measure<double><<<kSU2Blocks, 128, 0, h->stream>>>(
                                  static_cast<const double *>(u->f), static_cast<const double *>(u->p), u->prm, am, ag, u->d_part));
-  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kMeas><<<1, 256, 0, h->stream>>>(u->d_part, kSU2Blocks, u->d_sums));
+  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kMeas><<<1, 512, 0, h->stream>>>(u->d_part, kSU2Blocks, u->d_sums));
   double v[kMeas];
   e = cudaMemcpyAsync(v, u->d_sums, sizeof(v), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -832,7 +832,7 @@ static int tangent_energies(clb_handle *h, const char *where, Tan<double> (&en)[
   if (!u->tangent) return h->fail(CLB_ESTATE, std::string(where) + ": call clb_tangent_begin first");
   if (h->cfg.evolver == CLB_LF && !h->synced) return h->fail(CLB_ESTATE, std::string(where) + ": call clb_sync first");
   sweep(h, 0, true, true, Kick{});
-  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<2 * kRed><<<1, 256, 0, h->stream>>>(u->d_tpart, kSU2Blocks, u->d_tsums));
+  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<2 * kRed><<<1, 512, 0, h->stream>>>(u->d_tpart, kSU2Blocks, u->d_tsums));
   double v[2 * kRed];
   TState t;
   cudaError_t e = cudaMemcpyAsync(v, u->d_tsums, sizeof(v), cudaMemcpyDeviceToHost, h->stream);

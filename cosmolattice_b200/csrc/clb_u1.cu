@@ -62,7 +62,8 @@ struct U1Sector {
   int64_t seg_cap = 0;   // boundary states the segment buffer holds
   U1State *d_rec = nullptr;
   double *qbar = nullptr, *pbar[2] = {nullptr, nullptr};
-  double *d_apart = nullptr, *d_asums = nullptr;
+  double *d_apart = nullptr;
+  double *h_asums = nullptr; // pinned: the dot products of one adjoint sweep
   int64_t fwd_steps = -1, fwd_K = 0;
   // leapfrog: the forward's first kick weight (1/2 right after a sync), and whether it started
   // right after clb_initialize, where the previous half step's <pi^2> is that of the start momenta
@@ -179,7 +180,7 @@ void measure_sums(clb_handle *h)
   else
     CLB_LAUNCH(h, K_MEASURE, k_u1_measure<double><<<kU1Blocks, 256, 0, h->stream>>>(
                                  static_cast<const double *>(u->f), static_cast<const double *>(u->p), u->prm, u->d_part));
-  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kU1Meas><<<1, 256, 0, h->stream>>>(u->d_part, kU1Blocks, u->d_sums));
+  CLB_LAUNCH(h, K_MEASURE, k_sum_partials<kU1Meas><<<1, 512, 0, h->stream>>>(u->d_part, kU1Blocks, u->d_sums));
 }
 
 void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 = 0, int64_t hist_row = -1,
@@ -415,6 +416,9 @@ __attribute__((visibility("hidden"))) int u1_create(clb_handle *h)
   if (const char *env = std::getenv("CLB_U1_TILE")) u->tile_lx = std::atoi(env) == 0 ? 0 : u->tile_lx;
   if (const char *env = std::getenv("CLB_U1_TILE_LX"))
     if (u->tile_lx > 0) u->tile_lx = std::max(1, std::atoi(env));
+  // the adjoint sweep's runs: N / 8 planes (ms of a 10-step VV2 gradient at 8 / 12 / 16 / 32 planes: 64^3
+  // 2.21 / 2.31 / 2.44 / 2.55, 96^3 5.51 / 5.48 / 5.62 / 5.66, 128^3 12.2 / 12.2 / 12.15 / 12.2)
+  u->adj_lx = std::min(16, std::max(4, h->cfg.N / 8));
   if (const char *env = std::getenv("CLB_U1_ADJ_LX")) u->adj_lx = std::max(1, std::atoi(env));
   const size_t bytes = 5 * h->n3 * u->esz;
   bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -444,10 +448,12 @@ static void free_adjoint(U1Sector *u)
   u->seg = nullptr;
   u->d_rec = nullptr;
   u->seg_cap = 0;
-  for (double **b : {&u->qbar, &u->pbar[0], &u->pbar[1], &u->d_apart, &u->d_asums, &u->seed}) {
+  for (double **b : {&u->qbar, &u->pbar[0], &u->pbar[1], &u->d_apart, &u->seed}) {
     if (*b) cudaFree(*b);
     *b = nullptr;
   }
+  if (u->h_asums) cudaFreeHost(u->h_asums);
+  u->h_asums = nullptr;
   u->fwd_steps = -1;
   u->seed_which = -1;
 }
@@ -863,9 +869,10 @@ int adj_sweep(clb_handle *h, const void *f, const void *p, const double *pin, do
     CLB_LAUNCH(h, K_U1_ADJ, adj_launch<float>(h, f, p, pin, pout, g));
   else
     CLB_LAUNCH(h, K_U1_ADJ, adj_launch<double>(h, f, p, pin, pout, g));
-  CLB_LAUNCH(h, K_TAIL, k_sum_partials<kAdjSlots><<<1, 256, 0, h->stream>>>(u->d_apart, kU1Blocks, u->d_asums));
-  cudaError_t e = cudaMemcpyAsync(S, u->d_asums, sizeof(S), cudaMemcpyDeviceToHost, h->stream);
+  CLB_LAUNCH(h, K_TAIL, k_sum_partials<kAdjSlots><<<1, 512, 0, h->stream>>>(u->d_apart, kU1Blocks, u->h_asums));
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  for (int k = 0; k < kAdjSlots; ++k) S[k] = u->h_asums[k];
   return e == cudaSuccess ? CLB_OK : h->cuda_fail(e, "clb_backward");
 }
 
@@ -922,7 +929,7 @@ __attribute__((visibility("hidden"))) int u1_forward(clb_handle *h, int64_t nste
     ok = ok && cudaMalloc(&u->qbar, dbytes) == cudaSuccess && cudaMalloc(&u->pbar[0], dbytes) == cudaSuccess &&
          cudaMalloc(&u->pbar[1], dbytes) == cudaSuccess;
     ok = ok && cudaMalloc(&u->d_apart, (size_t)kU1Blocks * kAdjSlots * sizeof(double)) == cudaSuccess;
-    ok = ok && cudaMalloc(&u->d_asums, kAdjSlots * sizeof(double)) == cudaSuccess;
+    ok = ok && cudaMallocHost(&u->h_asums, kAdjSlots * sizeof(double)) == cudaSuccess;
     if (!ok) {
       free_adjoint(u);
       return h->fail(CLB_ENOMEM, "clb_forward: checkpoint or segment storage does not fit; use a smaller checkpoint_every");
