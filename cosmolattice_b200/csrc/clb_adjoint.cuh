@@ -66,16 +66,15 @@ struct U1Pieces {
 };
 
 // ld(c, site) returns component c at a site as (value, derivative along w).
-template <class LD>
-__device__ __forceinline__ void u1_pieces(LD ld, const U1Params &a, size_t s, const long long (&op)[3],
-                                          const long long (&om)[3], U1Pieces &o)
+template <class LD, class I, class O>
+__device__ __forceinline__ void u1_pieces(LD ld, const U1Params &a, I s, const O (&op)[3], const O (&om)[3], U1Pieces &o)
 {
   const double ndxg = -a.dx * a.gQ;
   const TD fr = ld(0, s), fi = ld(1, s);
   TD pr(0.0), pim(0.0), mr(0.0), mim(0.0);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const size_t sp = s + op[d], sm = s + om[d];
+    const I sp = s + op[d], sm = s + om[d];
     TD ur, ui, vr, vi;
     sincos_t(ndxg * ld(2 + d, s), ui, ur);
     const TD gr = ld(0, sp), gi = ld(1, sp);
@@ -104,7 +103,7 @@ __device__ __forceinline__ void u1_pieces(LD ld, const U1Params &a, size_t s, co
     for (int d = 0; d < 3; ++d) acc = acc + (ld(2 + i, s + op[d]) + ld(2 + i, s + om[d]) - 2.0 * c);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const size_t sij = i == j ? s : s + op[i] + om[j];
+      const I sij = i == j ? s : s + op[i] + om[j];
       acc = acc - ((ld(2 + j, s + op[i]) - ld(2 + j, s)) - (ld(2 + j, sij) - ld(2 + j, s + om[j])));
     }
     o.cc[i] = acc * a.inv_dx2;
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(128, 2)
       cp_async_commit();
     };
     // the JVP direction at ring index y: M^{-1} (hA lambda_A + hB lambda_B), as k_u1_adj's ld
-    auto ld = [&](int c, size_t y) -> TD {
+    auto ld = [&](int c, int y) -> TD {
       const double lA = rL[c * CS + y];
       const int sec = c < 2 ? 0 : 1;
       const double lB = lA + (sec == 0 ? cP : cE) * (double)rP[c * CS + y];
@@ -313,9 +312,8 @@ __global__ void __launch_bounds__(128, 2)
       issue(j + L);
       if (valid) {
         const int sc = j % D, sp = (j + 1) % D, sm = (j - 1) % D;
-        const size_t t = (size_t)sc * PL + (size_t)(ty + 1) * ROW + (size_t)(tz + 1);
-        const long long op[3] = {(long long)(sp - sc) * PL, ROW, 1};
-        const long long om[3] = {(long long)(sm - sc) * PL, -ROW, -1};
+        const int t = sc * PL + (ty + 1) * ROW + tz + 1;
+        const int op[3] = {(sp - sc) * PL, ROW, 1}, om[3] = {(sm - sc) * PL, -ROW, -1};
         const size_t s = ((size_t)x * N + (size_t)(y0 + ty)) * N + (size_t)(z0 + tz);
         U1Pieces o;
         u1_pieces(ld, a, t, op, om, o);

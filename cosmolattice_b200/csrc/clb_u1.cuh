@@ -104,12 +104,12 @@ template <class T> struct U1Site {
   T nrm;               // |phi|
 };
 
-template <bool KERNEL, class S, class T>
-__device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params &a, size_t s,
-                                        const long long (&op)[3], const long long (&om)[3], T kA, T kB2, T kG,
-                                        U1Site<T> &o)
+// I: the type of the indices, size_t for the arrays (n3 apart), int for a ring of staged planes (CS
+// apart), whose 64-bit arithmetic the compiler keeps otherwise.
+template <bool KERNEL, class S, class T, class I, class O>
+__device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params &a, I n3, I s, const O (&op)[3],
+                                        const O (&om)[3], T kA, T kB2, T kG, U1Site<T> &o)
 {
-  const size_t n3 = a.n3;
   const S *phr = f, *phi = f + n3;
   const S *A[3] = {f + 2 * n3, f + 3 * n3, f + 4 * n3};
   const T ndxg = (T)a.ndxg, inv_dx2 = (T)a.inv_dx2, c4 = (T)a.c4;
@@ -119,7 +119,7 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
   T pr = 0, pim = 0, mr = 0, mim = 0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const size_t sp = s + op[d];
+    const I sp = s + op[d];
     T ur, ui;
     u1_sincos(u1_m(ndxg, (T)A[d][s]), &ui, &ur);
     const T gr = (T)phr[sp], gi = (T)phi[sp];
@@ -127,7 +127,7 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
     o.wi[d] = u1_a(u1_m(ur, gi), u1_m(ui, gr));
     if (KERNEL) {
       // conj(U_d(x - d)) phi(x - d)
-      const size_t sm = s + om[d];
+      const I sm = s + om[d];
       T vr, vi;
       u1_sincos(u1_m(ndxg, (T)A[d][sm]), &vi, &vr);
       const T nvi = -vi, hr = (T)phr[sm], hi = (T)phi[sm];
@@ -170,8 +170,8 @@ __device__ __forceinline__ void u1_site(const S *__restrict__ f, const U1Params 
     T grad = 0;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const size_t sj = s + om[j];
-      const size_t sij = i == j ? s : s + op[i] + om[j]; // x + i - j
+      const I sj = s + om[j];
+      const I sij = i == j ? s : s + op[i] + om[j]; // x + i - j
       const T g1 = div_by(u1_s((T)A[j][sij], (T)A[j][sj]), a.ddx);
       const T tj = div_by(u1_s(o.g0[i][j], g1), a.ddx);
       grad = j == 0 ? tj : u1_a(grad, tj);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
     long long op[3], om[3];
     u1_offsets(a.N, s, op, om);
     U1Site<T> o;
-    u1_site<(NK > 0)>(f, a, s, op, om, kA, kB2, kG, o);
+    u1_site<(NK > 0)>(f, a, n3, s, op, om, kA, kB2, kG, o);
     if (RF) {
       acc[2] += (double)u1_cs_grad2(o, a.ddx);
       acc[3] += (double)u1_b2(o);
@@ -320,8 +320,6 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
   using T = typename std::conditional<FAST && sizeof(S) == 8, FD, S>::type;
   const int N = a.N;
   const size_t n3 = a.n3;
-  U1Params av = a;
-  av.n3 = (size_t)RG::CS; // u1_site reads component c of ring index t at ring[c * CS + t]
   griddep_wait();
   griddep_launch();
   const T kA = (T)st->kA, kB2 = (T)st->kB2, kG = (T)st->kG;
@@ -362,11 +360,10 @@ __global__ void __launch_bounds__(256, CLB_U1_KICK_MINB)
       issue(j + L);
       if (valid) {
         const int sc = j % D, sp = (j + 1) % D, sm = (j - 1) % D;
-        const size_t t = (size_t)sc * PL + (size_t)(ty + 1) * ROW + (size_t)(tz + 1);
-        const long long op[3] = {(long long)(sp - sc) * PL, ROW, 1};
-        const long long om[3] = {(long long)(sm - sc) * PL, -ROW, -1};
+        const int t = sc * PL + (ty + 1) * ROW + tz + 1;
+        const int op[3] = {(sp - sc) * PL, ROW, 1}, om[3] = {(sm - sc) * PL, -ROW, -1};
         U1Site<T> o;
-        u1_site<(NK > 0)>(ring, av, t, op, om, kA, kB2, kG, o);
+        u1_site<(NK > 0)>(ring, a, (int)RG::CS, t, op, om, kA, kB2, kG, o);
         if (RF) {
           acc[2] += (double)u1_cs_grad2(o, a.ddx);
           acc[3] += (double)u1_b2(o);
@@ -647,7 +644,7 @@ __global__ void __launch_bounds__(256)
     long long op[3], om[3];
     u1_offsets(a.N, s, op, om);
     U1Site<double> o;
-    u1_site<false>(f, a, s, op, om, 0.0, 0.0, 0.0, o);
+    u1_site<false>(f, a, n3, s, op, om, 0.0, 0.0, 0.0, o);
     const double pr = (double)p[s], pi = (double)p[n3 + s];
     double q[3], l[3];
 #pragma unroll
