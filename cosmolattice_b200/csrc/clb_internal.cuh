@@ -77,6 +77,8 @@ enum TailFlags : uint32_t {
   T_FB_PV_HALF = 1u << 23,   // aIM = aI; aI = fb; aSI = aI              (positionverlet.h:209-216)
   T_FB_ADOT = 1u << 24       // aDotI = fb                               (sync: velocityverlet.h:121)
 };
+// the tails' flags that take the scale-factor kernel of the cached averages at aI
+constexpr uint32_t kTailSF = T_VV_KICK_ONE | T_VV_KICK_HALF | T_LF_SYNC | T_LF_CTOR | T_LF_KICK;
 
 struct TailOp {
   uint32_t flags;

@@ -404,13 +404,15 @@ __device__ __forceinline__ void tail_apply(DevState &s, const TailOp &op, const 
     const double RHS = __dmul_rn(__dmul_rn(apow(s.aI, 2 * p.alpha + 2) / 3., p.fm2), rho);
     s.aDotI = sqrt(RHS);
   }
-  if (fl & T_VV_KICK_ONE) s.aDotI = __dadd_rn(s.aDotSI, __dmul_rn(__dmul_rn(dt / 2, sf_kernel(s, p)), op.w));
+  // the a-kicks of one tail act with the same averages at the same a
+  const double F = fl & kTailSF ? sf_kernel(s, p) : 0.0;
+  if (fl & T_VV_KICK_ONE) s.aDotI = __dadd_rn(s.aDotSI, __dmul_rn(__dmul_rn(dt / 2, F), op.w));
   if (hist && !(fl & T_HIST_EARLY)) write_hist();
-  if (fl & T_LF_SYNC) s.aDotI = __dadd_rn(s.aDotSI, __dmul_rn(dt / 2.0, sf_kernel(s, p)));
-  if (fl & T_LF_CTOR) s.aDotSI = __dsub_rn(s.aDotI, __dmul_rn(dt / 2.0, sf_kernel(s, p)));
+  if (fl & T_LF_SYNC) s.aDotI = __dadd_rn(s.aDotSI, __dmul_rn(dt / 2.0, F));
+  if (fl & T_LF_CTOR) s.aDotSI = __dsub_rn(s.aDotI, __dmul_rn(dt / 2.0, F));
   if (fl & T_LF_KICK) {
     s.aDotSIM = s.aDotSI;
-    s.aDotSI = __dadd_rn(s.aDotSI, __dmul_rn(dt, sf_kernel(s, p)));
+    s.aDotSI = __dadd_rn(s.aDotSI, __dmul_rn(dt, F));
     s.aDotI = (s.aDotSIM + s.aDotSI) / 2.0;
   }
   if (fl & T_LF_DRIFT) {
@@ -418,7 +420,7 @@ __device__ __forceinline__ void tail_apply(DevState &s, const TailOp &op, const 
     s.aI = __dadd_rn(s.aI, __dmul_rn(dt, s.aDotSI));
     s.aSI = (s.aIM + s.aI) / 2.0;
   }
-  if (fl & T_VV_KICK_HALF) s.aDotSI = __dadd_rn(s.aDotI, __dmul_rn(__dmul_rn(dt / 2, sf_kernel(s, p)), op.w2));
+  if (fl & T_VV_KICK_HALF) s.aDotSI = __dadd_rn(s.aDotI, __dmul_rn(__dmul_rn(dt / 2, F), op.w2));
   if (fl & T_VV_DRIFT) {
     s.aIM = s.aI;
     s.aI = __dadd_rn(s.aI, __dmul_rn(__dmul_rn(dt, s.aDotSI), op.w2));
@@ -473,8 +475,13 @@ static __global__ void __launch_bounds__(kTailThreads)
     k_tail(const double *__restrict__ partials, TailOp op, DevState *__restrict__ st, SFParams p)
 {
   __shared__ double smem[(kTailThreads / 32) * kRedSlots];
-  griddep_wait();   // the sweep's partials and state are complete
-  griddep_launch(); // the next sweep may set up its barriers meanwhile
+  __shared__ DevState ss; // read beside the partials, not after their sum
+  griddep_wait();         // the sweep's partials and state are complete
+  griddep_launch();       // the next sweep may set up its barriers meanwhile
+  constexpr int W = sizeof(DevState) / sizeof(double);
+  static_assert(W * sizeof(double) == sizeof(DevState) && W <= 32, "one warp copies the state");
+  if (threadIdx.x < W) reinterpret_cast<double *>(&ss)[threadIdx.x] = reinterpret_cast<const double *>(st)[threadIdx.x];
+  __syncwarp();
 
   double v[kRedSlots] = {0, 0, 0};
   if (op.nblocks > 0) {
@@ -496,7 +503,7 @@ static __global__ void __launch_bounds__(kTailThreads)
     block_reduce<kRedSlots, kTailThreads>(v, smem);
   }
   if (threadIdx.x != 0) return;
-  DevState s = *st;
+  DevState s = ss;
   tail_apply(s, op, p, v[0], v[1], v[2]);
   *st = s;
 }

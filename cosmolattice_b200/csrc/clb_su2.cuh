@@ -216,12 +216,19 @@ __global__ void __launch_bounds__(kTailThreads)
   __shared__ double smem[kRed * W * (kTailGroups + 1)];
   griddep_wait();
   griddep_launch();
+  // the state is read beside the partials, not after their sum
+  constexpr int SW = sizeof(StateT<T>) / sizeof(double);
+  static_assert(SW * sizeof(double) == sizeof(StateT<T>), "whole words");
+  __shared__ double ss[SW];
+  if (threadIdx.x < 32)
+    for (int i = threadIdx.x; i < SW; i += 32) ss[i] = reinterpret_cast<const double *>(stp)[i];
+  __syncwarp();
   double r[kRed * W];
   for (int k = 0; k < kRed * W; ++k) r[k] = 0;
   if (op.nblocks > 0) rows_reduce<kRed * W, kRed * W, kTailGroups>(partials, op.nblocks, smem, r);
   if (threadIdx.x >= 32) return;
   const int lane = (int)threadIdx.x;
-  StateT<T> s = *stp;
+  StateT<T> s = *reinterpret_cast<const StateT<T> *>(ss);
   T v[kRed];
   for (int k = 0; k < kRed; ++k) {
     if constexpr (TanTraits<T>::is)
@@ -264,13 +271,15 @@ __global__ void __launch_bounds__(kTailThreads)
       s.pi2[g] = 0.5 * (s.pi2SIM[g] + s.pi2SI[g]);
     }
   if (fl & T_CORRECT_ADOT) s.aDotI = sqrt(pow(s.aI, 2 * p.alpha + 2) / 3. * p.fm2 * rho_of(s, p));
-  if (fl & T_VV_KICK_ONE) s.aDotI = s.aDotSI + (dt / 2) * sf_kernel(s, p) * op.w;
+  // the a-kicks of one tail act with the same averages at the same a
+  const T F = fl & kTailSF ? sf_kernel(s, p) : T(0.0);
+  if (fl & T_VV_KICK_ONE) s.aDotI = s.aDotSI + (dt / 2) * F * op.w;
   if (hist && !(fl & T_HIST_EARLY)) write_hist();
-  if (fl & T_LF_SYNC) s.aDotI = s.aDotSI + dt / 2.0 * sf_kernel(s, p);
-  if (fl & T_LF_CTOR) s.aDotSI = s.aDotI - dt / 2.0 * sf_kernel(s, p);
+  if (fl & T_LF_SYNC) s.aDotI = s.aDotSI + dt / 2.0 * F;
+  if (fl & T_LF_CTOR) s.aDotSI = s.aDotI - dt / 2.0 * F;
   if (fl & T_LF_KICK) {
     s.aDotSIM = s.aDotSI;
-    s.aDotSI += dt * sf_kernel(s, p);
+    s.aDotSI += dt * F;
     s.aDotI = (s.aDotSIM + s.aDotSI) / 2.0;
   }
   if (fl & T_LF_DRIFT) {
@@ -278,7 +287,7 @@ __global__ void __launch_bounds__(kTailThreads)
     s.aI += dt * s.aDotSI;
     s.aSI = (s.aIM + s.aI) / 2.0;
   }
-  if (fl & T_VV_KICK_HALF) s.aDotSI = s.aDotI + (dt / 2) * sf_kernel(s, p) * op.w2;
+  if (fl & T_VV_KICK_HALF) s.aDotSI = s.aDotI + (dt / 2) * F * op.w2;
   if (fl & T_STORE_PI2_B)
     for (int g = 0; g < 5; ++g) s.pi2[g] = v[11 + g];
   if (fl & T_VV_DRIFT) {

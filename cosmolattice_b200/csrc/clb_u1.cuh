@@ -514,13 +514,15 @@ __device__ __forceinline__ void u1_tail_apply(U1State &s, const double (&v)[kU1R
                             s.potI);
     s.aDotI = sqrt(u1_m(u1_m(pow(s.aI, 2 * p.alpha + 2) / 3., p.fm2), rho));
   }
-  if (fl & T_VV_KICK_ONE) s.aDotI = u1_a(s.aDotSI, u1_m(u1_m(dt / 2, u1_sf_kernel(s, p)), op.w));
+  // the a-kicks of one tail act with the same averages at the same a
+  const double F = fl & kTailSF ? u1_sf_kernel(s, p) : 0.0;
+  if (fl & T_VV_KICK_ONE) s.aDotI = u1_a(s.aDotSI, u1_m(u1_m(dt / 2, F), op.w));
   if (hist && !(fl & T_HIST_EARLY)) write_hist();
-  if (fl & T_LF_SYNC) s.aDotI = u1_a(s.aDotSI, u1_m(dt / 2.0, u1_sf_kernel(s, p)));
-  if (fl & T_LF_CTOR) s.aDotSI = u1_s(s.aDotI, u1_m(dt / 2.0, u1_sf_kernel(s, p)));
+  if (fl & T_LF_SYNC) s.aDotI = u1_a(s.aDotSI, u1_m(dt / 2.0, F));
+  if (fl & T_LF_CTOR) s.aDotSI = u1_s(s.aDotI, u1_m(dt / 2.0, F));
   if (fl & T_LF_KICK) {
     s.aDotSIM = s.aDotSI;
-    s.aDotSI = u1_a(s.aDotSI, u1_m(dt, u1_sf_kernel(s, p)));
+    s.aDotSI = u1_a(s.aDotSI, u1_m(dt, F));
     s.aDotI = (s.aDotSIM + s.aDotSI) / 2.0;
   }
   if (fl & T_LF_DRIFT) {
@@ -528,7 +530,7 @@ __device__ __forceinline__ void u1_tail_apply(U1State &s, const double (&v)[kU1R
     s.aI = u1_a(s.aI, u1_m(dt, s.aDotSI));
     s.aSI = (s.aIM + s.aI) / 2.0;
   }
-  if (fl & T_VV_KICK_HALF) s.aDotSI = u1_a(s.aDotI, u1_m(u1_m(dt / 2, u1_sf_kernel(s, p)), op.w2));
+  if (fl & T_VV_KICK_HALF) s.aDotSI = u1_a(s.aDotI, u1_m(u1_m(dt / 2, F), op.w2));
   if (fl & T_STORE_PI2_B) {
     s.csPi2I = csP2;
     s.u1Pi2I = u1P2;
