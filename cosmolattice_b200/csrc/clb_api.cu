@@ -37,7 +37,7 @@ constexpr uint32_t kWaitTries = 1u << 24; // bound of each mbarrier wait in the 
 constexpr size_t kStageMin = (size_t)1 << 23; // host-transfer staging: >= 64 MiB of doubles
 constexpr int kDefaultShapeFP64 = 0;          // ShapeW
 constexpr int kDefaultShapeFP32 = 4;          // ShapeK
-constexpr int kPlanesPerBlock = 32;           // x-run length of one sweep block
+constexpr int kMaxRun = 22;                   // longest x-run of one sweep block
 
 } // namespace
 
@@ -93,23 +93,32 @@ __attribute__((visibility("hidden"))) void set_global_error(const std::string &m
 namespace {
 
 
-// Sweep geometry: bz x by (z, y) sites per block; the x direction is split so the grid holds about
-// two waves of resident blocks.
+// Sweep geometry: bz x by (z, y) sites per block and x-runs of LX planes.  A block's time goes as its
+// planes plus about one (its prologue and the halo planes), and the grid runs in waves of the resident
+// blocks, so the runs minimise waves x (LX + 0.8); runs longer than 22 planes lose L2 reuse between
+// neighbouring tiles.  us per VV2 step, this rule against runs of two waves of blocks or 32 planes:
+// 125^3 two fields FP64 43.8 against 50.4, 96^3 FP64 17.5 / 20.6, 128^3 FP32 17.5 / 22.1, 192^3
+// two fields FP64 113.9 / 125.4, 384^3 FP32 198.8 / 201.5, 512^3 FP64 798.4 / 803.
 void setup_geometry(clb_handle *h, int blocks_per_sm)
 {
   const int N = h->N;
   const int gx = (N + h->bz - 1) / h->bz, gy = (N + h->by - 1) / h->by;
-  // Many short x-runs (about 32 planes) beat few long ones: a block's plane rate is bounded by its
-  // own pipeline, so throughput comes from many blocks cycling through the SMs.  A small lattice
-  // has few (z, y) tiles (64^3: 8), so its runs are shortened, down to one plane, until the grid
-  // fills two waves of resident blocks (the extra halo planes then come from L2).
-  int xs = std::max(1, (N + kPlanesPerBlock - 1) / kPlanesPerBlock);
-  const int waves = 2 * 148 * std::max(1, blocks_per_sm);
-  if ((long long)gx * gy * xs < waves) xs = std::max(xs, std::min(N, (waves + gx * gy - 1) / (gx * gy)));
-  xs = std::max(1, std::min(xs, N));
-  if (const char *env = std::getenv("CLB_SWEEP_XS")) xs = std::max(1, std::min(N, std::atoi(env)));
-  int LX = (N + xs - 1) / xs;
-  xs = (N + LX - 1) / LX;
+  const long long slots = 148LL * std::max(1, blocks_per_sm), tiles = (long long)gx * gy;
+  int LX = 1;
+  double best = 0;
+  for (int l = std::min(N, kMaxRun); l >= 1; --l) {
+    const long long blocks = tiles * ((N + l - 1) / l);
+    const double cost = (double)((blocks + slots - 1) / slots) * (l + 0.8);
+    if (best == 0 || cost < best) {
+      best = cost;
+      LX = l;
+    }
+  }
+  if (const char *env = std::getenv("CLB_SWEEP_XS")) {
+    const int xs = std::max(1, std::min(N, std::atoi(env)));
+    LX = (N + xs - 1) / xs;
+  }
+  const int xs = (N + LX - 1) / LX;
   h->sa.LX = LX;
   h->sweep_grid = dim3(gx, gy, xs);
   h->sweep_blocks = gx * gy * xs;
@@ -161,6 +170,30 @@ void sweep(clb_handle *h, int kind, int fb, int pb, int fo, int po, double dtw, 
   }
   sweep_sh<R, NS, ShapeW, DRIFT, KICK, RED>(h, kind, fb, pb, fo, po, dtw, h1, h2, dtw0);
 }
+
+// Resident blocks per SM of the fused sweep as the handle launches it.
+template <class R, int NS> struct Occupancy {
+  template <class SH> static int of(const clb_handle *h)
+  {
+    int n = 0;
+    const auto k = k_sweep<R, NS, SH, 1, true, 3>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, SH::THREADS, h->sweep_smem) != cudaSuccess) n = 0;
+    return std::max(1, n);
+  }
+  static void run(clb_handle *h, int *out)
+  {
+    if constexpr (NS == 1) {
+      *out = h->shape == 1   ? of<ShapeQ>(h)
+             : h->shape == 2 ? of<ShapeH>(h)
+             : h->shape == 3 ? of<ShapeL>(h)
+             : h->shape == 4 ? of<ShapeK>(h)
+                             : of<ShapeW>(h);
+    } else {
+      *out = of<ShapeW>(h);
+    }
+  }
+};
 
 template <class R, int NS> struct Launch {
   // kick in place: pi += h K(phi)
@@ -802,11 +835,14 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
   const size_t box_bytes = (size_t)(h->bz + 2 * (16 / (int)h->esz)) * (size_t)(h->by + 2) * h->esz;
   const size_t slot = ((box_bytes + 127) / 128) * 128;
   const size_t stage_bytes = (size_t)h->NS * 2 * slot;
-  size_t ring_budget = 32 * 1024;
+  // two fields: the sweep's registers allow two blocks per SM, which leaves room for a deeper ring
+  // (192^3 FP64 126 -> 121.5 us per step at four stages instead of three)
+  size_t ring_budget = h->NS == 2 ? 96 * 1024 : 32 * 1024;
   if (const char *env = std::getenv("CLB_SWEEP_RING_KB")) ring_budget = (size_t)std::max(8, std::atoi(env)) * 1024;
   h->S = (int)std::max<size_t>(3, std::min<size_t>(8, ring_budget / stage_bytes));
   h->sweep_smem = (size_t)h->S * stage_bytes + (size_t)h->S * sizeof(uint64_t) + 8 * kRedSlots * sizeof(double);
-  const int bpsm = (int)std::max<size_t>(1, std::min<size_t>(8, (220 * 1024) / (h->sweep_smem + 1024)));
+  int bpsm = 1;
+  dispatch<Occupancy>(h, &bpsm);
   setup_geometry(h, bpsm);
   SweepArgs &w = h->sw;
   w.pd = h->pd;
