@@ -714,25 +714,28 @@ __global__ void __launch_bounds__(256)
   const double dtw = lf ? dt : dt * w;
   const size_t n3 = a.n3;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
-    f[s] = (S)((double)f[s] + p3 * (dtw * (double)p[s]));
-    for (int c = 1; c < 3; ++c) f[c * n3 + s] = (S)((double)f[c * n3 + s] + cC * (double)p[c * n3 + s]);
+    S pv[NP]; // all at once: the sweep waits on loads (95^3 FP32 56.0 us against 59.8)
+#pragma unroll
+    for (int c = 0; c < NP; ++c) pv[c] = p[c * n3 + s];
+    f[s] = (S)((double)f[s] + p3 * (dtw * (double)pv[0]));
+    for (int c = 1; c < 3; ++c) f[c * n3 + s] = (S)((double)f[c * n3 + s] + cC * (double)pv[c]);
     {
       S *fd = f + fidx(a, 3, s);
       V4<S> d = ld4(fd);
-      for (int c = 0; c < 4; ++c) d.v[c] = (S)((double)d.v[c] + cC * (double)p[(3 + c) * n3 + s]);
+      for (int c = 0; c < 4; ++c) d.v[c] = (S)((double)d.v[c] + cC * (double)pv[3 + c]);
       st4(fd, d.v[0], d.v[1], d.v[2], d.v[3]);
     }
     for (int i = 0; i < 3; ++i) {
       S *fa = f + fidx(a, 7 + i, s);
-      const S A = (S)((double)*fa + cA * (double)p[(7 + i) * n3 + s] * 1.0);
+      const S A = (S)((double)*fa + cA * (double)pv[7 + i] * 1.0);
       *fa = A;
       put_phases(ph, a, i, s, A);
     }
     for (int i = 0; i < 3; ++i) {
-      const size_t pb = (size_t)(10 + 3 * i) * n3 + s;
+      const S *pu = pv + 10 + 3 * i;
       S *fu = f + fidx(a, 10 + 4 * i, s);
       const V4<S> q = ld4(fu);
-      const Q4<double> E = qexp<S>(cG * (double)p[pb], cG * (double)p[pb + n3], cG * (double)p[pb + 2 * n3]);
+      const Q4<double> E = qexp<S>(cG * (double)pu[0], cG * (double)pu[1], cG * (double)pu[2]);
       const Q4<double> U = qmul(E, Q4<double>{(double)q.v[0], (double)q.v[1], (double)q.v[2], (double)q.v[3]});
       st4(fu, (S)U.w, (S)U.x, (S)U.y, (S)U.z);
     }
