@@ -833,24 +833,24 @@ int clb_batch_get_state(clb_batch *b, int32_t i, double *fields, double *momenta
   if (i < 0 || i >= b->n) return b->fail(CLB_EINVAL, "clb_batch_get_state: member index out of range");
   const BatchLat &L = b->lat[(size_t)i];
   const size_t n3 = (size_t)L.N * L.N * L.N;
-  DevState s;
-  cudaError_t e = cudaMemcpyAsync(b->rb, b->d_st + i, sizeof(s), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  s = *b->rb;
-  for (int w = 0; w < 2 && e == cudaSuccess; ++w) { // the two arrays in stream order, one wait
+  // the state and the two arrays in stream order, one wait
+  cudaError_t e = cudaMemcpyAsync(b->rb, b->d_st + i, sizeof(DevState), cudaMemcpyDeviceToHost, b->stream);
+  for (int w = 0; w < 2 && e == cudaSuccess; ++w) {
     double *dst = w == 0 ? fields : momenta;
     if (!dst) continue;
     const void *src = w == 0 ? b->f[b->cf] : b->p[b->cf];
     if (b->fp32)
       k_batch_unpack<float><<<kPackBlocks, 256, 0, b->stream>>>(static_cast<const float *>(src) + L.off, b->d_stage, n3,
-                                                                w == 0 ? s.ref_phi[b->rs][0] : s.ref_pi[b->rs][0]);
+                                                                w == 0 ? &b->d_st[i].ref_phi[b->rs][0]
+                                                                       : &b->d_st[i].ref_pi[b->rs][0]);
     else
-      k_batch_unpack<double><<<kPackBlocks, 256, 0, b->stream>>>(static_cast<const double *>(src) + L.off, b->d_stage, n3, 0.0);
+      k_batch_unpack<double><<<kPackBlocks, 256, 0, b->stream>>>(static_cast<const double *>(src) + L.off, b->d_stage, n3, nullptr);
     e = cudaMemcpyAsync(dst, b->d_stage, n3 * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "clb_batch_get_state");
   if (sf) {
+    const DevState &s = *b->rb;
     sf->aI = s.aI;
     sf->aSI = s.aSI;
     sf->aIM = s.aIM;

@@ -463,8 +463,10 @@ __global__ void __launch_bounds__(256) k_batch_pack(const double *__restrict__ s
     dst[i] = (R)(src[i] - off);
 }
 template <class R>
-__global__ void __launch_bounds__(256) k_batch_unpack(const R *__restrict__ src, double *__restrict__ dst, size_t n, double off)
+__global__ void __launch_bounds__(256) k_batch_unpack(const R *__restrict__ src, double *__restrict__ dst, size_t n,
+                                                                               const double *ref)
 {
+  const double off = ref ? *ref : 0.0; // the split form's reference, added back
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = off + (double)src[i];
 }
