@@ -303,6 +303,34 @@ template <class Fn> __device__ __forceinline__ void for_sites(int N, size_t n3, 
   }
 }
 
+// for_sites for a block whose threads stand in groups of T: thread t of each group visits the sites
+// that for_sites gives thread t of a block of T.  All of the block's threads make the same number of
+// calls, so fn may hold barriers: fn(s, false) beyond the lattice, with s a site of it all the same.
+template <int T, class Fn> __device__ __forceinline__ void for_sites_grouped(int N, size_t n3, int order, int t, Fn &&fn)
+{
+  if (order == 0) {
+    for (size_t b = (size_t)blockIdx.x * T; b < n3; b += (size_t)gridDim.x * T) {
+      const bool in = b + t < n3;
+      fn(in ? b + t : n3 - 1, in);
+    }
+    return;
+  }
+  constexpr int TY = T / 32;
+  const int ntz = (N + 31) >> 5, nty = (N + TY - 1) / TY, nxr = (N + order - 1) / order;
+  const long long items = (long long)ntz * nty * nxr;
+  const size_t plane = (size_t)N * N;
+  for (long long it = blockIdx.x; it < items; it += gridDim.x) {
+    const int zt = (int)(it % ntz);
+    const long long r = it / ntz;
+    const int yt = (int)(r % nty), xr = (int)(r / nty);
+    const int z = zt * 32 + (t & 31), y = yt * TY + (t >> 5);
+    const bool in = z < N && y < N;
+    const int xa = xr * order, xb = min(N, xa + order);
+    size_t s = (size_t)xa * plane + (size_t)min(y, N - 1) * N + min(z, N - 1);
+    for (int x = xa; x < xb; ++x, s += plane) fn(s, in);
+  }
+}
+
 // Asynchronous global -> shared copies (cp.async, sm_80+): 4, 8 or 16 bytes, both addresses
 // aligned to the size.  A commit closes a group; wait_group<K> returns when at most K of this
 // thread's groups are still in flight.

@@ -127,6 +127,8 @@ template <class T> struct StateT {
 };
 using State = StateT<double>;
 using TState = StateT<Tan<double>>;
+// the state that a kick sweep of arithmetic type T reads
+template <class T> using SweepState = typename std::conditional<TanTraits<T>::is, TState, State>::type;
 
 // Applies fn(x.m, y.m) to every floating member m of two scalar states.
 template <class A, class B, class Fn> inline void zip_state(StateT<A> &x, const StateT<B> &y, Fn fn)

@@ -106,6 +106,7 @@ template <class T> __device__ __forceinline__ T ipw(T x, int n)
 {
   if (n < 0) return T(1) / ipw(x, -n);
   T r = x;
+#pragma unroll
   for (int i = 1; i < n; ++i) r = r * x;
   return n == 0 ? T(1) : r;
 }
@@ -131,28 +132,22 @@ template <class S, class T> struct Site {
       return (T)f[i];
   }
   // the quadruple at index i of the field buffer
-  __device__ __forceinline__ V4<T> quad(size_t i) const
+  __device__ __forceinline__ Q4<T> quad(size_t i) const
   {
     const V4<S> v = ld4c(f + i);
-    V4<T> r;
     if constexpr (TanTraits<T>::is) {
       using B = typename TanTraits<T>::base;
       const V4<S> d = ld4c(df + i);
-      for (int k = 0; k < 4; ++k) r.v[k] = T((B)v.v[k], (B)d.v[k]);
+      return Q4<T>{T((B)v.v[0], (B)d.v[0]), T((B)v.v[1], (B)d.v[1]), T((B)v.v[2], (B)d.v[2]), T((B)v.v[3], (B)d.v[3])};
     } else {
-      for (int k = 0; k < 4; ++k) r.v[k] = (T)v.v[k];
+      return Q4<T>{(T)v.v[0], (T)v.v[1], (T)v.v[2], (T)v.v[3]};
     }
-    return r;
   }
-  __device__ __forceinline__ Q4<T> link(int i, uint32_t t) const
-  {
-    const V4<T> q = quad(fidx(*a, 10 + 4 * i, t));
-    return Q4<T>{q.v[0], q.v[1], q.v[2], q.v[3]};
-  }
+  __device__ __forceinline__ Q4<T> link(int i, uint32_t t) const { return quad(fidx(*a, 10 + 4 * i, t)); }
   __device__ __forceinline__ D2<T> dbl(uint32_t t) const
   {
-    const V4<T> q = quad(fidx(*a, 3, t));
-    return D2<T>{C2<T>{q.v[0], q.v[1]}, C2<T>{q.v[2], q.v[3]}};
+    const Q4<T> q = quad(fidx(*a, 3, t));
+    return D2<T>{C2<T>{q.w, q.x}, C2<T>{q.y, q.z}};
   }
   __device__ __forceinline__ C2<T> cs(uint32_t t) const { return C2<T>{F(1, t), F(2, t)}; }
   // the stored phases when the arithmetic type is the storage type (the same cos and sin of the
@@ -183,10 +178,8 @@ template <class S, class T> struct Site {
   }
   __device__ __forceinline__ T normD(uint32_t t) const
   {
-    const V4<T> d = quad(fidx(*a, 3, t));
-    T q = 0;
-    for (int c = 0; c < 4; ++c) q = c == 0 ? d.v[0] * d.v[0] : q + d.v[c] * d.v[c];
-    return sqrt(q);
+    const Q4<T> d = quad(fidx(*a, 3, t));
+    return sqrt(((d.w * d.w + d.x * d.x) + d.y * d.y) + d.z * d.z);
   }
   __device__ __forceinline__ T normC(uint32_t t) const { return sqrt(F(1, t) * F(1, t) + F(2, t) * F(2, t)); }
   __device__ __forceinline__ T potTerm(int k) const
@@ -211,6 +204,7 @@ template <class S, class T> struct Site {
   {
     const T c = F(comp, s);
     T t[3];
+#pragma unroll
     for (int d = 0; d < 3; ++d) t[d] = (F(comp, pl(d)) + F(comp, mi(d))) - 2 * c;
     return recip<T>(a->ddx2) * ((t[0] + t[1]) + t[2]);
   }
@@ -296,6 +290,7 @@ template <class S, class T> __device__ __forceinline__ T dgrad_term(const Site<S
 template <class S, class T> __device__ __forceinline__ C2<T> covLapC(const Site<S, T> &v, T *g2 = nullptr)
 {
   C2<T> plus{0, 0}, minus{0, 0};
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
     const C2<T> w = cmul(v.phaseC(d, v.s), v.cs(v.pl(d)));
     if (g2) {
@@ -314,6 +309,7 @@ template <class S, class T> __device__ __forceinline__ C2<T> covLapC(const Site<
 template <class S, class T> __device__ __forceinline__ void covLapD(const Site<S, T> &v, T out[4], T *g2 = nullptr)
 {
   D2<T> plus{}, minus{};
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
     const D2<T> w = qapply(v.link(d, v.s), dscale(v.phaseD(d, v.s), v.dbl(v.pl(d))));
     if (g2) {
@@ -376,6 +372,17 @@ template <class S, class T> __device__ __forceinline__ T sGrad2(const Site<S, T>
 template <class S, class T> __device__ __forceinline__ T aB2(const Site<S, T> &v, const T (*g)[3] = nullptr);
 template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v, const T *pw = nullptr);
 
+// (1/dx)^3 / gS; the tangent form's gS can carry a derivative
+template <class S, class T> __device__ __forceinline__ T su2_ngrad(const Site<S, T> &v)
+{
+  if constexpr (std::is_same<T, double>::value)
+    return v.a->ngrad;
+  else if constexpr (std::is_same<T, float>::value)
+    return v.a->ngrad_f;
+  else
+    return kdiv(T(ipw(recip<T>(v.a->ddx), 3)), v.gS);
+}
+
 // AVG: also form the SiteAvg terms of the sectors in SECT into *av, from the covariant products,
 // differences and plaquettes the kernels form anyway.
 template <int SECT = 0, bool AVG = false, class S, class T>
@@ -399,8 +406,10 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
       T dl[4];
       covLapD(v, dl, AVG ? &av->g2D : nullptr);
       const T ndD = c4 * (4 * ipw(nD, 3)) + nD * (2 * qG * ipw(Sv, 2) + 4 * qH * ipw(nC, 2));
-      const V4<T> d = v.quad(fidx(a, 3, s));
-      for (int c = 0; c < 4; ++c) K[3 + c] = A * dl[c] - B2 * (kdiv(ndD, nD) * d.v[c]);
+      const Q4<T> d = v.quad(fidx(a, 3, s));
+      const T dv[4] = {d.w, d.x, d.y, d.z};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) K[3 + c] = A * dl[c] - B2 * (kdiv(ndD, nD) * dv[c]);
     }
     if constexpr (AVG && sect_sphi(SECT)) {
       av->g2S = sGrad2(v);
@@ -411,9 +420,11 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
     const D2<T> D0 = v.dbl(s);
     const C2<T> C0 = v.cs(s);
     T g0s[3][3]; // g0s[i][j]: forward difference of A_j along i
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       const T lap = v.lapl(7 + i);
       T grad = 0;
+#pragma unroll
       for (int j = 0; j < 3; ++j) {
         const T g0 = v.fd(7 + j, s, v.pl(i));
         g0s[i][j] = g0;
@@ -430,24 +441,20 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
   }
   if constexpr (sect_su2(SECT)) {
     const D2<T> Dg = v.dbl(s);
-    T ngrad; // (1/dx)^3 / gS; the tangent form's gS can carry a derivative
-    if constexpr (std::is_same<T, double>::value)
-      ngrad = a.ngrad;
-    else if constexpr (std::is_same<T, float>::value)
-      ngrad = a.ngrad_f;
-    else
-      ngrad = kdiv(T(ipw(recip<T>(a.ddx), 3)), v.gS);
-    const T normGrad = ngrad * G;
+    const T normGrad = su2_ngrad(v) * G;
     const T normSrc = recip<T>(a.ddx) * A;
     T pw[3]; // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       T gr[3] = {0, 0, 0}, gb[3] = {0, 0, 0};
       bool first = true;
+#pragma unroll
       for (int j = 0; j < 3; ++j) {
         if (j == i) continue;
         const Q4<T> P = v.plaq(i, j), Pb = v.plaqBack(i, j);
         if (j < i) pw[i + j - 1] = P.w;
         const T pv[3] = {P.x, P.y, P.z}, bv[3] = {Pb.x, Pb.y, Pb.z};
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
           gr[c] = first ? pv[c] : gr[c] + pv[c];
           gb[c] = first ? bv[c] : gb[c] + bv[c];
@@ -455,6 +462,7 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
         first = false;
       }
       const D2<T> W = v.wD(i);
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
         const T J = rfo2 / 2 * (v.gS * sprod(W, isig(c, Dg)).re);
         K[10 + 3 * i + c] = -normGrad * (gr[c] - gb[c]) - normSrc * J;
@@ -468,6 +476,7 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
 template <class S, class T> __device__ __forceinline__ T sGrad2(const Site<S, T> &v)
 {
   T acc = 0;
+#pragma unroll
   for (int j = 0; j < 3; ++j) {
     const T g = v.fd(0, v.s, v.pl(j));
     acc = j == 0 ? g * g : acc + g * g;
@@ -478,6 +487,7 @@ template <class S, class T> __device__ __forceinline__ T cGrad2(const Site<S, T>
 {
   const C2<T> c = v.cs(v.s);
   T acc = 0;
+#pragma unroll
   for (int j = 0; j < 3; ++j) {
     const T n2 = cgrad_term(v, v.wC(j), c);
     acc = j == 0 ? n2 : acc + n2;
@@ -488,6 +498,7 @@ template <class S, class T> __device__ __forceinline__ T dGrad2(const Site<S, T>
 {
   const D2<T> c = v.dbl(v.s);
   T acc = 0;
+#pragma unroll
   for (int j = 0; j < 3; ++j) {
     const T n2 = dgrad_term(v, qapply(v.link(j, v.s), dscale(v.phaseD(j, v.s), v.dbl(v.pl(j)))), c);
     acc = j == 0 ? n2 : acc + n2;
@@ -542,8 +553,10 @@ template <int G0 = 0, int G1 = 5, class R> __device__ __forceinline__ void pi2s(
   if (G0 <= 3 && G1 > 3) out[3] = (q[7] * q[7] + q[8] * q[8]) + q[9] * q[9];
   if (G1 == 5) {
     double acc = 0;
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       double ai = 0;
+#pragma unroll
       for (int b = 0; b < 3; ++b) {
         const double e = q[10 + 3 * i + b];
         ai = b == 0 ? 4 * (e * e) : ai + 4 * (e * e);
@@ -568,14 +581,11 @@ __device__ __forceinline__ int sector(int c) { return c == 0 ? 0 : c < 3 ? 1 : c
 #ifndef CLB_SU2_KICK_MINB_F64
 #define CLB_SU2_KICK_MINB_F64 3
 #endif
-// SECT (as kernels()): 0 every sector in one sweep; 1 and 2 the two halves of a split sweep, or
-// 3, 4 and 2 the three parts of a three-way split, run one after the other over the same grid.
-// Each part updates, reduces and writes only its own components and partial slots (1: sectors S,
-// phi, Phi, A, the field sums but <B^2> of SU(2); 2: the SU(2) sector and its <B^2>; 3: sectors
-// S, phi, Phi, their gradient sums and <V>; 4: sector A and its <B^2>), so the parts hold fewer
-// registers than the whole.  The kicks read the fields only, so the parts' order is free.
-// The halves of a split sweep (192^3, ms per step, same call): FP64 8.17 whole, 6.23 halves at
-// three blocks, 5.73 at four; FP32 4.66 whole, 3.31 halves at four blocks, 3.64 at five.
+// SECT (as kernels()): 0 every sector in one sweep; else a part of a split sweep, run one after the
+// other over the same grid: 1 in halves, 3 and 4 in three parts, 5, 6 and 4 in four, each with the SU(2)
+// part (k_kick_links).  Each part updates, reduces and writes only its own components and partial slots
+// (sect_owns), so the parts hold fewer registers than the whole.  The kicks read the fields only, so
+// the parts' order is free.  Four blocks per SM timed best for the parts, FP64 and FP32.
 #ifndef CLB_SU2_HALF_MINB_F32
 #define CLB_SU2_HALF_MINB_F32 4
 #endif
@@ -615,28 +625,35 @@ __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_K
   griddep_launch();
   const State st = *stp;
   double acc[kRed];
+#pragma unroll
   for (int k = 0; k < kRed; ++k) acc[k] = 0;
   for_sites(a.N, a.n3, a.order, [&](uint32_t s) {
     Site<S, S> v = make_site<S, S>(f, a, s);
     v.ph = ph;
     S q[NP];
+#pragma unroll
     for (int c = C0; c < C1; ++c) q[c] = p[(size_t)c * a.n3 + s];
     SiteAvg<S> av; // with RF: formed by kernels() when the sweep kicks, else by site_avg()
     if (NK > 0) {
       S K[NP];
       kernels<SECT, RF>(v, Coef<S>{(S)st.kA, (S)st.kB, (S)st.kB2, (S)st.kG}, K, &av);
+#pragma unroll
       for (int k = 0; k < NK; ++k) {
+#pragma unroll
         for (int c = C0; c < C1; ++c) q[c] = (S)((double)q[c] + kc.h[k][sector(c)] * (double)K[c]);
         if (RP) {
           double t[5];
           pi2s<G0, G1>(q, t);
+#pragma unroll
           for (int g = G0; g < G1; ++g) acc[(k == 0 ? 0 : 11) + g] += t[g];
         }
       }
+#pragma unroll
       for (int c = C0; c < C1; ++c) p[(size_t)c * a.n3 + s] = q[c];
     } else if (RP) {
       double t[5];
       pi2s<G0, G1>(q, t);
+#pragma unroll
       for (int g = G0; g < G1; ++g) acc[g] += t[g];
     }
     if (RF && NK == 0) av = site_avg<SECT>(v);
@@ -654,6 +671,7 @@ __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_K
   if (RF || RP) {
     block_reduce<kRed, 128>(acc, smem);
     if (threadIdx.x == 0)
+#pragma unroll
       for (int k = 0; k < kRed; ++k)
         if (sect_owns(SECT, k)) partials[(size_t)blockIdx.x * kRed + k] = acc[k];
   }
@@ -880,6 +898,7 @@ template <int G0 = 0, int G1 = 5, class R> __device__ __forceinline__ void pi2s_
   if (G0 <= 3 && G1 > 3) out[3] = 2 * ((q[7] * d[7] + q[8] * d[8]) + q[9] * d[9]);
   if (G1 == 5) {
     double acc = 0;
+#pragma unroll
     for (int c = 10; c < NP; ++c) acc += 8 * (q[c] * d[c]);
     out[4] = acc;
   }
@@ -887,7 +906,10 @@ template <int G0 = 0, int G1 = 5, class R> __device__ __forceinline__ void pi2s_
 
 // Tangent kick sweep: k_kick on (p, dp) with kernels and field sums in Tan<S>; partials
 // [block][2 kRed]: the kRed sums of k_kick, then their tangents.
-// SECT as k_kick: 0 whole; 1 and 2 the halves, or 3, 4 and 2 the three parts, of a split sweep.
+// The parameters are grid constants and the loops over components unrolled, here and in kernels(): the
+// compiler otherwise kept a copy of the parameters and the components' arrays in local memory (944 bytes
+// a thread in the A part, 80 now; FP32 80^3 391 us per tangent step before, 370 with it).
+// SECT as k_kick; the SU(2) part 2 runs here in FP32 only (k_kick_links).
 // Resident blocks per SM of the tangent kick parts: four in FP32, in FP64 three, and four for the S
 // and phi part and the Phi part.  80^3, us per launch at 2 / 3 / 4 blocks: FP64 S and phi 84 / 77 /
 // 58, Phi 122 / 109 / 104, A 142 / 127 / 132, SU(2) 366 / 374 / 371; FP32 tangent step 567 / 509 /
@@ -905,8 +927,8 @@ template <class S, int NK, bool RF, bool RP, int SECT = 0>
 __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_MINB_F32
                                        : SECT == 5 || SECT == 6 ? CLB_SU2_TAN_P56_MINB_F64
                                                                 : CLB_SU2_TAN_MINB_F64)
-    k_kick_tan(const S *__restrict__ f, const S *__restrict__ df, S *__restrict__ p, S *__restrict__ dp, Params a,
-               Kick kc, const TState *__restrict__ stp, CoupDot cd, double *__restrict__ partials)
+    k_kick_tan(const S *__restrict__ f, const S *__restrict__ df, S *__restrict__ p, S *__restrict__ dp, const __grid_constant__ Params a,
+               const __grid_constant__ Kick kc, const TState *__restrict__ stp, const __grid_constant__ CoupDot cd, double *__restrict__ partials)
 {
   using T = Tan<S>;
   constexpr int G0 = sect_g0(SECT), G1 = sect_g1(SECT);                   // sectors [G0, G1)
@@ -916,10 +938,12 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
   griddep_launch();
   const Coef<T> C{T(stp->kA), T(stp->kB), T(stp->kB2), T(stp->kG)};
   double acc[2 * kRed];
+#pragma unroll
   for (int k = 0; k < 2 * kRed; ++k) acc[k] = 0;
   for_sites(a.N, a.n3, a.order, [&](uint32_t s) {
     const Site<S, T> v = make_site_tan<S>(f, df, a, s, cd);
     S q[NP], dq[NP];
+#pragma unroll
     for (int c = C0; c < C1; ++c) {
       q[c] = p[(size_t)c * a.n3 + s];
       dq[c] = dp[(size_t)c * a.n3 + s];
@@ -928,6 +952,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
       double t[5], td[5];
       pi2s<G0, G1>(q, t);
       pi2s_tan<G0, G1>(q, dq, td);
+#pragma unroll
       for (int g = G0; g < G1; ++g) {
         acc[base + g] += t[g];
         acc[kRed + base + g] += td[g];
@@ -937,7 +962,9 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
     if (NK > 0) {
       T K[NP];
       kernels<SECT, RF>(v, C, K, &av);
+#pragma unroll
       for (int k = 0; k < NK; ++k) {
+#pragma unroll
         for (int c = C0; c < C1; ++c) {
           const double h = kc.h[k][sector(c)];
           q[c] = (S)((double)q[c] + h * (double)K[c].v);
@@ -945,6 +972,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
         }
         if (RP) add_pi(k == 0 ? 0 : 11);
       }
+#pragma unroll
       for (int c = C0; c < C1; ++c) {
         p[(size_t)c * a.n3 + s] = q[c];
         dp[(size_t)c * a.n3 + s] = dq[c];
@@ -971,8 +999,170 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
   if (RF || RP) {
     block_reduce<2 * kRed, 128>(acc, smem);
     if (threadIdx.x == 0)
+#pragma unroll
       for (int k = 0; k < 2 * kRed; ++k) // value and tangent slots alike
         if (sect_owns(SECT, k % kRed)) partials[(size_t)blockIdx.x * 2 * kRed + k] = acc[k];
+  }
+}
+
+// The SU(2) part of a split kick sweep, plain (T = S) or tangent-linear (T = Tan<S>, FP64): thread
+// d * 128 + t takes direction d of the site that thread t of a 128-thread block of k_kick or k_kick_tan
+// takes, with the same arithmetic; direction 0 adds up the site's sums in the same order, so partials
+// are the same bits.  One thread per site ran 2300 instructions with few loads in flight at 16 warps per
+// SM (37 % of issue, DRAM at 30 %); a third of them per thread, in one copy for all directions, needs
+// fewer registers: 24 warps in FP64, 36 in FP32.  Whole steps, us: FP64 192^3 3068 against 3512, 95^3 418
+// against 466, 128^3 915 against 1046, 48^3 74 against 88; FP32 95^3 284 against 323, 48^3 54.6 against
+// 65.3.  Tangent FP64 80^3 734 against 848, 40^3 167 against 212 (with the loops of kernels() unrolled).
+// The FP32 tangent form stays with one thread per site: 80^3 370 us against 438 at two blocks per SM
+// here and 476 at one.
+#ifndef CLB_SU2_DIR_MINB_F64
+#define CLB_SU2_DIR_MINB_F64 2
+#endif
+#ifndef CLB_SU2_DIR_MINB_F32
+#define CLB_SU2_DIR_MINB_F32 3
+#endif
+template <class S, class T, int NK, bool RF, bool RP>
+__global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8 ? CLB_SU2_DIR_MINB_F64 : CLB_SU2_DIR_MINB_F32)
+    k_kick_links(const S *__restrict__ f, const S *__restrict__ df, S *__restrict__ p, S *__restrict__ dp, const __grid_constant__ Params a,
+                 const __grid_constant__ Kick kc, const SweepState<T> *__restrict__ stp, const __grid_constant__ CoupDot cd, double *__restrict__ partials,
+                 const S *__restrict__ ph)
+{
+  constexpr bool TAN = TanTraits<T>::is;
+  constexpr int W = TAN ? 2 : 1;
+  __shared__ double smem[(3 * 128 / 32) * 3 * W];
+  __shared__ double xe[2][NK][2][128];                        // pi^2 of directions 1 and 2 after each kick
+  __shared__ double xd[TAN ? 2 : 1][NK][2][3][TAN ? 128 : 1]; // the terms of its tangent
+  __shared__ T xw[2][3][128];                                 // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
+  const int d = threadIdx.x / 128, t = threadIdx.x % 128;
+  const int j1 = d == 0 ? 1 : 0, j2 = d == 2 ? 1 : 2; // the other directions, ascending
+  const size_t U = a.oU + (size_t)d * 4 * a.n3, U1 = a.oU + (size_t)j1 * 4 * a.n3, U2 = a.oU + (size_t)j2 * 4 * a.n3;
+  const size_t pc = (size_t)(10 + 3 * d) * a.n3;
+  const uint32_t N = a.divN.d;
+  auto stride = [&](int k) { return k == 0 ? N * N : k == 1 ? N : 1u; };
+  const uint32_t sd = stride(d), s1 = stride(j1), s2 = stride(j2);
+  griddep_wait();
+  griddep_launch();
+  const T A = T(stp->kA), G = T(stp->kG);
+  const typename TanTraits<T>::base rfo2 = (typename TanTraits<T>::base)a.rfo2;
+  double acc[3 * W]; // pi^2 after the first kick, <B^2>, pi^2 after the second; then their tangents
+#pragma unroll
+  for (int k = 0; k < 3 * W; ++k) acc[k] = 0;
+  int buf = 0;
+  for_sites_grouped<128>(a.N, a.n3, a.order, t, [&](size_t site, bool in) {
+    const uint32_t s = (uint32_t)site;
+    Site<S, T> v;
+    if constexpr (TAN)
+      v = make_site_tan<S>(f, df, a, s, cd);
+    else
+      v = make_site<S, S>(f, a, s);
+    v.ph = ph;
+    // as site_offsets, of this thread's three directions
+    const uint32_t xy = fast_div(s, a.divN), x = fast_div(xy, a.divN), y = xy - x * N, z = s - xy * N;
+    auto next = [&](int k, uint32_t st) { return (k == 0 ? x : k == 1 ? y : z) + 1 == N ? 0u - (N - 1) * st : st; };
+    auto prev = [&](int k, uint32_t st) { return (k == 0 ? x : k == 1 ? y : z) == 0 ? (N - 1) * st : 0u - st; };
+    const uint32_t op = next(d, sd), o1 = next(j1, s1), o2 = next(j2, s2), m1 = prev(j1, s1), m2 = prev(j2, s2);
+    auto at = [&](size_t base, uint32_t r) { return v.quad(base + 4 * (size_t)r); };
+    S q[3], dq[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      q[c] = p[pc + c * a.n3 + s];
+      if (TAN) dq[c] = dp[pc + c * a.n3 + s];
+    }
+    const Q4<T> Ud = at(U, s);
+    auto plaq = [&](size_t Uj, uint32_t oj) {
+      return qmul(qmul(qmul(Ud, at(Uj, s + op)), qdag(at(U, s + oj))), qdag(at(Uj, s)));
+    };
+    auto plaqBack = [&](size_t Uj, uint32_t mj) {
+      return qdag(qmul(qmul(qmul(Ud, qdag(at(Uj, s + op + mj))), qdag(at(U, s + mj))), at(Uj, s + mj)));
+    };
+    T gr[3], gb[3], pw1, pw2;
+    {
+      const Q4<T> P = plaq(U1, o1), B = plaqBack(U1, m1);
+      gr[0] = P.x, gr[1] = P.y, gr[2] = P.z, pw1 = P.w;
+      gb[0] = B.x, gb[1] = B.y, gb[2] = B.z;
+    }
+    {
+      const Q4<T> P = plaq(U2, o2), B = plaqBack(U2, m2);
+      gr[0] = gr[0] + P.x, gr[1] = gr[1] + P.y, gr[2] = gr[2] + P.z, pw2 = P.w;
+      gb[0] = gb[0] + B.x, gb[1] = gb[1] + B.y, gb[2] = gb[2] + B.z;
+    }
+    const T normGrad = su2_ngrad(v) * G, normSrc = recip<T>(a.ddx) * A;
+    const D2<T> Dg = v.dbl(s), Wd = dscale(v.phaseD(d, s), qapply(Ud, v.dbl(s + op)));
+    double e[NK], ed[NK][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T J = rfo2 / 2 * (v.gS * sprod(Wd, isig(c, Dg)).re);
+      const T K = -normGrad * (gr[c] - gb[c]) - normSrc * J;
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        const double h = kc.h[k][4];
+        if constexpr (TAN) {
+          q[c] = (S)((double)q[c] + h * (double)K.v);
+          dq[c] = (S)((double)dq[c] + h * (double)K.d);
+          ed[k][c] = 8 * ((double)q[c] * (double)dq[c]);
+        } else {
+          q[c] = (S)((double)q[c] + h * (double)K);
+        }
+        const double e2 = 4 * ((double)q[c] * (double)q[c]);
+        e[k] = c == 0 ? e2 : e[k] + e2;
+      }
+    }
+    if (in)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        p[pc + c * a.n3 + s] = q[c];
+        if (TAN) dp[pc + c * a.n3 + s] = dq[c];
+      }
+    if (RP || RF) {
+      if (d > 0) {
+        if (RP)
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            xe[buf][k][d - 1][t] = e[k];
+            if (TAN)
+#pragma unroll
+              for (int c = 0; c < 3; ++c) xd[buf][k][d - 1][c][t] = ed[k][c];
+          }
+        if (RF) xw[buf][d - 1][t] = pw1;
+        if (RF && d == 2) xw[buf][2][t] = pw2;
+      }
+      __syncthreads(); // the next site's values go to the other buffer
+      if (d == 0 && in) {
+        if (RP)
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            acc[2 * k] += (e[k] + xe[buf][k][0][t]) + xe[buf][k][1][t];
+            if constexpr (TAN) {
+              double td = (ed[k][0] + ed[k][1]) + ed[k][2];
+#pragma unroll
+              for (int m = 0; m < 6; ++m) td += xd[buf][k][m / 3][m % 3][t];
+              acc[3 + 2 * k] += td;
+            }
+          }
+        if (RF) {
+          const T pw[3] = {xw[buf][0][t], xw[buf][1][t], xw[buf][2][t]};
+          const T b2 = gB2(v, pw);
+          if constexpr (TAN) {
+            acc[1] += (double)b2.v;
+            acc[4] += (double)b2.d;
+          } else {
+            acc[1] += (double)b2;
+          }
+        }
+      }
+      buf ^= 1;
+    }
+  });
+  if (RF || RP) {
+    block_reduce<3 * W, 128>(acc, smem); // direction 0's four warps
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        double *row = partials + ((size_t)blockIdx.x * W + w) * kRed;
+        row[4] = acc[3 * w];
+        row[9] = acc[3 * w + 1];
+        row[15] = acc[3 * w + 2];
+      }
   }
 }
 
@@ -1035,6 +1225,7 @@ __global__ void __launch_bounds__(256)
   auto ld4t = [&](size_t i) {
     const V4<S> v = ld4(f + i), d = ld4(df + i);
     V4<T> r;
+#pragma unroll
     for (int k = 0; k < 4; ++k) r.v[k] = T((double)v.v[k], (double)d.v[k]);
     return r;
   };
@@ -1044,17 +1235,21 @@ __global__ void __launch_bounds__(256)
   };
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
     put(f, df, s, ld(f, df, s) + p3 * (dtw * ld(p, dp, s)));
+#pragma unroll
     for (int c = 1; c < 3; ++c) put(f, df, c * n3 + s, ld(f, df, c * n3 + s) + cC * ld(p, dp, c * n3 + s));
     {
       const size_t fb = fidx(a, 3, s);
       V4<T> d = ld4t(fb);
+#pragma unroll
       for (int c = 0; c < 4; ++c) d.v[c] = d.v[c] + cC * ld(p, dp, (3 + c) * n3 + s);
       put4(fb, d.v[0], d.v[1], d.v[2], d.v[3]);
     }
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       const size_t fa = fidx(a, 7 + i, s);
       put(f, df, fa, ld(f, df, fa) + cA * ld(p, dp, (7 + i) * n3 + s) * 1.0);
     }
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       const size_t pb = (size_t)(10 + 3 * i) * n3 + s, fb = fidx(a, 10 + 4 * i, s);
       const V4<T> q = ld4t(fb);
@@ -1073,8 +1268,10 @@ template <class S> __global__ void __launch_bounds__(256) k_unitarize_tan(S *__r
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < 3 * n3; s += (size_t)gridDim.x * blockDim.x) {
     const V4<S> v = ld4(f + a.oU + 4 * s), d = ld4(df + a.oU + 4 * s);
     T q[4], u[4];
+#pragma unroll
     for (int c = 0; c < 4; ++c) q[c] = T((double)v.v[c], (double)d.v[c]);
     const T r = 1.0 / sqrt(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
+#pragma unroll
     for (int c = 0; c < 4; ++c) u[c] = q[c] * r;
     st4(f + a.oU + 4 * s, (S)u[0].v, (S)u[1].v, (S)u[2].v, (S)u[3].v);
     st4(df + a.oU + 4 * s, (S)u[0].d, (S)u[1].d, (S)u[2].d, (S)u[3].d);

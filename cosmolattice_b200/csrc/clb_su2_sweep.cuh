@@ -23,11 +23,13 @@ struct SU2Sector {
   void *ph = nullptr;        // U(1) link phases (6 x N^3 pairs, storage type), kept by the drifts
   // kick sweeps: 0 one sweep, 1 two halves, 2 three parts, 3 four parts (S and phi; Phi; A; SU(2))
   // (CLB_SU2_SPLIT sets both forms).  su2_create takes four parts in FP64 and three in FP32, by
-  // timing at 384^3 VV2 since the kick forms the field averages from its own products (ms per
-  // step): FP64 83.0 whole, 58.3 halves, 45.2 three parts, 40.9 four parts; FP32 44.0, 26.9, 23.3,
-  // 23.3 (at 192^3: FP64 9.20, 6.53, 5.10, 4.73; FP32 4.93, 3.18, 2.90, 2.93).  The tangent-linear
-  // sweep takes four parts in both (256^3 VV2, ms per tangent step, three / four parts: FP64 37.9,
-  // 31.4; FP32 21.5, 19.5).  Every form gives the same state to the last bit.
+  // timing at 192^3 VV2, when every part still had a thread per site and the fields were one array
+  // per component (ms per step): FP64 9.20 whole, 6.53 halves, 5.10 three parts, 4.73 four parts;
+  // FP32 4.93, 3.18, 2.90, 2.93.  The tangent-linear sweep takes four parts in both (256^3 VV2, ms
+  // per tangent step, three / four parts: FP64 37.9, 31.4; FP32 21.5, 19.5).  The SU(2) part has a
+  // thread per site and direction (k_kick_links; the FP32 tangent form one per site), with which the
+  // four parts take 3.07 ms at 192^3 FP64 and the three parts 2.13 in FP32.  Every form gives the
+  // same state to the last bit.
   int split = 2;
   int tan_split = 3;
   int64_t steps_since_unitarize = 0;

@@ -11,27 +11,34 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
   const int kind = nk == 0 ? K_U1_REDUCE : K_U1_KICK;
   const S *f = static_cast<const S *>(u->f);
   S *p = static_cast<S *>(u->p);
-  // kick sweeps run as two halves (sectors S, phi, Phi, A; then SU(2)) or three parts (S, phi, Phi;
-  // A; SU(2)), which hold fewer registers than one sweep over every sector; reduction-only sweeps
-  // run whole
+  // kick sweeps run as two halves (sectors S, phi, Phi, A; then SU(2)), three parts (S, phi, Phi; A;
+  // SU(2)) or four (S, phi; Phi; A; SU(2)), which hold fewer registers than one sweep over every sector;
+  // reduction-only sweeps run whole
 #define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
   CLB_LAUNCH(h, kind,                                                                                                   \
              launch_pdl(k_kick<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, p, u->prm, kc,       \
                         (const State *)u->d_st, u->d_part, static_cast<const S *>(u->ph)))
+#define CLB_SU2KL(NK, RF, RP)                                                                                          \
+  CLB_LAUNCH(h, kind,                                                                                                  \
+             launch_pdl(k_kick_links<S, S, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f,              \
+                        (const S *)nullptr, p, (S *)nullptr, u->prm, kc, (const State *)u->d_st, CoupDot{}, u->d_part, \
+                        static_cast<const S *>(u->ph)))
 #define CLB_SU2K(NK, RF, RP)                                                                                            \
   do {                                                                                                                 \
-    if (NK > 0 && u->split == 3) {                                                                                     \
-      CLB_SU2K1(NK, RF, RP, 5);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 6);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->split == 2) {                                                                              \
-      CLB_SU2K1(NK, RF, RP, 3);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->split) {                                                                                   \
-      CLB_SU2K1(NK, RF, RP, 1);                                                                                        \
-      CLB_SU2K1(NK, RF, RP, 2);                                                                                        \
+    if constexpr (NK > 0) {                                                                                            \
+      if (u->split == 3) {                                                                                             \
+        CLB_SU2K1(NK, RF, RP, 5);                                                                                      \
+        CLB_SU2K1(NK, RF, RP, 6);                                                                                      \
+        CLB_SU2K1(NK, RF, RP, 4);                                                                                      \
+      } else if (u->split == 2) {                                                                                      \
+        CLB_SU2K1(NK, RF, RP, 3);                                                                                      \
+        CLB_SU2K1(NK, RF, RP, 4);                                                                                      \
+      } else if (u->split) {                                                                                           \
+        CLB_SU2K1(NK, RF, RP, 1);                                                                                      \
+      } else {                                                                                                         \
+        CLB_SU2K1(NK, RF, RP, 0);                                                                                      \
+      }                                                                                                                \
+      if (u->split) CLB_SU2KL(NK, RF, RP);                                                                             \
     } else {                                                                                                           \
       CLB_SU2K1(NK, RF, RP, 0);                                                                                        \
     }                                                                                                                  \
@@ -57,6 +64,7 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
       CLB_SU2K(2, false, false);
   }
 #undef CLB_SU2K
+#undef CLB_SU2KL
 #undef CLB_SU2K1
 }
 
@@ -70,20 +78,31 @@ template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, c
   CLB_LAUNCH(h, kind,                                                                                                   \
              launch_pdl(k_kick_tan<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, df, p, dp,       \
                         u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart))
+#define CLB_SU2TL(NK, RF, RP)                                                                                          \
+  do {                                                                                                                 \
+    if constexpr (sizeof(S) == sizeof(double))                                                                         \
+      CLB_LAUNCH(h, kind,                                                                                              \
+                 launch_pdl(k_kick_links<S, Tan<S>, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f, df, \
+                            p, dp, u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart, (const S *)nullptr));  \
+    else                                                                                                               \
+      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
+  } while (0)
 #define CLB_SU2T(NK, RF, RP)                                                                                            \
   do {                                                                                                                 \
-    if (NK > 0 && u->tan_split == 3) {                                                                                 \
-      CLB_SU2T1(NK, RF, RP, 5);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 6);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->tan_split == 2) {                                                                          \
-      CLB_SU2T1(NK, RF, RP, 3);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 4);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
-    } else if (NK > 0 && u->tan_split) {                                                                               \
-      CLB_SU2T1(NK, RF, RP, 1);                                                                                        \
-      CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
+    if constexpr (NK > 0) {                                                                                            \
+      if (u->tan_split == 3) {                                                                                         \
+        CLB_SU2T1(NK, RF, RP, 5);                                                                                      \
+        CLB_SU2T1(NK, RF, RP, 6);                                                                                      \
+        CLB_SU2T1(NK, RF, RP, 4);                                                                                      \
+      } else if (u->tan_split == 2) {                                                                                  \
+        CLB_SU2T1(NK, RF, RP, 3);                                                                                      \
+        CLB_SU2T1(NK, RF, RP, 4);                                                                                      \
+      } else if (u->tan_split) {                                                                                       \
+        CLB_SU2T1(NK, RF, RP, 1);                                                                                      \
+      } else {                                                                                                         \
+        CLB_SU2T1(NK, RF, RP, 0);                                                                                      \
+      }                                                                                                                \
+      if (u->tan_split) CLB_SU2TL(NK, RF, RP);                                                                         \
     } else {                                                                                                           \
       CLB_SU2T1(NK, RF, RP, 0);                                                                                        \
     }                                                                                                                  \
@@ -109,6 +128,7 @@ template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, c
       CLB_SU2T(2, false, false);
   }
 #undef CLB_SU2T
+#undef CLB_SU2TL
 #undef CLB_SU2T1
 }
 

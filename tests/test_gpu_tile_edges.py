@@ -92,3 +92,34 @@ def test_su2_site_orders_compute_the_same_step(monkeypatch, precision, tol):
         lat.close()
     for r in res[1:]:
         assert rel(r[0], res[0][0], 22) < tol and rel(r[1], res[0][1], 19) < tol
+
+
+@pytest.mark.parametrize("tangent", [False, True])
+@pytest.mark.parametrize("N,order", [(5, 0), (33, 0), (33, 1), (34, 5)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_su2_force_by_direction_is_the_whole_sweep(monkeypatch, precision, N, order, tangent):
+    # the SU(2) part with a thread per site and direction against the one-thread sweep over every
+    # sector, in lattices that end inside a block, a tile and a run: states and a(t) to the last bit
+    from cosmolattice_b200 import Lattice
+    from cosmolattice_b200.initializers import su2u1_initial_state_tangent
+
+    monkeypatch.setenv("CLB_GAUGE_ORDER", str(order))
+    par, rp, m, f, p, sf = make_su2_case(N=N, evolver="VV2", expansion=True, amp=3e-2)
+    rng = np.random.default_rng(N)
+    f = f + 1e-2 * rng.standard_normal(f.shape)
+    for i in range(3):
+        f[10 + 4 * i:14 + 4 * i] /= np.sqrt((f[10 + 4 * i:14 + 4 * i] ** 2).sum(axis=0))
+    out = []
+    for split in ("0", "3"):
+        monkeypatch.setenv("CLB_SU2_SPLIT", split)
+        lat = Lattice(m, rp, precision=precision)
+        lat.set_state(f, p, sf)
+        if tangent:
+            df, dp, cd = su2u1_initial_state_tangent(m, rp, "gSU2", (f, p))
+            lat.tangent_begin(cd, df, dp)
+        lat.initialize()
+        lat.evolve(3)
+        out.append([lat.get_state()] + ([lat.tangent_get_state()] if tangent else []))
+        lat.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2]
