@@ -38,6 +38,7 @@ constexpr size_t kStageMin = (size_t)1 << 23; // host-transfer staging: >= 64 Mi
 constexpr int kDefaultShapeFP64 = 0;          // ShapeW
 constexpr int kDefaultShapeFP32 = 4;          // ShapeK
 constexpr int kMaxRun = 22;                   // longest x-run of one sweep block
+constexpr int kMaxRunLarge = 32;              // ... of a large FP64 lattice
 
 } // namespace
 
@@ -98,15 +99,19 @@ namespace {
 // blocks, so the runs minimise waves x (LX + 0.8); runs longer than 22 planes lose L2 reuse between
 // neighbouring tiles.  us per VV2 step, this rule against runs of two waves of blocks or 32 planes:
 // 125^3 two fields FP64 43.8 against 50.4, 96^3 FP64 17.5 / 20.6, 128^3 FP32 17.5 / 22.1, 192^3
-// two fields FP64 113.9 / 125.4, 384^3 FP32 198.8 / 201.5, 512^3 FP64 798.4 / 803.
+// two fields FP64 113.9 / 125.4, 384^3 FP32 198.8 / 201.5.  From 20 waves on (512^3) the length of a
+// run matters little to the waves (FP64 790 at 16, 27 and 32 planes), and longer FP64 runs spare halo
+// planes, which counts under the power cap: 200 steps and the read 207.0 ms at 32, 208.6 at 16.  FP32
+// keeps 22 (384^3, 200 steps and the read 56.0 ms, 56.6 at 32).
 void setup_geometry(clb_handle *h, int blocks_per_sm)
 {
   const int N = h->N;
   const int gx = (N + h->bz - 1) / h->bz, gy = (N + h->by - 1) / h->by;
   const long long slots = 148LL * std::max(1, blocks_per_sm), tiles = (long long)gx * gy;
+  const bool large = h->cfg.precision != CLB_PREC_FP32_SPLIT && tiles * ((N + kMaxRun - 1) / kMaxRun) > 20 * slots;
   int LX = 1;
   double best = 0;
-  for (int l = std::min(N, kMaxRun); l >= 1; --l) {
+  for (int l = std::min(N, large ? kMaxRunLarge : kMaxRun); l >= 1; --l) {
     const long long blocks = tiles * ((N + l - 1) / l);
     const double cost = (double)((blocks + slots - 1) / slots) * (l + 0.8);
     if (best == 0 || cost < best) {
