@@ -582,8 +582,8 @@ __device__ __forceinline__ int sector(int c) { return c == 0 ? 0 : c < 3 ? 1 : c
 #define CLB_SU2_KICK_MINB_F64 3
 #endif
 // SECT (as kernels()): 0 every sector in one sweep; else a part of a split sweep, run one after the
-// other over the same grid: 1 in halves, 3 and 4 in three parts, 5, 6 and 4 in four, each with the SU(2)
-// part (k_kick_links).  Each part updates, reduces and writes only its own components and partial slots
+// other over the same grid: 1 in halves, 3 in three parts, 5 and 6 in four, each with the SU(2) part, that
+// of the three and four parts with A (k_kick_links).  Each part updates, reduces and writes only its own components and partial slots
 // (sect_owns), so the parts hold fewer registers than the whole.  The kicks read the fields only, so
 // the parts' order is free.  Four blocks per SM timed best for the parts, FP64 and FP32.
 #ifndef CLB_SU2_HALF_MINB_F32
@@ -592,13 +592,9 @@ __device__ __forceinline__ int sector(int c) { return c == 0 ? 0 : c < 3 ? 1 : c
 #ifndef CLB_SU2_HALF_MINB_F64
 #define CLB_SU2_HALF_MINB_F64 4
 #endif
-// the FP64 three-part sweep's S, phi, Phi part (SECT 3) and A part (SECT 4); four blocks timed
-// best at 192^3 (ms per step): 4.99, against 5.37 with three for SECT 3 and 5.04 with five for SECT 4
+// the FP64 S, phi, Phi part (SECT 3); four blocks timed best at 192^3 (4.99 ms per step, 5.37 with three)
 #ifndef CLB_SU2_P3_MINB_F64
 #define CLB_SU2_P3_MINB_F64 CLB_SU2_HALF_MINB_F64
-#endif
-#ifndef CLB_SU2_P4_MINB_F64
-#define CLB_SU2_P4_MINB_F64 CLB_SU2_HALF_MINB_F64
 #endif
 // the FP64 four-part sweep's S and phi part (SECT 5) and Phi part (SECT 6)
 #ifndef CLB_SU2_P5_MINB_F64
@@ -611,7 +607,6 @@ template <class S, int NK, bool RF, bool RP, int SECT = 0>
 __global__ void __launch_bounds__(128, SECT == 0   ? (sizeof(S) == 4 ? CLB_SU2_KICK_MINB_F32 : CLB_SU2_KICK_MINB_F64)
                                        : sizeof(S) == 4 ? CLB_SU2_HALF_MINB_F32
                                        : SECT == 3      ? CLB_SU2_P3_MINB_F64
-                                       : SECT == 4      ? CLB_SU2_P4_MINB_F64
                                        : SECT == 5      ? CLB_SU2_P5_MINB_F64
                                        : SECT == 6      ? CLB_SU2_P6_MINB_F64
                                                         : CLB_SU2_HALF_MINB_F64)
@@ -1015,13 +1010,16 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4             ? CLB_SU2_TAN_
 // 65.3.  Tangent FP64 80^3 734 against 848, 40^3 167 against 212 (with the loops of kernels() unrolled).
 // The FP32 tangent form stays with one thread per site: 80^3 370 us against 438 at two blocks per SM
 // here and 476 at one.
+// WA: with the A component of the same direction, whose currents need the same covariant products, links
+// and phases: FP64 192^3 2833 us per step against 3066 with the A part in a sweep of its own, 95^3 390
+// against 418; FP32 95^3 267 against 284, 48^3 50.1 against 54.3.
 #ifndef CLB_SU2_DIR_MINB_F64
 #define CLB_SU2_DIR_MINB_F64 2
 #endif
 #ifndef CLB_SU2_DIR_MINB_F32
 #define CLB_SU2_DIR_MINB_F32 3
 #endif
-template <class S, class T, int NK, bool RF, bool RP>
+template <class S, class T, bool WA, int NK, bool RF, bool RP>
 __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8 ? CLB_SU2_DIR_MINB_F64 : CLB_SU2_DIR_MINB_F32)
     k_kick_links(const S *__restrict__ f, const S *__restrict__ df, S *__restrict__ p, S *__restrict__ dp, const __grid_constant__ Params a,
                  const __grid_constant__ Kick kc, const SweepState<T> *__restrict__ stp, const __grid_constant__ CoupDot cd, double *__restrict__ partials,
@@ -1033,6 +1031,9 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
   __shared__ double xe[2][NK][2][128];                        // pi^2 of directions 1 and 2 after each kick
   __shared__ double xd[TAN ? 2 : 1][NK][2][3][TAN ? 128 : 1]; // the terms of its tangent
   __shared__ T xw[2][3][128];                                 // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
+  static_assert(!(WA && TAN), "the A part of the tangent form has its own sweep");
+  __shared__ double xq[2][NK][2][WA ? 128 : 1]; // pi_A^2 of directions 1 and 2 after each kick
+  __shared__ S xg[2][4][WA ? 128 : 1];          // the differences d_1 A_0, d_1 A_2, d_2 A_0, d_2 A_1
   const int d = threadIdx.x / 128, t = threadIdx.x % 128;
   const int j1 = d == 0 ? 1 : 0, j2 = d == 2 ? 1 : 2; // the other directions, ascending
   const size_t U = a.oU + (size_t)d * 4 * a.n3, U1 = a.oU + (size_t)j1 * 4 * a.n3, U2 = a.oU + (size_t)j2 * 4 * a.n3;
@@ -1047,6 +1048,7 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
   double acc[3 * W]; // pi^2 after the first kick, <B^2>, pi^2 after the second; then their tangents
 #pragma unroll
   for (int k = 0; k < 3 * W; ++k) acc[k] = 0;
+  double accA[3] = {0, 0, 0}; // the same of A
   int buf = 0;
   for_sites_grouped<128>(a.N, a.n3, a.order, t, [&](size_t site, bool in) {
     const uint32_t s = (uint32_t)site;
@@ -1113,6 +1115,37 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
         p[pc + c * a.n3 + s] = q[c];
         if (TAN) dp[pc + c * a.n3 + s] = dq[c];
       }
+    double eA[NK];
+    S ga[3];
+    if constexpr (WA) { // kernels()' A component of this direction, with the SU(2) part's W and Phi
+      const S *Ad = f + fidx(a, 7, 0) + (size_t)d * a.n3;
+      S *pA = p + (size_t)(7 + d) * a.n3;
+      S qA = pA[s];
+      const uint32_t on[3] = {next(0, N * N), next(1, N), next(2, 1)}, om[3] = {prev(0, N * N), prev(1, N), prev(2, 1)};
+      const S c = Ad[s];
+      S tl[3], grad = 0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) tl[k] = (Ad[s + on[k]] + Ad[s + om[k]]) - 2 * c;
+      const S lap = recip<S>(a.ddx2) * ((tl[0] + tl[1]) + tl[2]);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        ga[j] = v.fd(7 + j, s, s + op);
+        const S g1 = v.fd(7 + j, s + om[j], d == j ? s : s + op + om[j]);
+        const S tg = div_by(ga[j] - g1, a.ddx);
+        grad = j == 0 ? tg : grad + tg;
+      }
+      const C2<S> wC = cmul(v.phaseC(d, s), v.cs(s + op));
+      const S Jc = v.gC * cmul(conj_(wC), v.cs(s)).im;
+      const S Jd = v.gD * sprod(Wd, Dg).im;
+      const S J = 2 * recip<S>(a.ddx) * rfo2 * (Jc + Jd);
+      const S K = G * (lap - grad) - A * J;
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        qA = (S)((double)qA + kc.h[k][3] * (double)K);
+        eA[k] = (double)qA * (double)qA;
+      }
+      if (in) pA[s] = qA;
+    }
     if (RP || RF) {
       if (d > 0) {
         if (RP)
@@ -1125,6 +1158,15 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
           }
         if (RF) xw[buf][d - 1][t] = pw1;
         if (RF && d == 2) xw[buf][2][t] = pw2;
+        if constexpr (WA) {
+          if (RP)
+#pragma unroll
+            for (int k = 0; k < NK; ++k) xq[buf][k][d - 1][t] = eA[k];
+          if (RF) {
+            xg[buf][2 * d - 2][t] = ga[0];
+            xg[buf][2 * d - 1][t] = d == 1 ? ga[2] : ga[1];
+          }
+        }
       }
       __syncthreads(); // the next site's values go to the other buffer
       if (d == 0 && in) {
@@ -1132,6 +1174,7 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
 #pragma unroll
           for (int k = 0; k < NK; ++k) {
             acc[2 * k] += (e[k] + xe[buf][k][0][t]) + xe[buf][k][1][t];
+            if constexpr (WA) accA[2 * k] += (eA[k] + xq[buf][k][0][t]) + xq[buf][k][1][t];
             if constexpr (TAN) {
               double td = (ed[k][0] + ed[k][1]) + ed[k][2];
 #pragma unroll
@@ -1142,6 +1185,10 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
         if (RF) {
           const T pw[3] = {xw[buf][0][t], xw[buf][1][t], xw[buf][2][t]};
           const T b2 = gB2(v, pw);
+          if constexpr (WA) { // aB2
+            const S f21 = xg[buf][0][t] - ga[1], f31 = xg[buf][2][t] - ga[2], f32 = xg[buf][3][t] - xg[buf][1][t];
+            accA[1] += (double)(f21 * f21 + (f31 * f31 + f32 * f32));
+          }
           if constexpr (TAN) {
             acc[1] += (double)b2.v;
             acc[4] += (double)b2.d;
@@ -1163,6 +1210,16 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
         row[9] = acc[3 * w + 1];
         row[15] = acc[3 * w + 2];
       }
+    if constexpr (WA) {
+      __syncthreads();
+      block_reduce<3, 128>(accA, smem);
+      if (threadIdx.x == 0) {
+        double *row = partials + (size_t)blockIdx.x * kRed;
+        row[3] = accA[0];
+        row[8] = accA[1];
+        row[14] = accA[2];
+      }
+    }
   }
 }
 

@@ -27,8 +27,8 @@ struct SU2Sector {
   // per component (ms per step): FP64 9.20 whole, 6.53 halves, 5.10 three parts, 4.73 four parts;
   // FP32 4.93, 3.18, 2.90, 2.93.  The tangent-linear sweep takes four parts in both (256^3 VV2, ms
   // per tangent step, three / four parts: FP64 37.9, 31.4; FP32 21.5, 19.5).  The SU(2) part has a
-  // thread per site and direction (k_kick_links; the FP32 tangent form one per site), with which the
-  // four parts take 3.07 ms at 192^3 FP64 and the three parts 2.13 in FP32.  Every form gives the
+  // thread per site and direction (k_kick_links; the FP32 tangent form one per site), and in the plain
+  // form A with it, with which a step takes 2.83 ms at 192^3 FP64.  Every form gives the
   // same state to the last bit.
   int split = 2;
   int tan_split = 3;

@@ -13,14 +13,14 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
   S *p = static_cast<S *>(u->p);
   // kick sweeps run as two halves (sectors S, phi, Phi, A; then SU(2)), three parts (S, phi, Phi; A;
   // SU(2)) or four (S, phi; Phi; A; SU(2)), which hold fewer registers than one sweep over every sector;
-  // reduction-only sweeps run whole
+  // of three and four the last two run in one launch (k_kick_links); reduction-only sweeps run whole
 #define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
   CLB_LAUNCH(h, kind,                                                                                                   \
              launch_pdl(k_kick<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, p, u->prm, kc,       \
                         (const State *)u->d_st, u->d_part, static_cast<const S *>(u->ph)))
-#define CLB_SU2KL(NK, RF, RP)                                                                                          \
+#define CLB_SU2KL(WA, NK, RF, RP)                                                                                          \
   CLB_LAUNCH(h, kind,                                                                                                  \
-             launch_pdl(k_kick_links<S, S, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f,              \
+             launch_pdl(k_kick_links<S, S, WA, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f,              \
                         (const S *)nullptr, p, (S *)nullptr, u->prm, kc, (const State *)u->d_st, CoupDot{}, u->d_part, \
                         static_cast<const S *>(u->ph)))
 #define CLB_SU2K(NK, RF, RP)                                                                                            \
@@ -29,16 +29,17 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
       if (u->split == 3) {                                                                                             \
         CLB_SU2K1(NK, RF, RP, 5);                                                                                      \
         CLB_SU2K1(NK, RF, RP, 6);                                                                                      \
-        CLB_SU2K1(NK, RF, RP, 4);                                                                                      \
       } else if (u->split == 2) {                                                                                      \
         CLB_SU2K1(NK, RF, RP, 3);                                                                                      \
-        CLB_SU2K1(NK, RF, RP, 4);                                                                                      \
       } else if (u->split) {                                                                                           \
         CLB_SU2K1(NK, RF, RP, 1);                                                                                      \
       } else {                                                                                                         \
         CLB_SU2K1(NK, RF, RP, 0);                                                                                      \
       }                                                                                                                \
-      if (u->split) CLB_SU2KL(NK, RF, RP);                                                                             \
+      if (u->split > 1)                                                                                                \
+        CLB_SU2KL(true, NK, RF, RP);                                                                                   \
+      else if (u->split)                                                                                               \
+        CLB_SU2KL(false, NK, RF, RP);                                                                                  \
     } else {                                                                                                           \
       CLB_SU2K1(NK, RF, RP, 0);                                                                                        \
     }                                                                                                                  \
@@ -82,7 +83,7 @@ template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, c
   do {                                                                                                                 \
     if constexpr (sizeof(S) == sizeof(double))                                                                         \
       CLB_LAUNCH(h, kind,                                                                                              \
-                 launch_pdl(k_kick_links<S, Tan<S>, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f, df, \
+                 launch_pdl(k_kick_links<S, Tan<S>, false, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f, df, \
                             p, dp, u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart, (const S *)nullptr));  \
     else                                                                                                               \
       CLB_SU2T1(NK, RF, RP, 2);                                                                                        \
