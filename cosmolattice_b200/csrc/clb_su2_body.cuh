@@ -370,7 +370,35 @@ template <class T> struct SiteAvg {
 };
 template <class S, class T> __device__ __forceinline__ T sGrad2(const Site<S, T> &v);
 template <class S, class T> __device__ __forceinline__ T aB2(const Site<S, T> &v, const T (*g)[3] = nullptr);
-template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v, const T *pw = nullptr);
+template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v, const T *dev = nullptr);
+
+// The Wilson term 2 - 2 w of a plaquette in <B^2>, in two steps so that the parts of a kick can hand on one
+// value: plaq_dev() of the plaquette, then gap().  FP64 links keep the expression as it stands (plaq_dev
+// is w).  Links held in FP32 give a w next to 1 whose rounding (6e-8) is of the size of the gap itself on
+// a fine lattice, and the factor 4 / (dx^4 g^2) carries it through the start's a-dot into all momenta:
+// with links of rms 1e-3 the magnetic energy was off by 1e-5 to 2e-3 and the tangent observable by up to
+// a tenth, and every change of the products' rounding shifted a(t).  There plaq_dev is the gap, formed as
+// 2 (x^2 + y^2 + z^2) / (1 + w), the same for a unit quaternion and free of the cancellation.
+template <class S, class T> __device__ __forceinline__ T gap(T dev)
+{
+  if constexpr (sizeof(S) == 4)
+    return dev;
+  else
+    return 2 - 2 * dev;
+}
+template <class S, class T> __device__ __forceinline__ T plaq_dev(const Q4<T> &P)
+{
+  if constexpr (sizeof(S) == 4) {
+    typename TanTraits<T>::base w;
+    if constexpr (TanTraits<T>::is)
+      w = P.w.v;
+    else
+      w = P.w;
+    return w > 0 ? kdiv(2 * ((P.x * P.x + P.y * P.y) + P.z * P.z), 1 + P.w) : 2 - 2 * P.w;
+  } else {
+    return P.w;
+  }
+}
 
 // (1/dx)^3 / gS; the tangent form's gS can carry a derivative
 template <class S, class T> __device__ __forceinline__ T su2_ngrad(const Site<S, T> &v)
@@ -443,7 +471,7 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
     const D2<T> Dg = v.dbl(s);
     const T normGrad = su2_ngrad(v) * G;
     const T normSrc = recip<T>(a.ddx) * A;
-    T pw[3]; // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
+    T dev[3]; // plaq_dev of plaq(1, 0), plaq(2, 0), plaq(2, 1)
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       T gr[3] = {0, 0, 0}, gb[3] = {0, 0, 0};
@@ -452,7 +480,7 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
       for (int j = 0; j < 3; ++j) {
         if (j == i) continue;
         const Q4<T> P = v.plaq(i, j), Pb = v.plaqBack(i, j);
-        if (j < i) pw[i + j - 1] = P.w;
+        if (j < i) dev[i + j - 1] = plaq_dev<S>(P);
         const T pv[3] = {P.x, P.y, P.z}, bv[3] = {Pb.x, Pb.y, Pb.z};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -468,7 +496,7 @@ __device__ __forceinline__ void kernels(const Site<S, T> &v, const Coef<T> &C, T
         K[10 + 3 * i + c] = -normGrad * (gr[c] - gb[c]) - normSrc * J;
       }
     }
-    if constexpr (AVG) av->b2G = gB2(v, pw);
+    if constexpr (AVG) av->b2G = gB2(v, dev);
   }
 }
 
@@ -505,7 +533,7 @@ template <class S, class T> __device__ __forceinline__ T dGrad2(const Site<S, T>
   }
   return acc;
 }
-// aB2's g and gB2's pw: the differences and plaquettes as kernels() formed them
+// aB2's g and gB2's dev: the differences and plaquettes as kernels() formed them
 template <class S, class T> __device__ __forceinline__ T Fij(const Site<S, T> &v, int i, int j)
 {
   return v.fd(7 + j, v.s, v.pl(i)) - v.fd(7 + i, v.s, v.pl(j));
@@ -516,11 +544,11 @@ template <class S, class T> __device__ __forceinline__ T aB2(const Site<S, T> &v
   const T f21 = F(1, 0), f31 = F(2, 0), f32 = F(2, 1);
   return f21 * f21 + (f31 * f31 + f32 * f32);
 }
-template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v, const T *pw)
+template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v, const T *dev)
 {
   const T c = kdiv(T(4.0), ipw(v.dx, 4) * ipw(v.gS, 2));
-  const T t10 = 2 - 2 * (pw ? pw[0] : v.plaq(1, 0).w), t20 = 2 - 2 * (pw ? pw[1] : v.plaq(2, 0).w),
-          t21 = 2 - 2 * (pw ? pw[2] : v.plaq(2, 1).w);
+  const T t10 = gap<S>(dev ? dev[0] : plaq_dev<S>(v.plaq(1, 0))), t20 = gap<S>(dev ? dev[1] : plaq_dev<S>(v.plaq(2, 0))),
+          t21 = gap<S>(dev ? dev[2] : plaq_dev<S>(v.plaq(2, 1)));
   return c * (t10 + (t20 + t21));
 }
 // The SiteAvg terms of the sectors in SECT, formed on their own (a sweep that does not kick).
@@ -1030,7 +1058,7 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
   __shared__ double smem[(3 * 128 / 32) * 3 * W];
   __shared__ double xe[2][NK][2][128];                        // pi^2 of directions 1 and 2 after each kick
   __shared__ double xd[TAN ? 2 : 1][NK][2][3][TAN ? 128 : 1]; // the terms of its tangent
-  __shared__ T xw[2][3][128];                                 // plaq(1, 0).w, plaq(2, 0).w, plaq(2, 1).w
+  __shared__ T xw[2][3][128];                                 // plaq_dev of plaq(1, 0), plaq(2, 0), plaq(2, 1)
   static_assert(!(WA && TAN), "the A part of the tangent form has its own sweep");
   __shared__ double xq[2][NK][2][WA ? 128 : 1]; // pi_A^2 of directions 1 and 2 after each kick
   __shared__ S xg[2][4][WA ? 128 : 1];          // the differences d_1 A_0, d_1 A_2, d_2 A_0, d_2 A_1
@@ -1077,15 +1105,15 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
     auto plaqBack = [&](size_t Uj, uint32_t mj) {
       return qdag(qmul(qmul(qmul(Ud, qdag(at(Uj, s + op + mj))), qdag(at(U, s + mj))), at(Uj, s + mj)));
     };
-    T gr[3], gb[3], pw1, pw2;
+    T gr[3], gb[3], dev1, dev2;
     {
       const Q4<T> P = plaq(U1, o1), B = plaqBack(U1, m1);
-      gr[0] = P.x, gr[1] = P.y, gr[2] = P.z, pw1 = P.w;
+      gr[0] = P.x, gr[1] = P.y, gr[2] = P.z, dev1 = plaq_dev<S>(P);
       gb[0] = B.x, gb[1] = B.y, gb[2] = B.z;
     }
     {
       const Q4<T> P = plaq(U2, o2), B = plaqBack(U2, m2);
-      gr[0] = gr[0] + P.x, gr[1] = gr[1] + P.y, gr[2] = gr[2] + P.z, pw2 = P.w;
+      gr[0] = gr[0] + P.x, gr[1] = gr[1] + P.y, gr[2] = gr[2] + P.z, dev2 = plaq_dev<S>(P);
       gb[0] = gb[0] + B.x, gb[1] = gb[1] + B.y, gb[2] = gb[2] + B.z;
     }
     const T normGrad = su2_ngrad(v) * G, normSrc = recip<T>(a.ddx) * A;
@@ -1156,8 +1184,8 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
 #pragma unroll
               for (int c = 0; c < 3; ++c) xd[buf][k][d - 1][c][t] = ed[k][c];
           }
-        if (RF) xw[buf][d - 1][t] = pw1;
-        if (RF && d == 2) xw[buf][2][t] = pw2;
+        if (RF) xw[buf][d - 1][t] = dev1;
+        if (RF && d == 2) xw[buf][2][t] = dev2;
         if constexpr (WA) {
           if (RP)
 #pragma unroll
@@ -1183,8 +1211,8 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
             }
           }
         if (RF) {
-          const T pw[3] = {xw[buf][0][t], xw[buf][1][t], xw[buf][2][t]};
-          const T b2 = gB2(v, pw);
+          const T dev[3] = {xw[buf][0][t], xw[buf][1][t], xw[buf][2][t]};
+          const T b2 = gB2(v, dev);
           if constexpr (WA) { // aB2
             const S f21 = xg[buf][0][t] - ga[1], f31 = xg[buf][2][t] - ga[2], f32 = xg[buf][3][t] - xg[buf][1][t];
             accA[1] += (double)(f21 * f21 + (f31 * f31 + f32 * f32));

@@ -84,6 +84,36 @@ def make_su2_case(N=8, evolver="VV2", expansion=True, dt=0.005, seed="s", amp=1e
     return par, rp, m, f, p, sf
 
 
+def make_fine_su2_case(N, seed):
+    """Run parameters, lphi4SU2U1 model and state with smooth fluctuations of rms 1e-3 about the
+    homogeneous doublet and links of the same size: what a run starts from on a fine lattice, where a
+    plaquette's trace is 1 to seven digits."""
+    import numpy as np
+
+    from cosmolattice_b200 import MODELS, ParameterParser, RunParameters
+
+    par = ParameterParser(params={"N": N, "kIR": 1.0, "dt": 0.005, "evolver": "VV2", "expansion": "true", "lambda": 1.0,
+                                  "qG": 50.0, "qH": 50.0, "SU2Doublet_initial_norm": "5.25151e18", "gU1s": 0.35, "gSU2s": 0.6})
+    rp = RunParameters(par)
+    m = MODELS["lphi4SU2U1"](par, rp)
+    rng = np.random.default_rng(seed)
+    k = np.fft.fftfreq(N, 1 / N)
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + k[None, None, :N // 2 + 1] ** 2
+    filt = np.where((k2 > 0) & (k2 <= (N / 4) ** 2), (k2 + 1) ** -0.25, 0.0)
+
+    def noise(rms=1e-3):
+        n = np.fft.irfftn(np.fft.rfftn(rng.standard_normal((N,) * 3)) * filt, s=(N,) * 3, axes=(0, 1, 2))
+        return n * (rms / np.sqrt((n * n).mean()))
+
+    f = [noise() for _ in range(3)] + [noise() + 0.5 for _ in range(4)] + [noise() for _ in range(3)]
+    for _ in range(3):
+        v = np.stack([noise() for _ in range(3)])
+        n = np.sqrt((v * v).sum(axis=0))
+        f += [np.cos(n), *(np.sin(n) / n * v)]
+    p = [noise(4e-3) for _ in range(7)] + [noise() for _ in range(12)]
+    return rp, m, np.stack(f), np.stack(p), {"aI": 1.0, "aSI": 1.0, "aIM": 1.0, "aDotI": 0.0, "aDotSI": 0.0}
+
+
 @pytest.fixture(scope="session")
 def gpu_available():
     try:

@@ -12,7 +12,7 @@ import math
 import numpy as np
 import pytest
 
-from conftest import make_su2_case, site_metrics
+from conftest import make_fine_su2_case, make_su2_case, site_metrics
 
 pytestmark = pytest.mark.gpu
 
@@ -283,3 +283,32 @@ def test_kick_split_is_bitwise_the_whole_sweep(monkeypatch, evolver, precision):
         assert np.array_equal(fs, f0) and np.array_equal(ps, p0), split
         assert ss == s0, split
         assert ms["energies"] == m0["energies"], split
+
+
+@pytest.mark.parametrize("N", [63, 96, 128])
+@pytest.mark.parametrize("seed", [1, 2])
+def test_fp32_magnetic_energy_and_scale_factor_on_fine_lattices(N, seed):
+    # <B^2> of the SU(2) links must not cancel in FP32: the start's a-dot is formed from it.  A link's
+    # vector part is stored to 6e-8 of itself, independently at each site, so its square's average
+    # agrees to far less; the bar is 1e-6 (2 - 2 w of an FP32 w is off by 1e-5 to 4e-4 here).  a and
+    # a-dot, formed from averages over as many sites, agree to the roundoff of one value, 1e-7.
+    from cosmolattice_b200 import Lattice
+
+    rp, m, f, p, sf = make_fine_su2_case(N, seed)
+    res = {}
+    for prec in ("fp64", "fp32"):
+        lat = Lattice(m, rp, precision=prec)
+        lat.set_state(f, p, sf)
+        lat.initialize()
+        start = lat.measure()
+        lat.evolve(10)
+        res[prec] = (start, lat.measure(), lat.get_state()[2])
+        lat.close()
+    for k in (0, 1):
+        x, y = res["fp32"][k]["energies"][9], res["fp64"][k]["energies"][9]
+        print("SU(2) magnetic energy", N, seed, k, abs(x - y) / y)
+        assert abs(x - y) <= 1e-6 * y
+    for key in ("aI", "aDotI"):
+        x, y = res["fp32"][2][key], res["fp64"][2][key]
+        print(key, abs(x - y) / y)
+        assert abs(x - y) <= 1e-7 * y

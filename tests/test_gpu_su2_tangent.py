@@ -9,7 +9,7 @@ part of the tangent run must equal the plain run bitwise.
 import numpy as np
 import pytest
 
-from conftest import make_su2_case
+from conftest import make_fine_su2_case, make_su2_case
 
 pytestmark = pytest.mark.gpu
 
@@ -265,3 +265,27 @@ def test_tangent_kick_split_is_bitwise_the_whole_sweep(monkeypatch, precision):
     for split in ("1", "2", "3"):
         for (a, b) in zip(out[split], out["0"]):
             assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2], split
+
+
+@pytest.mark.parametrize("N", [35, 56])
+def test_fp32_observable_and_its_derivative_on_a_fine_lattice(N):
+    # the SU(2) magnetic energy and its derivative, from FP32 links of rms 1e-3 (2 - 2 w of an FP32 w
+    # puts the derivative off by a hundredth to a tenth here)
+    from cosmolattice_b200 import Lattice
+    from cosmolattice_b200.adjoint import SU2_GAUGE_FRACTION
+
+    rp, m, f, p, sf = make_fine_su2_case(N, N)
+    dp = np.zeros_like(p)
+    dp[10:] = -p[10:] / BASE["gSU2"]
+    res = {}
+    for prec in ("fp64", "fp32"):
+        lat = Lattice(m, rp, precision=prec)
+        lat.set_state(f, p, sf)
+        lat.tangent_begin([0, 0, 0, 0, 1.0, 0], momenta_dot=dp)
+        lat.initialize()
+        lat.evolve(8)
+        res[prec] = lat.tangent_observable(SU2_GAUGE_FRACTION)
+        lat.close()
+    for x, y in zip(res["fp32"], res["fp64"]):
+        print(N, x, y, abs(x - y) / abs(y))
+        assert abs(x - y) <= REL * abs(y)
