@@ -1058,7 +1058,9 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
   __shared__ double smem[(3 * 128 / 32) * 3 * W];
   __shared__ double xe[2][NK][2][128];                        // pi^2 of directions 1 and 2 after each kick
   __shared__ double xd[TAN ? 2 : 1][NK][2][3][TAN ? 128 : 1]; // the terms of its tangent
-  __shared__ T xw[2][3][128];                                 // plaq_dev of plaq(1, 0), plaq(2, 0), plaq(2, 1)
+  // plaq_dev of plaq(1, 0), plaq(2, 0), plaq(2, 1), and its tangent: plain numbers, since a shared array
+  // of pairs would be set to zero by every thread at its own time
+  __shared__ typename TanTraits<T>::base xw[W][2][3][128];
   static_assert(!(WA && TAN), "the A part of the tangent form has its own sweep");
   __shared__ double xq[2][NK][2][WA ? 128 : 1]; // pi_A^2 of directions 1 and 2 after each kick
   __shared__ S xg[2][4][WA ? 128 : 1];          // the differences d_1 A_0, d_1 A_2, d_2 A_0, d_2 A_1
@@ -1184,8 +1186,16 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
 #pragma unroll
               for (int c = 0; c < 3; ++c) xd[buf][k][d - 1][c][t] = ed[k][c];
           }
-        if (RF) xw[buf][d - 1][t] = dev1;
-        if (RF && d == 2) xw[buf][2][t] = dev2;
+        auto put_dev = [&](int k, const T &x) {
+          if constexpr (TAN) {
+            xw[0][buf][k][t] = x.v;
+            xw[1][buf][k][t] = x.d;
+          } else {
+            xw[0][buf][k][t] = x;
+          }
+        };
+        if (RF) put_dev(d - 1, dev1);
+        if (RF && d == 2) put_dev(2, dev2);
         if constexpr (WA) {
           if (RP)
 #pragma unroll
@@ -1211,7 +1221,13 @@ __global__ void __launch_bounds__(3 * 128, TanTraits<T>::is ? 1 : sizeof(S) == 8
             }
           }
         if (RF) {
-          const T dev[3] = {xw[buf][0][t], xw[buf][1][t], xw[buf][2][t]};
+          auto get_dev = [&](int k) -> T {
+            if constexpr (TAN)
+              return T(xw[0][buf][k][t], xw[1][buf][k][t]);
+            else
+              return xw[0][buf][k][t];
+          };
+          const T dev[3] = {get_dev(0), get_dev(1), get_dev(2)};
           const T b2 = gB2(v, dev);
           if constexpr (WA) { // aB2
             const S f21 = xg[buf][0][t] - ga[1], f31 = xg[buf][2][t] - ga[2], f32 = xg[buf][3][t] - xg[buf][1][t];
