@@ -717,11 +717,11 @@ template <class R, int NS> struct Measure {
   static void run(clb_handle *h, double am) { Launch<R, NS>::measure(h, am); }
 };
 
-// The device's scalar state and error flag in h->rb, with the stream idle.
+// The device's scalar state and error flag, as the work queued on the stream leaves them, in h->rb.
 cudaError_t read_back(clb_handle *h)
 {
   if (h->rb_valid) return cudaSuccess;
-  cudaError_t e = cudaMemcpyAsync(h->rb, h->d_st, sizeof(Readback), cudaMemcpyDeviceToHost, h->stream);
+  cudaError_t e = cudaMemcpyAsync(&h->rb, h->d_st, sizeof(Readback), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   h->rb_valid = e == cudaSuccess;
   return e;
@@ -733,8 +733,8 @@ int sync_and_check(clb_handle *h, const char *where)
   if (e == cudaSuccess) e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, where);
   collect_profile(h);
-  if (h->rb->err != 0) return h->fail(CLB_ETIMEOUT, std::string(where) + ": a sweep's bounded wait for its tile loads gave up");
-  if (h->rb->st.status != 0) return h->fail(CLB_ENONFINITE, std::string(where) + ": a volume average or a(t) is not finite");
+  if (h->rb.err != 0) return h->fail(CLB_ETIMEOUT, std::string(where) + ": a sweep's bounded wait for its tile loads gave up");
+  if (h->rb.st.status != 0) return h->fail(CLB_ENONFINITE, std::string(where) + ": a volume average or a(t) is not finite");
   return CLB_OK;
 }
 
@@ -886,7 +886,6 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
     if (ok) ok = cudaMemset(h->fld[b], 0, bytes) == cudaSuccess && cudaMemset(h->pi[b], 0, bytes) == cudaSuccess;
   }
   ok = ok && cudaMalloc(&h->d_st, sizeof(Readback)) == cudaSuccess && cudaMemset(h->d_st, 0, sizeof(Readback)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->rb, sizeof(Readback)) == cudaSuccess;
   if (ok) h->d_err = &reinterpret_cast<Readback *>(h->d_st)->err;
   ok = ok && cudaMalloc(&h->d_part, h->part_rows * kMeasSlots * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_sums, kMeasSlots * sizeof(double)) == cudaSuccess;
@@ -934,7 +933,6 @@ void clb_destroy(clb_handle *h)
   if (h->d_st) cudaFree(h->d_st);
   if (h->d_part) cudaFree(h->d_part);
   if (h->d_sums) cudaFree(h->d_sums);
-  if (h->rb) cudaFreeHost(h->rb);
   if (h->d_hist) cudaFree(h->d_hist);
   if (h->d_stage) cudaFree(h->d_stage);
   if (h->plan_ok) cufftDestroy(h->plan);
@@ -1042,7 +1040,7 @@ int clb_get_state(clb_handle *h, double *fields, double *momenta, clb_scalefacto
   if (h->su2) return su2_get_state(h, fields, momenta, sf);
   cudaError_t e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
-  const DevState cur = h->rb->st;
+  const DevState cur = h->rb.st;
   CompOffsets fo{{0.0, 0.0}}, po{{0.0, 0.0}};
   if (h->fp32)
     for (int f = 0; f < h->NS; ++f) {
@@ -1211,7 +1209,7 @@ int clb_measure(clb_handle *h, double e0, clb_measurement *m)
   if (h->su2) return su2_measure(h, e0, m);
   cudaError_t e = read_back(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_measure");
-  DevState s = h->rb->st;
+  DevState s = h->rb.st;
   const double al = h->md.alpha;
   const double am = std::pow(s.aI, al - 3);
   dispatch<Measure>(h, am);
@@ -1262,9 +1260,12 @@ int clb_measure(clb_handle *h, double e0, clb_measurement *m)
     m->friedmann[0] = (LHS - RHS) / (LHS + RHS);
     m->friedmann[1] = LHS;
     m->friedmann[2] = RHS;
-    h->rb->st = s; // the stream is idle: no copy into or out of rb is in flight
-    e = cudaMemcpyAsync(h->d_st, &h->rb->st, sizeof(s), cudaMemcpyHostToDevice, h->stream);
-    if (e != cudaSuccess) return h->cuda_fail(e, "clb_measure");
+    e = cudaMemcpyAsync(h->d_st, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream); // s is read before this returns
+    if (e != cudaSuccess) {
+      h->rb_valid = false;
+      return h->cuda_fail(e, "clb_measure");
+    }
+    h->rb.st = s;
   } else {
     m->friedmann[0] = std::fabs(1.0 - Etot / e0);
   }
@@ -1430,7 +1431,7 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
     double ref = 0.0;
     if (h->fp32) {
       if ((e = read_back(h)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
-      const DevState &cur = h->rb->st;
+      const DevState &cur = h->rb.st;
       ref = which == 0 ? cur.ref_phi[h->rs][comp] : cur.ref_pi[h->rs][comp];
       CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather<float><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const float *>(src) + comp_off, h->d_spec, h->pd, ref));
     } else {
@@ -1469,7 +1470,7 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
     aI = sf.aI;
   } else {
     if ((e = read_back(h)) != cudaSuccess) return h->cuda_fail(e, "clb_spectrum");
-    aI = h->rb->st.aI;
+    aI = h->rb.st.aI;
   }
   const double kIR = 2 * 3.14159265358979323846 / (N * h->cfg.dx);
   // momenta: a^{2 alpha - 6} for matter (scalarsingletmeasurer.h:80), a^{2 alpha - 2} for gauge

@@ -74,7 +74,6 @@ struct clb_batch {
   int *d_blk = nullptr;
   DevState *d_st = nullptr;
   double *d_part = nullptr, *d_sums = nullptr, *d_stage = nullptr;
-  DevState *rb = nullptr; // pinned: one member's state on its way to the host
   size_t stage_n = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -649,7 +648,6 @@ void clb_batch_destroy(clb_batch *b)
   for (void *q : {(void *)b->d_lat, (void *)b->d_blk, (void *)b->d_st, (void *)b->d_part, (void *)b->d_sums,
                   (void *)b->d_stage, (void *)b->d_plat, (void *)b->d_members, (void *)b->d_offsets})
     if (q) cudaFree(q);
-  if (b->rb) cudaFreeHost(b->rb);
   for (auto e : b->ev)
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -741,7 +739,6 @@ int clb_batch_create(const clb_config *cfgs, const clb_model_desc *mds, int32_t 
   ok = ok && cudaMalloc(&b->d_offsets, (size_t)(n + 1) * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_sums, 8 * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&b->d_stage, b->stage_n * sizeof(double)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&b->rb, sizeof(DevState)) == cudaSuccess;
   ok = ok && cudaEventCreate(&b->ev[0]) == cudaSuccess && cudaEventCreate(&b->ev[1]) == cudaSuccess;
   if (ok) {
     // a configuration tuned earlier in this process for the same ensemble, else the default
@@ -833,8 +830,8 @@ int clb_batch_get_state(clb_batch *b, int32_t i, double *fields, double *momenta
   if (i < 0 || i >= b->n) return b->fail(CLB_EINVAL, "clb_batch_get_state: member index out of range");
   const BatchLat &L = b->lat[(size_t)i];
   const size_t n3 = (size_t)L.N * L.N * L.N;
-  // the state and the two arrays in stream order, one wait
-  cudaError_t e = cudaMemcpyAsync(b->rb, b->d_st + i, sizeof(DevState), cudaMemcpyDeviceToHost, b->stream);
+  // the two arrays and the state in stream order, one wait (the state's copy into ordinary memory is it)
+  cudaError_t e = cudaSuccess;
   for (int w = 0; w < 2 && e == cudaSuccess; ++w) {
     double *dst = w == 0 ? fields : momenta;
     if (!dst) continue;
@@ -847,10 +844,11 @@ int clb_batch_get_state(clb_batch *b, int32_t i, double *fields, double *momenta
       k_batch_unpack<double><<<kPackBlocks, 256, 0, b->stream>>>(static_cast<const double *>(src) + L.off, b->d_stage, n3, nullptr);
     e = cudaMemcpyAsync(dst, b->d_stage, n3 * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
   }
+  DevState s;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&s, b->d_st + i, sizeof(s), cudaMemcpyDeviceToHost, b->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "clb_batch_get_state");
   if (sf) {
-    const DevState &s = *b->rb;
     sf->aI = s.aI;
     sf->aSI = s.aSI;
     sf->aIM = s.aIM;

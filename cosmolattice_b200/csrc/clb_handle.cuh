@@ -52,10 +52,11 @@ struct clb_handle {
   size_t sweep_smem = 0;
   DevState *d_st = nullptr; // the first member of a Readback on the device
   int *d_err = nullptr;     // its second: set by a sweep whose bounded wait gave up
-  // The last Readback in pinned memory (scalar singlets): one asynchronous copy behind a call's work
-  // takes the place of a synchronous copy per value (about 10 us each), and calls between which
-  // nothing ran read it as it is.  rb_valid: nothing that changes the device's was launched since.
-  Readback *rb = nullptr;
+  // The last Readback (scalar singlets): one copy behind a call's work takes the place of a synchronous
+  // copy per value (about 10 us each), and calls between which nothing ran read it as it is.  rb_valid:
+  // it is what the device holds once the work queued on the stream is done; that stream need not be idle.
+  // In ordinary memory: a pinned allocation took 0.9 to 2.5 ms of every clb_create (2.1 ms without).
+  Readback rb{};
   bool rb_valid = false;
   double *d_part = nullptr;
   double *d_sums = nullptr;
