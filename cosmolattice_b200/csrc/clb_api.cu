@@ -1023,7 +1023,9 @@ __attribute__((visibility("hidden"))) int clb::scalar_set_state(clb_handle *h, c
     s.ref_pi[0][f] = s.ref_pi[1][f] = po.v[f];
   }
   h->rb_valid = false;
-  e = cudaMemcpy(h->d_st, &s, sizeof(s), cudaMemcpyHostToDevice);
+  // on the handle's stream, where the read-backs are: it does not wait for copies on the default stream
+  e = cudaMemcpyAsync(h->d_st, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_set_state");
   h->has_state = true;
   h->initialized = false;
