@@ -73,7 +73,7 @@ int su2_tangent_get_state(clb_handle *h, double *fields_dot, double *momenta_dot
 int su2_tangent_observable(clb_handle *h, const double *w, int32_t nw, double *obs, double *dobs);
 int su2_tangent_end(clb_handle *h);
 int su2_tangent_energies(clb_handle *h, double *E, double *dE);
-const double *su2_tangent_component(clb_handle *h, int which, int comp, double *aI, double *daI);
+bool su2_tangent_component(clb_handle *h, int which, int comp, CompView *out, double *aI, double *daI);
 
 const double *u1_component(clb_handle *h, int which, int comp, bool *gauge);
 const double *su2_component(clb_handle *h, int which, int comp, bool *gauge);
@@ -1371,6 +1371,15 @@ double spec_value(const clb_handle *h, int ps_type, int ps_version, double dk, i
   return t * t * t / dk / 2.0 / (pi * pi) * (sum / (double)c);
 }
 
+// A component as the real input of an in-place R2C transform.
+void gather_view(clb_handle *h, const CompView &v, double *dst)
+{
+  if (v.f32)
+    CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<float><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const float *>(v.p), dst, h->N, v.stride));
+  else
+    CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<double><<<kElemBlocks, 256, 0, h->stream>>>(static_cast<const double *>(v.p), dst, h->N, v.stride));
+}
+
 // clb_spectrum, also returning the raw bin sums [sum |f|^2 | sum |n|] and counts, and whether the
 // component belongs to a gauge field.
 int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, int32_t ps_version, double dk,
@@ -1567,9 +1576,9 @@ int clb_tangent_spectrum(clb_handle *h, int32_t which, int32_t comp, int32_t ps_
   if (!h->su2) return h->fail(CLB_EUNSUPPORTED, "clb_tangent_spectrum: the tangent-linear form covers lphi4SU2U1");
   if (!d_value_out) return h->fail(CLB_EINVAL, "clb_tangent_spectrum: null output");
   double aI = 1, daI = 0;
-  const double *tsrc = nullptr;
-  if (which == 0 || which == 1) tsrc = su2_tangent_component(h, which, comp, &aI, &daI);
-  if (!tsrc && (which == 0 || which == 1) && comp >= 0 && comp < (which == 0 ? 22 : 19))
+  CompView tsrc{};
+  const bool found = (which == 0 || which == 1) && su2_tangent_component(h, which, comp, &tsrc, &aI, &daI);
+  if (!found && (which == 0 || which == 1) && comp >= 0 && comp < (which == 0 ? 22 : 19))
     return h->fail(CLB_ESTATE, "clb_tangent_spectrum: call clb_tangent_begin first");
   std::vector<double> sums;
   std::vector<unsigned long long> cnt;
@@ -1583,7 +1592,7 @@ int clb_tangent_spectrum(clb_handle *h, int32_t which, int32_t comp, int32_t ps_
   cudaError_t e = cudaSuccess;
   if (!h->d_spec2 && (e = cudaMalloc(&h->d_spec2, spec_n * sizeof(double))) != cudaSuccess)
     return h->fail(CLB_ENOMEM, std::string("clb_tangent_spectrum: ") + cudaGetErrorString(e));
-  CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_raw<double><<<kElemBlocks, 256, 0, h->stream>>>(tsrc, h->d_spec2, N));
+  gather_view(h, tsrc, h->d_spec2);
   if (cufftExecD2Z(h->plan, h->d_spec2, reinterpret_cast<cufftDoubleComplex *>(h->d_spec2)) != CUFFT_SUCCESS)
     return h->fail(CLB_ECUDA, "clb_tangent_spectrum: cufftExecD2Z failed");
   const size_t smem = (size_t)nbins * sizeof(double);

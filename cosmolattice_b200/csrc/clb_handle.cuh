@@ -24,6 +24,13 @@ using clb::U1Sector;
 using clb::SU2Sector;
 using namespace clb;
 
+// One component of N^3 sites on the device, its elements stride apart.
+struct CompView {
+  const void *p;
+  int stride;
+  bool f32;
+};
+
 // What every call of a scalar-singlet handle checks or reads at its end.
 struct Readback {
   DevState st;

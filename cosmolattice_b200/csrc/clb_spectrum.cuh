@@ -40,15 +40,17 @@ static __global__ void __launch_bounds__(256) k_spec_gather_plain(const double *
   }
 }
 
-// Unpadded N^3 component of storage type R -> real input of an in-place R2C transform.
+// Unpadded N^3 component of storage type R, its elements stride apart -> real input of an in-place R2C
+// transform.
 template <class R>
-static __global__ void __launch_bounds__(256) k_spec_gather_raw(const R *__restrict__ src, double *__restrict__ dst, int N)
+static __global__ void __launch_bounds__(256)
+    k_spec_gather_raw(const R *__restrict__ src, double *__restrict__ dst, int N, int stride = 1)
 {
   const long long pitch = 2LL * (N / 2 + 1);
   for (long long r = blockIdx.x; r < (long long)N * N; r += gridDim.x) {
-    const R *s = src + r * N;
+    const R *s = src + r * N * stride;
     double *d = dst + r * pitch;
-    for (int z = threadIdx.x; z < N; z += blockDim.x) d[z] = (double)s[z];
+    for (int z = threadIdx.x; z < N; z += blockDim.x) d[z] = (double)s[z * stride];
   }
 }
 

@@ -267,6 +267,26 @@ void free_tangent(SU2Sector *u)
   u->d_tpart = u->d_tsums = nullptr;
   u->tangent = false;
 }
+
+// The stored link phases of A.
+void link_phases(clb_handle *h)
+{
+  SU2Sector *u = h->su2;
+  if (u->fp32)
+    k_phases<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(u->f), static_cast<float *>(u->ph), u->prm);
+  else
+    k_phases<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(u->f), static_cast<double *>(u->ph), u->prm);
+}
+
+// The tangent form's kicks form the link phases themselves; the plain kicks read them again.
+cudaError_t leave_tangent(clb_handle *h)
+{
+  link_phases(h);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  free_tangent(h->su2);
+  return e;
+}
 } // namespace
 
 __attribute__((visibility("hidden"))) void su2_destroy(clb_handle *h)
@@ -287,6 +307,16 @@ template <class S> S *comp_at(const clb_handle *h, void *buf, bool field, int c,
 {
   stride = field && ((c >= 3 && c < 7) || c >= 10) ? 4 : 1;
   return static_cast<S *>(buf) + (field ? fidx(h->su2->prm, c, 0) : (size_t)c * h->n3);
+}
+CompView comp_view(const clb_handle *h, void *buf, bool field, int c)
+{
+  int st;
+  if (h->su2->fp32) {
+    const float *p = comp_at<float>(h, buf, field, c, st);
+    return CompView{p, st, true};
+  }
+  const double *p = comp_at<double>(h, buf, field, c, st);
+  return CompView{p, st, false};
 }
 // The component from / to an FP64 array on the host or the device, through the staging buffer where
 // the device holds it in FP32 or among others; ordered on the handle's stream.
@@ -340,11 +370,7 @@ __attribute__((visibility("hidden"))) int su2_set_state(clb_handle *h, const dou
   for (int c = 0; c < NF && e == cudaSuccess; ++c) e = set_comp(h, u->f, true, c, fields + (size_t)c * h->n3);
   for (int c = 0; c < NP && e == cudaSuccess; ++c) e = set_comp(h, u->p, false, c, momenta + (size_t)c * h->n3);
   if (e == cudaSuccess) {
-    // the link phases of the new A
-    if (u->fp32)
-      k_phases<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(u->f), static_cast<float *>(u->ph), u->prm);
-    else
-      k_phases<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(u->f), static_cast<double *>(u->ph), u->prm);
+    link_phases(h); // of the new A
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -755,9 +781,9 @@ __attribute__((visibility("hidden"))) int su2_tangent_begin(clb_handle *h, const
   if (h->gw) return h->fail(CLB_EUNSUPPORTED, "clb_tangent_begin: the tangent-linear form runs without the GW sector");
   if (n < 0 || n > 6 || (n > 0 && !couplings_dot))
     return h->fail(CLB_EINVAL, "clb_tangent_begin: up to 6 coupling derivatives");
-  cudaError_t e = cudaStreamSynchronize(h->stream);
+  // an earlier tangent form ends first: where this call fails, the plain form goes on from its state
+  cudaError_t e = u->tangent ? leave_tangent(h) : cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_tangent_begin");
-  free_tangent(u);
   bool ok = cudaMalloc(&u->df, u->nf * u->esz) == cudaSuccess && cudaMalloc(&u->dp, NP * h->n3 * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_tst, sizeof(TState)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_tpart, (size_t)kSU2Blocks * 2 * kRed * sizeof(double)) == cudaSuccess;
@@ -890,30 +916,22 @@ __attribute__((visibility("hidden"))) int su2_tangent_observable(clb_handle *h, 
 
 __attribute__((visibility("hidden"))) int su2_tangent_end(clb_handle *h)
 {
-  SU2Sector *u = h->su2;
-  // the tangent form's kicks form the link phases themselves; the plain kicks read them again
-  if (u->fp32)
-    k_phases<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(u->f), static_cast<float *>(u->ph), u->prm);
-  else
-    k_phases<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(u->f), static_cast<double *>(u->ph), u->prm);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  free_tangent(u);
+  const cudaError_t e = leave_tangent(h);
   return e == cudaSuccess ? CLB_OK : h->cuda_fail(e, "clb_tangent_end");
 }
 
-// Tangent of one state component (clb_tangent_spectrum) as one FP64 array, and the scale factor with
-// its tangent.  The link-phase buffer, which the tangent form does not use, stages it.
-__attribute__((visibility("hidden"))) const double *su2_tangent_component(clb_handle *h, int which, int comp, double *aI,
-                                                                          double *daI)
+// Tangent of one state component (clb_tangent_spectrum), and the scale factor with its tangent.
+__attribute__((visibility("hidden"))) bool su2_tangent_component(clb_handle *h, int which, int comp, CompView *out, double *aI,
+                                                                 double *daI)
 {
   SU2Sector *u = h->su2;
-  if (!u->tangent || comp < 0 || comp >= (which == 0 ? NF : NP)) return nullptr;
+  if (!u->tangent || comp < 0 || comp >= (which == 0 ? NF : NP)) return false;
   TState t;
-  if (cudaMemcpy(&t, u->d_tst, sizeof(t), cudaMemcpyDeviceToHost) != cudaSuccess) return nullptr;
+  if (cudaMemcpy(&t, u->d_tst, sizeof(t), cudaMemcpyDeviceToHost) != cudaSuccess) return false;
   *aI = t.aI.v;
   *daI = t.aI.d;
-  return flat_comp(h, which == 0 ? u->df : u->dp, which == 0, comp, static_cast<double *>(u->ph));
+  *out = comp_view(h, which == 0 ? u->df : u->dp, which == 0, comp);
+  return true;
 }
 
 } // namespace clb

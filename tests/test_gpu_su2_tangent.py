@@ -289,3 +289,28 @@ def test_fp32_observable_and_its_derivative_on_a_fine_lattice(N):
     for x, y in zip(res["fp32"], res["fp64"]):
         print(N, x, y, abs(x - y) / abs(y))
         assert abs(x - y) <= REL * abs(y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_plain_evolution_after_a_spectrum_and_a_second_tangent_begin_is_bitwise(precision):
+    # the spectrum's tangent component touches none of what the plain kicks read, and a second
+    # clb_tangent_begin ends the first form as clb_tangent_end does
+    from cosmolattice_b200 import Lattice
+
+    par, rp, m, f, p, sf = case(8, "VV2", True)
+    out = []
+    for tangent in (False, True):
+        lat = Lattice(m, rp, precision=precision)
+        lat.set_state(f, p, sf)
+        if tangent:
+            lat.tangent_begin([0, 0, 0, 0, 1, 0])
+        lat.initialize()
+        lat.evolve(7)
+        if tangent:
+            lat.tangent_spectrum(0, 11)
+            lat.tangent_begin([0, 0, 1, 1, 0, 0])
+            lat.tangent_end()
+        lat.evolve(6)
+        out.append(lat.get_state())
+        lat.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
