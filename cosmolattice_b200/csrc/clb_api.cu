@@ -76,7 +76,7 @@ int su2_tangent_energies(clb_handle *h, double *E, double *dE);
 bool su2_tangent_component(clb_handle *h, int which, int comp, CompView *out, double *aI, double *daI);
 
 const double *u1_component(clb_handle *h, int which, int comp, bool *gauge);
-const double *su2_component(clb_handle *h, int which, int comp, bool *gauge);
+bool su2_component(clb_handle *h, int which, int comp, CompView *out, bool *gauge);
 
 // gravitational waves of the scalar singlets (clb_gws.cu)
 void gw_kick_step(clb_handle *h);
@@ -1389,11 +1389,12 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
   if (!h->initialized) return h->fail(CLB_ESTATE, "clb_spectrum: call clb_initialize first");
   const bool gauge_model = h->u1 || h->su2;
   bool gauge_comp = false;
-  const double *plain = nullptr;
+  CompView view{nullptr, 1, false};
   if (gauge_model) {
     if (which < 0 || which > 1) return h->fail(CLB_EINVAL, "clb_spectrum: which must be 0 (field) or 1 (momentum)");
-    plain = h->u1 ? u1_component(h, which, comp, &gauge_comp) : su2_component(h, which, comp, &gauge_comp);
-    if (!plain) return h->fail(CLB_EINVAL, "clb_spectrum: component index out of range");
+    const bool found = h->u1 ? (view.p = u1_component(h, which, comp, &gauge_comp)) != nullptr
+                             : su2_component(h, which, comp, &view, &gauge_comp);
+    if (!found) return h->fail(CLB_EINVAL, "clb_spectrum: component index out of range");
   }
   if (!gauge_model && (which < 0 || which > 1 || comp < 0 || comp >= h->NS))
     return h->fail(CLB_EINVAL, "clb_spectrum: which must be 0 (field) or 1 (momentum) and comp a scalar index");
@@ -1434,8 +1435,8 @@ int spectrum_impl(clb_handle *h, int32_t which, int32_t comp, int32_t ps_type, i
     }
     h->spec_nbins_cap = nbins;
   }
-  if (plain) {
-    CLB_LAUNCH(h, K_SPECTRUM, k_spec_gather_plain<<<kElemBlocks, 256, 0, h->stream>>>(plain, h->d_spec, N));
+  if (gauge_model) {
+    gather_view(h, view, h->d_spec);
   } else {
     void *src = which == 0 ? h->fld[h->cf] : h->pi[h->cp];
     const size_t comp_off = (size_t)comp * (size_t)h->pd.comp;

@@ -29,18 +29,7 @@ static __global__ void __launch_bounds__(256) k_spec_gather(const R *__restrict_
   }
 }
 
-// Unpadded N^3 component (x slowest) -> real input of an in-place R2C transform.
-static __global__ void __launch_bounds__(256) k_spec_gather_plain(const double *__restrict__ src, double *__restrict__ dst, int N)
-{
-  const long long pitch = 2LL * (N / 2 + 1);
-  for (long long r = blockIdx.x; r < (long long)N * N; r += gridDim.x) {
-    const double *s = src + r * N;
-    double *d = dst + r * pitch;
-    for (int z = threadIdx.x; z < N; z += blockDim.x) d[z] = s[z];
-  }
-}
-
-// Unpadded N^3 component of storage type R, its elements stride apart -> real input of an in-place R2C
+// Unpadded N^3 component (x slowest) of storage type R, its elements stride apart -> real input of an in-place R2C
 // transform.
 template <class R>
 static __global__ void __launch_bounds__(256)

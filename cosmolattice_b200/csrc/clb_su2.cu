@@ -11,6 +11,7 @@
 #include "clb_su2_sweep.cuh"
 #include "clb_vv.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -20,6 +21,8 @@
 namespace clb {
 
 namespace {
+constexpr size_t kStageMax = (size_t)1 << 23; // elements of the staging buffer: 64 MiB
+
 // PITensor.h's GW source for lphi4SU2U1: the singlet S (component 0), the complex scalar phi
 // (1, 2) and the U(1) field (7..9, the arrays 3..5; momenta 7..9), in the order scalarSinglet + complexScalar +
 // electricU1 + magneticU1; the doublet and the SU(2) field source none.
@@ -245,7 +248,8 @@ __attribute__((visibility("hidden"))) int su2_create(clb_handle *h)
   ok = ok && cudaMemset(u->f, 0, u->nf * u->esz) == cudaSuccess;
   ok = ok && cudaMemset(u->p, 0, NP * h->n3 * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->ph, 12 * h->n3 * u->esz) == cudaSuccess;
-  ok = ok && cudaMalloc(&u->d_stage, h->n3 * sizeof(double)) == cudaSuccess;
+  u->stage_n = std::min(h->n3, kStageMax);
+  ok = ok && cudaMalloc(&u->d_stage, u->stage_n * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_st, sizeof(State)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_part, (size_t)kSU2Blocks * kMeas * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_sums, kMeas * sizeof(double)) == cudaSuccess;
@@ -318,46 +322,40 @@ CompView comp_view(const clb_handle *h, void *buf, bool field, int c)
   const double *p = comp_at<double>(h, buf, field, c, st);
   return CompView{p, st, false};
 }
-// The component from / to an FP64 array on the host or the device, through the staging buffer where
-// the device holds it in FP32 or among others; ordered on the handle's stream.
+// The component from / to an FP64 array on the host or the device, in runs through the staging buffer
+// where the device holds it in FP32 or among others; ordered on the handle's stream.
 cudaError_t set_comp(clb_handle *h, void *buf, bool field, int c, const double *src)
 {
   SU2Sector *u = h->su2;
-  int st;
-  const size_t bytes = h->n3 * sizeof(double);
-  if (!u->fp32) {
-    double *dst = comp_at<double>(h, buf, field, c, st);
-    if (st == 1) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, h->stream);
-    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src, bytes, cudaMemcpyDefault, h->stream);
+  const CompView v = comp_view(h, buf, field, c);
+  if (!v.f32 && v.stride == 1)
+    return cudaMemcpyAsync(const_cast<void *>(v.p), src, h->n3 * sizeof(double), cudaMemcpyDefault, h->stream);
+  for (size_t i = 0; i < h->n3; i += u->stage_n) {
+    const size_t n = std::min(u->stage_n, h->n3 - i);
+    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src + i, n * sizeof(double), cudaMemcpyDefault, h->stream);
     if (e != cudaSuccess) return e;
-    k_comp_set<double><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, dst, st, h->n3);
-  } else {
-    float *dst = comp_at<float>(h, buf, field, c, st);
-    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src, bytes, cudaMemcpyDefault, h->stream);
-    if (e != cudaSuccess) return e;
-    k_comp_set<float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, dst, st, h->n3);
+    if (v.f32)
+      k_comp_set<float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, static_cast<float *>(const_cast<void *>(v.p)) + i * v.stride, v.stride, n);
+    else
+      k_comp_set<double><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, static_cast<double *>(const_cast<void *>(v.p)) + i * v.stride, v.stride, n);
   }
   return cudaGetLastError();
 }
-// The component in FP64 as one array: its own place on the device or tmp (N^3).
-const double *flat_comp(clb_handle *h, void *buf, bool field, int c, double *tmp)
-{
-  int st;
-  if (!h->su2->fp32) {
-    const double *src = comp_at<double>(h, buf, field, c, st);
-    if (st == 1) return src;
-    k_comp_get<double><<<kSU2Blocks, 256, 0, h->stream>>>(src, st, tmp, h->n3);
-  } else {
-    const float *src = comp_at<float>(h, buf, field, c, st);
-    k_comp_get<float><<<kSU2Blocks, 256, 0, h->stream>>>(src, st, tmp, h->n3);
-  }
-  return tmp;
-}
 cudaError_t get_comp(clb_handle *h, void *buf, bool field, int c, double *dst)
 {
-  const double *src = flat_comp(h, buf, field, c, h->su2->d_stage);
-  const cudaError_t e = cudaGetLastError();
-  return e != cudaSuccess ? e : cudaMemcpyAsync(dst, src, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+  SU2Sector *u = h->su2;
+  const CompView v = comp_view(h, buf, field, c);
+  if (!v.f32 && v.stride == 1) return cudaMemcpyAsync(dst, v.p, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+  for (size_t i = 0; i < h->n3; i += u->stage_n) {
+    const size_t n = std::min(u->stage_n, h->n3 - i);
+    if (v.f32)
+      k_comp_get<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(v.p) + i * v.stride, v.stride, u->d_stage, n);
+    else
+      k_comp_get<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(v.p) + i * v.stride, v.stride, u->d_stage, n);
+    const cudaError_t e = cudaMemcpyAsync(dst + i, u->d_stage, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaGetLastError();
 }
 } // namespace
 
@@ -755,15 +753,15 @@ __attribute__((visibility("hidden"))) int su2_measure(clb_handle *h, double e0, 
   return CLB_OK;
 }
 
-// Device array of one state component (clb_spectrum): which 0 fields (22), 1 momenta (19); gauge
-// tells whether the component belongs to the U(1) or SU(2) field.
-__attribute__((visibility("hidden"))) const double *su2_component(clb_handle *h, int which, int comp, bool *gauge)
+// One state component where it lies (clb_spectrum): which 0 fields (22), 1 momenta (19); gauge tells
+// whether the component belongs to the U(1) or SU(2) field.
+__attribute__((visibility("hidden"))) bool su2_component(clb_handle *h, int which, int comp, CompView *out, bool *gauge)
 {
   SU2Sector *u = h->su2;
-  if (comp < 0 || comp >= (which == 0 ? NF : NP)) return nullptr;
+  if (comp < 0 || comp >= (which == 0 ? NF : NP)) return false;
   *gauge = comp >= 7;
-  // in FP64 as one array (in the staging buffer, ordered on the handle's stream, unless it is one)
-  return flat_comp(h, which == 0 ? u->f : u->p, which == 0, comp, u->d_stage);
+  *out = comp_view(h, which == 0 ? u->f : u->p, which == 0, comp);
+  return true;
 }
 
 // ---- tangent-linear form -------------------------------------------------------------------------

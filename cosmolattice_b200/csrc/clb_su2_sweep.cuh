@@ -19,7 +19,8 @@ struct SU2Sector {
   size_t esz = 8;
   State *d_st = nullptr;
   double *d_part = nullptr, *d_sums = nullptr;
-  double *d_stage = nullptr; // one FP64 component, for conversions
+  double *d_stage = nullptr; // FP64 values on their way in or out, stage_n at a time
+  size_t stage_n = 0;
   void *ph = nullptr;        // U(1) link phases (6 x N^3 pairs, storage type), kept by the drifts
   // kick sweeps: 0 one sweep, 1 two halves, 2 three parts, 3 four parts (S and phi; Phi; A; SU(2))
   // (CLB_SU2_SPLIT sets both forms).  su2_create takes four parts in FP64 and three in FP32, by

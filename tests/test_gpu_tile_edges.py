@@ -123,3 +123,47 @@ def test_su2_force_by_direction_is_the_whole_sweep(monkeypatch, precision, N, or
         lat.close()
     for a, b in zip(*out):
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_su2_state_round_trip_in_several_runs_of_the_staging_buffer(precision):
+    # 205^3 sites: a whole run of 2^23 and a remainder; every value is a whole number below 2^24, which
+    # FP32 holds
+    from cosmolattice_b200 import MODELS, Lattice, ParameterParser, RunParameters
+
+    N = 205
+    par = ParameterParser(params={"N": N, "kIR": 1.0, "dt": 0.005, "evolver": "VV2", "expansion": "true", "lambda": 1.0,
+                                  "qG": 50.0, "qH": 50.0, "SU2Doublet_initial_norm": "5.25151e18", "gU1s": 0.35, "gSU2s": 0.6})
+    rp = RunParameters(par)
+    m = MODELS["lphi4SU2U1"](par, rp)
+    base = np.arange(N ** 3, dtype=np.float64).reshape(N, N, N)
+    f, p = np.empty((22, N, N, N)), np.empty((19, N, N, N))
+    for c in range(22):
+        f[c] = base + c
+    for c in range(19):
+        p[c] = base + 100 + c
+    lat = Lattice(m, rp, precision=precision)
+    lat.set_state(f, p, {"aI": 1.0, "aSI": 1.0, "aIM": 1.0, "aDotI": 0.0, "aDotSI": 0.0})
+    g = lat.get_state()
+    lat.close()
+    assert np.array_equal(g[0].ravel(), f.ravel()) and np.array_equal(g[1].ravel(), p.ravel())
+
+
+def test_su2_handle_holds_no_more_than_its_state_and_phases():
+    # 22 fields, 19 momenta and 12 phases per site, a staging buffer of 64 MiB and small change (partial
+    # sums, the allocator's granularity: under 32 MiB)
+    import torch
+
+    from cosmolattice_b200 import MODELS, Lattice, ParameterParser, RunParameters
+
+    N = 256
+    par = ParameterParser(params={"N": N, "kIR": 1.0, "dt": 0.005, "evolver": "VV2", "expansion": "true", "lambda": 1.0,
+                                  "qG": 50.0, "qH": 50.0, "SU2Doublet_initial_norm": "5.25151e18", "gU1s": 0.35, "gSU2s": 0.6})
+    rp = RunParameters(par)
+    m = MODELS["lphi4SU2U1"](par, rp)
+    Lattice(m, rp).close()  # the context and the kernels are loaded
+    free = torch.cuda.mem_get_info()[0]
+    lat = Lattice(m, rp)
+    held = free - torch.cuda.mem_get_info()[0]
+    lat.close()
+    assert held <= 53 * 8 * N ** 3 + (96 << 20), held
