@@ -153,7 +153,7 @@ void sweep_sh(clb_handle *h, int kind, int fb, int pb, int fo, int po, double dt
   if (h->pdl_now)
     CLB_LAUNCH(h, kind,
                launch_pdl(k_sweep<R, NS, SH, DRIFT, KICK, RED>, h->sweep_grid, dim3(SH::TZ, SH::TY), h->sweep_smem,
-                          h->stream, h->tm_f[fb], h->tm_p[pb], static_cast<R *>(h->fld[fo]), static_cast<R *>(h->pi[po]),
+                          h, h->tm_f[fb], h->tm_p[pb], static_cast<R *>(h->fld[fo]), static_cast<R *>(h->pi[po]),
                           a, (const DevState *)h->d_st, h->d_part, h->d_err));
   else
     CLB_LAUNCH(h, kind,
@@ -368,7 +368,7 @@ void tail(clb_handle *h, uint32_t flags, int nblocks, double w = 0, double w2 = 
   h->rb_valid = false;
   TailOp op{flags, nblocks, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
   if (h->pdl_now)
-    CLB_LAUNCH(h, K_TAIL, launch_pdl(k_tail, dim3(1), dim3(kTailThreads), 0, h->stream, (const double *)h->d_part, op,
+    CLB_LAUNCH(h, K_TAIL, launch_pdl(k_tail, dim3(1), dim3(kTailThreads), 0, h, (const double *)h->d_part, op,
                                      h->d_st, h->sp));
   else
     CLB_LAUNCH(h, K_TAIL, k_tail<<<1, kTailThreads, 0, h->stream>>>(h->d_part, op, h->d_st, h->sp));
@@ -818,6 +818,7 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
     h->fb_H0 = cfg->H0;
     h->fb_t = cfg->t0;
   }
+  if (const char *env = std::getenv("CLB_PDL")) h->pdl = std::atoi(env) != 0;
   if (u1 || su2) {
     h->ws = ws;
     const int r = u1 ? u1_create(h) : su2_create(h);
@@ -852,7 +853,6 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
     h->bz = kShapeBZ[h->shape];
     h->by = kShapeBY[h->shape];
   }
-  if (const char *env = std::getenv("CLB_PDL")) h->pdl = std::atoi(env) != 0;
   const size_t box_bytes = (size_t)(h->bz + 2 * (16 / (int)h->esz)) * (size_t)(h->by + 2) * h->esz;
   const size_t slot = ((box_bytes + 127) / 128) * 128;
   const size_t stage_bytes = (size_t)h->NS * 2 * slot;

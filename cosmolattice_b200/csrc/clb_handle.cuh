@@ -53,7 +53,7 @@ struct clb_handle {
   int S = 3;          // sweep ring stages
   int rs = 0;         // FP32 split storage: current reference slot in DevState
   int shape = 0;      // sweep block shape: 0 ShapeW, 1 ShapeQ, 2 ShapeH (clb_sweep.cuh)
-  bool pdl = true;     // programmatic dependent launch in the fused VV loop (CLB_PDL=0: off)
+  bool pdl = true;     // programmatic dependent launches (CLB_PDL=0: off)
   bool pdl_now = false; // set while the fused loop issues its sweeps and tails
   int bz = 64, by = 8; // sites per block tile in z and y
   size_t sweep_smem = 0;
@@ -150,19 +150,20 @@ const char *const kKindNames[K_NKINDS] = {"scalar_fused_sweep", "scalar_kick_swe
                                           "gauge_reduce",       "u1_adjoint_sweep",  "initial_conditions",
                                           "gw_sweep"};
 
-// Launch with the programmatic-stream-serialization attribute: the kernel may start while the
-// previous kernel in the stream drains; it waits (griddep_wait) before touching dependent data.
+// Launch on the handle's stream with the programmatic-stream-serialization attribute (off with CLB_PDL=0):
+// the kernel may start while the previous kernel in the stream drains; it waits (griddep_wait) before
+// touching dependent data.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, const clb_handle *h, Args &&...args)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
+  cfg.stream = h->stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = h->pdl ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);

@@ -136,7 +136,7 @@ template <class S> void drift_tan_t(clb_handle *h, double w, bool lf)
 {
   SU2Sector *u = h->su2;
   CLB_LAUNCH(h, K_U1_DRIFT,
-             launch_pdl(k_drift_tan<S>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<S *>(u->f),
+             launch_pdl(k_drift_tan<S>, dim3(kSU2Blocks), dim3(256), 0, h, static_cast<S *>(u->f),
                         static_cast<S *>(u->df), static_cast<const S *>(u->p), static_cast<const S *>(u->dp), u->prm, w,
                         lf ? 1 : 0, (const TState *)u->d_tst, u->tan_cd));
 }
@@ -154,12 +154,12 @@ void drift(clb_handle *h, double w, bool lf, double dtd = -1.0)
   }
   if (u->fp32)
     CLB_LAUNCH(h, K_U1_DRIFT,
-               launch_pdl(su2d::k_drift<float>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<float *>(u->f),
+               launch_pdl(su2d::k_drift<float>, dim3(kSU2Blocks), dim3(256), 0, h, static_cast<float *>(u->f),
                           static_cast<const float *>(u->p), u->prm, w, lf ? 1 : 0, (const State *)u->d_st,
                           static_cast<float *>(u->ph), dtd));
   else
     CLB_LAUNCH(h, K_U1_DRIFT,
-               launch_pdl(su2d::k_drift<double>, dim3(kSU2Blocks), dim3(256), 0, h->stream, static_cast<double *>(u->f),
+               launch_pdl(su2d::k_drift<double>, dim3(kSU2Blocks), dim3(256), 0, h, static_cast<double *>(u->f),
                           static_cast<const double *>(u->p), u->prm, w, lf ? 1 : 0, (const State *)u->d_st,
                           static_cast<double *>(u->ph), dtd));
 }
@@ -185,10 +185,10 @@ void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 =
   SU2Sector *u = h->su2;
   TailOp op{flags, reduced ? kSU2Blocks : 0, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
   if (u->tangent)
-    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<Tan<double>>, dim3(1), dim3(su2d::kTailThreads), 0, h->stream,
+    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<Tan<double>>, dim3(1), dim3(su2d::kTailThreads), 0, h,
                                      (const double *)u->d_tpart, op, u->d_tst, u->prm));
   else
-    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<double>, dim3(1), dim3(su2d::kTailThreads), 0, h->stream,
+    CLB_LAUNCH(h, K_TAIL, launch_pdl(su2d::k_tail<double>, dim3(1), dim3(su2d::kTailThreads), 0, h,
                                      (const double *)u->d_part, op, u->d_st, u->prm));
 }
 

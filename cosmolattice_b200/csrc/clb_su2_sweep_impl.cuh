@@ -16,11 +16,11 @@ template <class S> void su2_sweep(clb_handle *h, int nk, bool rf, bool rp, const
   // of three and four the last two run in one launch (k_kick_links); reduction-only sweeps run whole
 #define CLB_SU2K1(NK, RF, RP, SECT)                                                                                     \
   CLB_LAUNCH(h, kind,                                                                                                   \
-             launch_pdl(k_kick<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, p, u->prm, kc,       \
+             launch_pdl(k_kick<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h, f, p, u->prm, kc,       \
                         (const State *)u->d_st, u->d_part, static_cast<const S *>(u->ph)))
 #define CLB_SU2KL(WA, NK, RF, RP)                                                                                          \
   CLB_LAUNCH(h, kind,                                                                                                  \
-             launch_pdl(k_kick_links<S, S, WA, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f,              \
+             launch_pdl(k_kick_links<S, S, WA, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h, f,              \
                         (const S *)nullptr, p, (S *)nullptr, u->prm, kc, (const State *)u->d_st, CoupDot{}, u->d_part, \
                         static_cast<const S *>(u->ph)))
 #define CLB_SU2K(NK, RF, RP)                                                                                            \
@@ -77,13 +77,13 @@ template <class S> void su2_sweep_tan(clb_handle *h, int nk, bool rf, bool rp, c
   S *p = static_cast<S *>(u->p), *dp = static_cast<S *>(u->dp);
 #define CLB_SU2T1(NK, RF, RP, SECT)                                                                                     \
   CLB_LAUNCH(h, kind,                                                                                                   \
-             launch_pdl(k_kick_tan<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h->stream, f, df, p, dp,       \
+             launch_pdl(k_kick_tan<S, NK, RF, RP, SECT>, dim3(kSU2Blocks), dim3(128), 0, h, f, df, p, dp,       \
                         u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart))
 #define CLB_SU2TL(NK, RF, RP)                                                                                          \
   do {                                                                                                                 \
     if constexpr (sizeof(S) == sizeof(double))                                                                         \
       CLB_LAUNCH(h, kind,                                                                                              \
-                 launch_pdl(k_kick_links<S, Tan<S>, false, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h->stream, f, df, \
+                 launch_pdl(k_kick_links<S, Tan<S>, false, NK, RF, RP>, dim3(kSU2Blocks), dim3(3 * 128), 0, h, f, df, \
                             p, dp, u->prm, kc, (const TState *)u->d_tst, u->tan_cd, u->d_tpart, (const S *)nullptr));  \
     else                                                                                                               \
       CLB_SU2T1(NK, RF, RP, 2);                                                                                        \

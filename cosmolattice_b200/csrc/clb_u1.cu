@@ -138,13 +138,13 @@ template <int NK, bool RF, bool RP, class S> void kick_t(clb_handle *h, int kind
       attr = true;
     }
     CLB_LAUNCH(h, kind,
-               launch_pdl(k_u1_kick_tile<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), U1Ring<S>::BYTES, h->stream,
+               launch_pdl(k_u1_kick_tile<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), U1Ring<S>::BYTES, h,
                           static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc, (const U1State *)u->d_st,
                           u->d_part, u->tile_lx, (S *)nullptr, (S *)nullptr));
     return;
   }
   CLB_LAUNCH(h, kind,
-             launch_pdl(k_u1_kick<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), 0, h->stream, static_cast<const S *>(u->f),
+             launch_pdl(k_u1_kick<NK, RF, RP, S>, dim3(kU1Blocks), dim3(256), 0, h, static_cast<const S *>(u->f),
                         static_cast<S *>(u->p), u->prm, kc, (const U1State *)u->d_st, u->d_part, (S *)nullptr,
                         (S *)nullptr));
 }
@@ -158,7 +158,7 @@ template <class S> void drift_t(clb_handle *h, double w, double dtd)
 {
   U1Sector *u = h->u1;
   CLB_LAUNCH(h, K_U1_DRIFT,
-             launch_pdl(k_u1_drift<S>, dim3(kU1Blocks), dim3(256), 0, h->stream, static_cast<S *>(u->f),
+             launch_pdl(k_u1_drift<S>, dim3(kU1Blocks), dim3(256), 0, h, static_cast<S *>(u->f),
                         static_cast<const S *>(u->p), h->n3, w, dtd, (const U1State *)u->d_st));
 }
 // field drifts of weight w over dt (the position Verlet's half drifts pass dt/2: halving is exact,
@@ -188,7 +188,7 @@ void tail(clb_handle *h, uint32_t flags, bool reduced, double w = 0, double w2 =
 {
   U1Sector *u = h->u1;
   TailOp op{flags, reduced ? kU1Blocks : 0, w, w2, hist_row >= 0 ? h->d_hist : nullptr, hist_row, fa, fb};
-  CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail, dim3(1), dim3(kU1TailThreads), 0, h->stream, (const double *)u->d_part, op,
+  CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail, dim3(1), dim3(kU1TailThreads), 0, h, (const double *)u->d_part, op,
                                    u->d_st, u->prm));
 }
 
@@ -239,7 +239,7 @@ template <int NK, bool RED, class S> void kick_save_t(clb_handle *h, const U1Kic
     }
     CLB_LAUNCH(h, K_U1_KICK,
                launch_pdl(k_u1_kick_tile<NK, RED, RED, S, true, true>, dim3(kU1Blocks), dim3(256), U1Ring<S>::BYTES,
-                          h->stream, static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc,
+                          h, static_cast<const S *>(u->f), static_cast<S *>(u->p), u->prm, kc,
                           (const U1State *)u->d_st, u->d_part, u->tile_lx, reinterpret_cast<S *>(slot),
                           reinterpret_cast<S *>(slot + half)));
     return;
@@ -302,7 +302,7 @@ void vv_run(clb_handle *h, int64_t nsteps, const SegSave *sv, bool hist = true, 
         U1Sector *u = h->u1;
         const TailOp a{T_STORE_FIELDS | T_STORE_PI2_I | T_VV_KICK_ONE, kU1Blocks, w, 0.0, nullptr, -1};
         const TailOp b{more ? (uint32_t)(T_VV_KICK_HALF | T_STORE_PI2_B | T_VV_DRIFT) : 0u, kU1Blocks, w, wn, nullptr, -1};
-        CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail_split, dim3(1), dim3(kU1TailThreads), 0, h->stream,
+        CLB_LAUNCH(h, K_TAIL, launch_pdl(k_u1_tail_split, dim3(1), dim3(kU1TailThreads), 0, h,
                                          (const double *)u->d_part, a, b, u->d_st, u->prm, sv->rec, k + 1));
       } else {
         k_u1_record<<<1, 1, 0, h->stream>>>(h->u1->d_st, sv->rec, k + 1);

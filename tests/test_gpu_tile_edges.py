@@ -4,7 +4,7 @@ maximum), and the lphi4SU2U1 site orders against each other."""
 import numpy as np
 import pytest
 
-from conftest import make_su2_case
+from conftest import make_su2_case, make_u1_case
 
 pytestmark = pytest.mark.gpu
 
@@ -167,3 +167,23 @@ def test_su2_handle_holds_no_more_than_its_state_and_phases():
     held = free - torch.cuda.mem_get_info()[0]
     lat.close()
     assert held <= 53 * 8 * N ** 3 + (96 << 20), held
+
+
+@pytest.mark.parametrize("make", [make_u1_case, make_su2_case])
+@pytest.mark.parametrize("evolver", ["VV2", "LF"])
+def test_gauge_loops_without_dependent_launches(monkeypatch, make, evolver):
+    # CLB_PDL=0 launches every kernel after the one before has drained: the same state to the last bit
+    from cosmolattice_b200 import Lattice
+
+    par, rp, m, f, p, sf = make(N=19, evolver=evolver, expansion=True, amp=3e-2)
+    res = []
+    for pdl in ("1", "0"):
+        monkeypatch.setenv("CLB_PDL", pdl)
+        lat = Lattice(m, rp)
+        lat.set_state(f, p, sf)
+        lat.initialize()
+        lat.evolve(6)
+        lat.sync()
+        res.append(lat.get_state())
+        lat.close()
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1]) and res[0][2] == res[1][2]
