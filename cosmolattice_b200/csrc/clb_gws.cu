@@ -35,6 +35,7 @@
 #include "clb_vv.h"
 
 #include <cmath>
+#include <cstdlib>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -297,7 +298,8 @@ int clb_gws_enable(clb_handle *h)
     gw_destroy(h);
     return h->fail(CLB_ENOMEM, std::string("clb_gws_enable: ") + cudaGetErrorString(e));
   }
-  alloc_pair(&g->u2, &g->pi2, bytes); // without it the drift and the kick run as two sweeps
+  const char *pair = std::getenv("CLB_GW_PAIR");
+  if (!pair || std::atoi(pair) != 0) alloc_pair(&g->u2, &g->pi2, bytes); // without it the drift and the kick run as two sweeps
   return CLB_OK;
 }
 

@@ -15,7 +15,7 @@ import math
 import numpy as np
 import pytest
 
-from conftest import make_scalar_case
+from conftest import make_scalar_case, make_su2_case, make_u1_case
 
 pytestmark = pytest.mark.gpu
 
@@ -305,3 +305,38 @@ def test_run_writes_gw_files(tmp_path):
     vals = np.array([list(map(float, l.split())) for l in lines[1:]])
     assert vals[0, 1] == 0.0 and np.all(vals[1:, 1] > 0)  # the GWs start at zero and grow
     assert (tmp_path / "spectra_energy_gws.txt").exists()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("model,evolver,extra", [
+    ("lphi4", "VV4", None), ("lphi4", "LF", None), ("lphi4", "PV2", None),
+    ("lphi4", "VV2", {"fixedBackground": "true", "H0": 2.0e18, "omegaEoS": 0.0}),
+    ("u1", "VV2", None), ("u1", "LF", None), ("su2", "PV2", None),
+    ("su2", "LF", {"fixedBackground": "true", "H0": 2.0e18, "omegaEoS": 0.0})])
+def test_drift_and_kick_in_one_sweep_are_the_two_sweeps(monkeypatch, model, evolver, extra, precision):
+    # without the second pair of arrays (no memory for it; here CLB_GW_PAIR=0) the drift of a step and
+    # the kick of the next run as two sweeps: the same GW state over several calls, to the last bit in
+    # FP64, whose every rounding is pinned; FP32 products may contract, so there ten steps' few roundings
+    # of 6e-8 of the largest value are allowed (2e-6)
+    from cosmolattice_b200 import Lattice
+
+    make = {"u1": make_u1_case, "su2": make_su2_case}.get(model)
+    if make:
+        _, rp, m, f, p, sf = make(N=11, evolver=evolver, expansion=True, extra=extra)
+    else:
+        _, rp, m, f, p, sf = make_scalar_case(N=19, evolver=evolver, model="lphi4", amp=1e-2, extra=extra)
+    out = []
+    for pair in ("1", "0"):
+        monkeypatch.setenv("CLB_GW_PAIR", pair)
+        lat = Lattice(m, rp, precision=precision)
+        lat.gws_enable()
+        lat.set_state(f, p, sf)
+        lat.initialize()
+        for n in (5, 1, 4):
+            lat.evolve(n)
+        lat.sync()
+        out.append(lat.gws_get_state() + lat.get_state()[:2])
+        lat.close()
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= (0 if precision == "fp64" else 2e-6) * np.abs(b).max()
+    assert np.abs(out[0][0]).max() > 0
