@@ -38,7 +38,6 @@ constexpr size_t kStageMin = (size_t)1 << 23; // host-transfer staging: >= 64 Mi
 constexpr int kDefaultShapeFP64 = 0;          // ShapeW
 constexpr int kDefaultShapeFP32 = 4;          // ShapeK
 constexpr int kMaxRun = 22;                   // longest x-run of one sweep block
-constexpr int kMaxRunLarge = 32;              // ... of a large FP64 lattice
 
 } // namespace
 
@@ -95,28 +94,30 @@ namespace {
 
 
 // Sweep geometry: bz x by (z, y) sites per block and x-runs of LX planes.  A block's time goes as its
-// planes plus about one (its prologue and the halo planes), and the grid runs in waves of the resident
-// blocks, so the runs minimise waves x (LX + 0.8); runs longer than 22 planes lose L2 reuse between
-// neighbouring tiles.  us per VV2 step, this rule against runs of two waves of blocks or 32 planes:
-// 125^3 two fields FP64 43.8 against 50.4, 96^3 FP64 17.5 / 20.6, 128^3 FP32 17.5 / 22.1, 192^3
-// two fields FP64 113.9 / 125.4, 384^3 FP32 198.8 / 201.5.  From 20 waves on (512^3) the length of a
-// run matters little to the waves (FP64 790 at 16, 27 and 32 planes), and longer FP64 runs spare halo
-// planes, which counts under the power cap: 200 steps and the read 207.0 ms at 32, 208.6 at 16.  FP32
-// keeps 22 (384^3, 200 steps and the read 56.0 ms, 56.6 at 32).
+// planes plus about one (its prologue and the halo planes).  While the grid is a few waves of resident
+// blocks, whole waves matter, and the runs minimise waves x (LX + 0.8): us per VV2 step against runs
+// of 22 planes, 128^3 FP64 23.2 / 34.4, 192^3 57.9 / 68.2, 125^3 with two fields 41.5 / 54.6, 128^3 FP32
+// 16.2 / 28.0, 160^3 with two fields 81.8 / 89.6.  From three waves on the blocks no longer finish together,
+// and the fewest halo planes win: equal runs of at most 22 planes, beyond which neighbouring tiles' reuse in L2 is lost (22 / the
+// waves' choice / 32: 288^3 FP64 180.6 / 184.9 / 189.5, 384^3 380 / 385 / 392, 512^3 882 / 891 / 882, two
+// fields 256^3 249 / 258 / 266, 384^3 795 / 818 / 810; FP32 288^3 119.8 / 122.6 / 129.3, 384^3 203 / 209 / 209,
+// 512^3 455 / 462 / 460; the worst, 352^3 FP32, 181 / 177 / 187).
 void setup_geometry(clb_handle *h, int blocks_per_sm)
 {
   const int N = h->N;
   const int gx = (N + h->bz - 1) / h->bz, gy = (N + h->by - 1) / h->by;
   const long long slots = 148LL * std::max(1, blocks_per_sm), tiles = (long long)gx * gy;
-  const bool large = h->cfg.precision != CLB_PREC_FP32_SPLIT && tiles * ((N + kMaxRun - 1) / kMaxRun) > 20 * slots;
-  int LX = 1;
-  double best = 0;
-  for (int l = std::min(N, large ? kMaxRunLarge : kMaxRun); l >= 1; --l) {
-    const long long blocks = tiles * ((N + l - 1) / l);
-    const double cost = (double)((blocks + slots - 1) / slots) * (l + 0.8);
-    if (best == 0 || cost < best) {
-      best = cost;
-      LX = l;
+  const int long_runs = (N + kMaxRun - 1) / kMaxRun;
+  int LX = (N + long_runs - 1) / long_runs;
+  if (tiles * long_runs < 3 * slots) {
+    double best = 0;
+    for (int l = std::min(N, kMaxRun); l >= 1; --l) {
+      const long long blocks = tiles * ((N + l - 1) / l);
+      const double cost = (double)((blocks + slots - 1) / slots) * (l + 0.8);
+      if (best == 0 || cost < best) {
+        best = cost;
+        LX = l;
+      }
     }
   }
   if (const char *env = std::getenv("CLB_SWEEP_XS")) {
