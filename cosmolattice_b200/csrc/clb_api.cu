@@ -840,7 +840,6 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
   a.N = h->N;
   a.inv_dx2 = 1.0 / (cfg->dx * cfg->dx);
   a.cs.mc = ScalarModel::couplings(md->couplings);
-  // ring depth: as many plane stages as fit in ~48 KiB, at least 3 (planes x, x+1 and one in flight)
   // sweep shape: default per storage type and field count, CLB_SWEEP_SHAPE=0..4 overrides (one field)
   h->shape = (h->NS == 1) ? (h->fp32 ? kDefaultShapeFP32 : kDefaultShapeFP64) : 0;
   if (const char *env = std::getenv("CLB_SWEEP_SHAPE")) {
@@ -857,7 +856,8 @@ int clb_create(const clb_config *cfg, const clb_model_desc *md, clb_handle **out
   const size_t box_bytes = (size_t)(h->bz + 2 * (16 / (int)h->esz)) * (size_t)(h->by + 2) * h->esz;
   const size_t slot = ((box_bytes + 127) / 128) * 128;
   const size_t stage_bytes = (size_t)h->NS * 2 * slot;
-  // two fields: the sweep's registers allow two blocks per SM, which leaves room for a deeper ring
+  // ring depth: as many plane stages as fit in 32 KiB, between 3 (planes x, x+1 and one in flight) and 8;
+  // two fields: the sweep's registers allow two blocks per SM, which leaves room for a deeper ring in 96 KiB
   // (192^3 FP64 126 -> 121.5 us per step at four stages instead of three)
   size_t ring_budget = h->NS == 2 ? 96 * 1024 : 32 * 1024;
   if (const char *env = std::getenv("CLB_SWEEP_RING_KB")) ring_budget = (size_t)std::max(8, std::atoi(env)) * 1024;

@@ -17,8 +17,9 @@ namespace clb {
 //   q0 = RN(x rh + RN(x rl)), rh + rl = 1/y to twice the precision, so q0 is a faithful rounding;
 //   q  = RN(q0 + rh RN(x - q0 y)), Markstein's correction (IBM J. Res. Dev. 34, 1990): with rh =
 //        RN(1/y) and q0 faithful the remainder is exact and q = RN(x / y).
-// (Outside |x| in about [1e-290, 1e290] / max(1, 1/y) the last bit can differ, and an infinite x
-// gives NaN: a run whose state has left the finite numbers reports CLB_ENONFINITE either way.)
+// (Outside |x| in about [1e-290, 1e290] / max(1, 1/y) the last bit can differ, a negative zero may lose
+// its sign, and an infinite x gives NaN: a run whose state has left the finite numbers reports
+// CLB_ENONFINITE either way.)
 // The compiler's division is a call on its slow path and a branch per quotient, which serialises
 // the ~30 of a gauge kick's site: with div_by the lphi4U1 FP64 kick at 128^3 went from 190 to 118
 // us, the lphi4SU2U1 FP64 step at 192^3 from 4.54 to 4.00 ms and its tangent step at 80^3 from 2.34

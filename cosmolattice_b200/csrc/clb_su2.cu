@@ -59,7 +59,6 @@ Params su2_params(const clb_handle *h)
   a.n3 = h->n3;
   a.dx = c.dx;
   a.dx2 = c.dx * c.dx;
-  a.inv_dx2 = 1.0 / (c.dx * c.dx);
   a.inv_dx = 1.0 / c.dx;
   const float dxf = (float)c.dx;
   a.ddx = make_div(a.dx, dxf);

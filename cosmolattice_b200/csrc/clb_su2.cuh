@@ -46,7 +46,7 @@ constexpr int kMeas = 64; // measurement partial slots
 struct Params {
   int N;
   size_t n3;
-  double dx, dx2, inv_dx2, inv_dx;
+  double dx, dx2, inv_dx;
   DivBy ddx, ddx2;          // divisions by dx and dx^2
   double ngrad;             // (1/dx)^3 / gS (su2kernels.h:44), in the form's arithmetic below
   float ngrad_f;

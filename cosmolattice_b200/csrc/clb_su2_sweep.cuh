@@ -23,14 +23,14 @@ struct SU2Sector {
   size_t stage_n = 0;
   void *ph = nullptr;        // U(1) link phases (6 x N^3 pairs, storage type), kept by the drifts
   // kick sweeps: 0 one sweep, 1 two halves, 2 three parts, 3 four parts (S and phi; Phi; A; SU(2))
-  // (CLB_SU2_SPLIT sets both forms).  su2_create takes four parts in FP64 and three in FP32, by
-  // timing at 192^3 VV2, when every part still had a thread per site and the fields were one array
-  // per component (ms per step): FP64 9.20 whole, 6.53 halves, 5.10 three parts, 4.73 four parts;
-  // FP32 4.93, 3.18, 2.90, 2.93.  The tangent-linear sweep takes four parts in both (256^3 VV2, ms
-  // per tangent step, three / four parts: FP64 37.9, 31.4; FP32 21.5, 19.5).  The SU(2) part has a
-  // thread per site and direction (k_kick_links; the FP32 tangent form one per site), and in the plain
-  // form A with it, with which a step takes 2.83 ms at 192^3 FP64.  Every form gives the
-  // same state to the last bit.
+  // (CLB_SU2_SPLIT sets both forms).  The SU(2) part has a thread per site and direction (k_kick_links;
+  // the FP32 tangent form one per site), and in the plain form A with it.  su2_create takes four parts in
+  // FP64 and three in FP32: ms per VV2 step whole / halves / three / four parts, FP64 192^3 6.19 / 3.09 /
+  // 2.85 / 2.82, 256^3 15.7 / 7.76 / 6.97 / 6.86, 96^3 0.660 / 0.380 / 0.369 / 0.364; FP32 192^3 3.32 / 2.00 /
+  // 1.95 / 1.98, 256^3 8.50 / 4.87 / 4.64 / 4.72, 95^3 0.383 / 0.246 / 0.253 / 0.252 (48^3 is fastest in
+  // halves: 0.061 against 0.065, FP32 0.044 against 0.047).  The tangent-linear sweep takes four parts in
+  // both (three / four: FP64 80^3 0.790 / 0.690, 128^3 2.91 / 2.53; FP32 80^3 0.400 / 0.345, 128^3 1.37 /
+  // 1.24).  Every form gives the same state to the last bit.
   int split = 2;
   int tan_split = 3;
   int64_t steps_since_unitarize = 0;

@@ -12,7 +12,11 @@ namespace clb {
 // ~60 FP64 instructions on the reduction and its branches.  Up to 1/32 the Taylor polynomials to
 // x^7 and x^8 are exact to 0.03 of the last place, so the results are correctly rounded but for a
 // few in a hundred; beyond, the library's.  A gauge kick forms 6 (lphi4U1) to 21 (the tangent form of
-// lphi4SU2U1) of them per site.
+// lphi4SU2U1) of them per site.  Where a field has grown so far that some lanes of a warp are beyond
+// (phases of rms 0.0125 and more, dx g A), the kick takes both: us per VV2 step at rms 0.005 / 0.0125 /
+// 0.02 / 0.06, lphi4U1 128^3 FP64 160 / 167 / 189 / 194, 99^3 FP32 65 / 68 / 74 / 77 (271 and 110 at every
+// angle with the general function, before the other changes to these kicks); lphi4SU2U1, whose kicks
+// read stored phases, 128^3 FP64 883 / 884 / 887 / 887, 95^3 FP32 278 / 277 / 279 / 279.
 constexpr double kSmallPhase = 0.03125;
 
 #ifdef __CUDA_ARCH__

@@ -406,8 +406,6 @@ __attribute__((visibility("hidden"))) int u1_create(clb_handle *h)
   u->prm = make_params(h);
   u->fp32 = h->cfg.precision == CLB_PREC_FP32_SPLIT;
   u->esz = u->fp32 ? sizeof(float) : sizeof(double);
-  // x-run of the staged kick: 8 planes FP64, 32 FP32 (128^3 VV4, ms per step: FP64 0.726 / 0.751 /
-  // 0.742 for 8 / 16 / 32, FP32 0.340 / 0.340 / 0.325; the site-by-site kick 0.885 and 0.386)
   // x-runs of the staged kick: N / 16 planes, so that the tiles fill the chip at every size and the
   // two extra planes a run stages stay few.  us per VV2 step at runs of 4 / 8 / 16 / 32 planes:
   // FP64 64^3 32 / 45 / 71 / 126, 128^3 168 / 165 / 174 / 175; FP32 48^3 23 / 27 / 40 / 62,
