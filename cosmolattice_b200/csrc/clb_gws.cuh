@@ -39,26 +39,63 @@ constexpr int kGWBlocks = 148 * 8;
 __host__ __device__ constexpr int gw_pair_i(int k) { return k < 3 ? 0 : k < 5 ? 1 : 2; }
 __host__ __device__ constexpr int gw_pair_j(int k) { return k < 3 ? k : k < 5 ? k - 2 : 2; }
 
-// The GW sweep: with DRIFT first u += pow(a_SI, alpha - 3) (dt pi_u), then pi_u += h K(u; a_I), the
-// source src(s, x, y, z, xp, yp, zp, P) giving the anisotropic tensor P at site s = (x, y, z) (xp, yp,
-// zp: its forward neighbours' coordinates).  kA points at the device copy of pow(a_I, 1 + alpha), pd
-// at that of pow(a_SI, alpha - 3), or aSI at a_SI's (from_aSI: the position-Verlet tails keep a_SI as
-// the reference does, positionverlet.h:213-235, but their drift coefficient is a_I's).
+// pi_u += h K(u; a_I) at every site, the source src(s, x, y, z, xp, yp, zp, P) giving the
+// anisotropic tensor P at site s = (x, y, z) (xp, yp, zp: its forward neighbours' coordinates);
+// kA points at the device copy of pow(a_I, 1 + alpha).  The kick on its own: the first of a call, a sync's,
+// and every one of a handle without the second pair of arrays.  It loads its neighbours where they lie, at
+// 48 registers; in the form of the sweep below, without its drift, it waits for loads at a quarter of
+// the warps (128^3 FP64 117 us against 76; a call per step with GWs 189 us a step against 150, FP32 150
+// against 101).
+template <class R, class Src>
+__global__ void __launch_bounds__(256) k_gw_kick(const R *__restrict__ u, R *__restrict__ piu, int N, double inv_dx2d,
+                                                 double hd, const double *__restrict__ kA_ptr, Src src)
+{
+  using A = Ar<R>;
+  const size_t n3 = (size_t)N * N * N;
+  const R kA = (R)*kA_ptr, h = (R)hd, inv_dx2 = (R)inv_dx2d, two = R(2), third = R(1.0 / 3.0);
+  for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += (size_t)gridDim.x * blockDim.x) {
+    const int z = (int)(s % N), y = (int)((s / N) % N), x = (int)(s / ((size_t)N * N));
+    const int xp = x + 1 == N ? 0 : x + 1, xm = x == 0 ? N - 1 : x - 1;
+    const int yp = y + 1 == N ? 0 : y + 1, ym = y == 0 ? N - 1 : y - 1;
+    const int zp = z + 1 == N ? 0 : z + 1, zm = z == 0 ? N - 1 : z - 1;
+    R P[6];
+    src(s, x, y, z, xp, yp, zp, P);
+    const R tr3 = A::mul(A::add(A::add(P[0], P[3]), P[5]), third);
+    const R S[5] = {A::sub(P[0], tr3), P[1], P[2], A::sub(P[3], tr3), P[4]};
+    const R kA2 = A::mul(kA, two);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const R *U = u + (size_t)c * n3;
+      const R uc = U[s];
+      const R tx = A::sub(A::add(U[((size_t)xp * N + y) * N + z], U[((size_t)xm * N + y) * N + z]), A::mul(two, uc));
+      const R ty = A::sub(A::add(U[((size_t)x * N + yp) * N + z], U[((size_t)x * N + ym) * N + z]), A::mul(two, uc));
+      const R tz = A::sub(A::add(U[((size_t)x * N + y) * N + zp], U[((size_t)x * N + y) * N + zm]), A::mul(two, uc));
+      const R lap = A::mul(inv_dx2, A::add(A::add(tx, ty), tz));
+      const R K = A::add(A::mul(kA, lap), A::mul(kA2, S[c]));
+      piu[(size_t)c * n3 + s] = A::add(piu[(size_t)c * n3 + s], A::mul(h, K));
+    }
+  }
+}
+
+// The GW sweep between two steps: first u += pow(a_SI, alpha - 3) (dt pi_u), then the kick of k_gw_kick on
+// the drifted u.  pd points at the device copy of pow(a_SI, alpha - 3), or aSI at a_SI's (from_aSI: the
+// position-Verlet tails keep a_SI as the reference does, positionverlet.h:213-235, but their drift
+// coefficient is a_I's).
 //
-// Memory-bound: between two steps the drift of one and the kick of the next act on the same state,
-// so one sweep reads u and pi_u (10 values a site) and writes both, where a drift and a kick sweep
-// move 31.  A block marches a 32 x 8 (z, y) tile along LX planes.  Each thread loads its site (and
-// one thread in three a cell of the rows and columns next to the tile) two planes ahead into
-// registers, drifts the values when their plane comes and shares them through shared memory (two
-// planes, so one barrier per plane); the planes before and after stay in registers.  (Loads one plane
-// ahead: 145 us at 128^3 FP64; a cp.async ring of raw planes, drifted at each read: 130, held by
-// shared-memory reads.)  The neighbouring tiles read the undrifted state, so with DRIFT the sweep
-// writes another pair of arrays.  128^3 FP64: 83 us, against 36 (drift) + 76 (kick, a grid-stride
-// sweep) before.
+// Memory-bound: the drift and the kick act on the same state, so one sweep reads u and pi_u (10 values a
+// site) and writes both, where a drift and a kick sweep move 31.  A block marches a 32 x 8 (z, y) tile along
+// LX planes.  Each thread loads its site (and one thread in three a cell of the rows and columns next to
+// the tile) two planes ahead into registers, drifts the values when their plane comes and shares them
+// through shared memory (two planes, so one barrier per plane); the planes before and after stay in
+// registers.  (Loads one plane ahead: 145 us at 128^3 FP64; a cp.async ring of raw planes, drifted at each
+// read: 130, held by shared-memory reads.)  The neighbouring tiles read the undrifted state, so the sweep
+// writes another pair of arrays.  128^3 FP64: 81 us (ncu), against 36 (drift) + 76 (kick); what GWs add to
+// a step in the two forms, us: FP64 128^3 89 / 124, 192^3 246 / 397, 256^3 597 / 962; FP32 128^3 70 / 79,
+// 192^3 194 / 243.
 constexpr int kGWTileZ = 32, kGWTileY = 8;
-template <class R, class Src, bool DRIFT>
+template <class R, class Src>
 __global__ void __launch_bounds__(kGWTileZ *kGWTileY, 2)
-    k_gw_sweep(const R *__restrict__ u, const R *pi, R *__restrict__ uo, R *po, int N, int LX, double inv_dx2d, double dtd,
+    k_gw_sweep(const R *__restrict__ u, const R *__restrict__ pi, R *__restrict__ uo, R *__restrict__ po, int N, int LX, double inv_dx2d, double dtd,
                double hd, const double *__restrict__ kA_ptr, const double *__restrict__ pd_ptr,
                const double *__restrict__ aSI, double alpha, int from_aSI, Src src)
 {
@@ -67,8 +104,7 @@ __global__ void __launch_bounds__(kGWTileZ *kGWTileY, 2)
   __shared__ R sm[2][5][PL];
   const size_t n3 = (size_t)N * N * N, plane = (size_t)N * N;
   const R kA = (R)*kA_ptr, h = (R)hd, inv_dx2 = (R)inv_dx2d, two = R(2), third = R(1.0 / 3.0), dt = (R)dtd;
-  R pd = R(0);
-  if (DRIFT) pd = from_aSI ? (R)apow(*aSI, alpha - 3) : (R)*pd_ptr;
+  const R pd = from_aSI ? (R)apow(*aSI, alpha - 3) : (R)*pd_ptr;
   const int tz = threadIdx.x % BZ, ty = threadIdx.x / BZ;
   const int z0 = blockIdx.x * BZ, y0 = blockIdx.y * BY, x0 = blockIdx.z * LX, x1 = min(N, x0 + LX);
   const int hz = min(BZ, N - z0), hy = min(BY, N - y0);
@@ -101,15 +137,15 @@ __global__ void __launch_bounds__(kGWTileZ *kGWTileY, 2)
     for (int c = 0; c < 5; ++c) {
       if (valid) {
         r.u[c] = u[c * n3 + o + own];
-        if (DRIFT) r.p[c] = pi[c * n3 + o + own];
+        r.p[c] = pi[c * n3 + o + own];
       }
       if (with_halo && hal) {
         r.hu[c] = u[c * n3 + o + halo];
-        if (DRIFT) r.hp[c] = pi[c * n3 + o + halo];
+        r.hp[c] = pi[c * n3 + o + halo];
       }
     }
   };
-  auto moved = [&](R v, R p) -> R { return DRIFT ? drift_val<R>(v, p, pd, dt) : v; };
+  auto moved = [&](R v, R p) -> R { return drift_val<R>(v, p, pd, dt); };
   auto share = [&](int b, const R (&v)[5], const Raw &r) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
@@ -160,8 +196,8 @@ __global__ void __launch_bounds__(kGWTileZ *kGWTileY, 2)
         const R lap = A::mul(inv_dx2, A::add(A::add(tx, tyv), tzv));
         const R K = A::add(A::mul(kA, lap), A::mul(kA2, S[c]));
         const size_t i = c * n3 + s;
-        if (DRIFT) uo[i] = uc;
-        po[i] = A::add(DRIFT ? pc[c] : pi[i], A::mul(h, K));
+        uo[i] = uc;
+        po[i] = A::add(pc[c], A::mul(h, K));
       }
     }
     __syncthreads();
@@ -196,32 +232,25 @@ __global__ void __launch_bounds__(256) k_gw_drift_a(R *__restrict__ u, const R *
     u[i] = drift_val<R>(u[i], piu[i], pd, dt);
 }
 
-// A GW kick of weight w, with drift after the drift of the step before (launch_gw_drift).  Runs are
-// 32 planes, halved until there are four blocks per SM.
-template <class R, class Src, bool DRIFT>
-inline void launch_gw_sweep(GWSector *g, int N, double dx, double dt, double w, const double *kA, const double *pd,
-                            const double *aSI, double alpha, bool from_aSI, const Src &src, cudaStream_t stream)
-{
-  const int gz = (N + kGWTileZ - 1) / kGWTileZ, gy = (N + kGWTileY - 1) / kGWTileY;
-  int LX = 32;
-  while (LX > 4 && (long long)gz * gy * ((N + LX - 1) / LX) < 4LL * 148) LX /= 2;
-  R *u = static_cast<R *>(g->u), *pi = static_cast<R *>(g->pi);
-  k_gw_sweep<R, Src, DRIFT><<<dim3(gz, gy, (N + LX - 1) / LX), kGWTileZ * kGWTileY, 0, stream>>>(
-      u, pi, static_cast<R *>(g->u2), DRIFT ? static_cast<R *>(g->pi2) : pi, N, LX, 1.0 / (dx * dx), dt, w * dt, kA, pd, aSI,
-      alpha, from_aSI, src);
-  if (DRIFT) {
-    std::swap(g->u, g->u2);
-    std::swap(g->pi, g->pi2);
-  }
-}
+// A GW kick of weight w, with drift after the drift of the step before (launch_gw_drift) in one sweep,
+// whose runs are 32 planes, halved until there are four blocks per SM.
 template <class R, class Src>
 inline void launch_gw_kick(GWSector *g, int N, double dx, double dt, double w, bool drift, const double *kA, const double *pd,
                            const double *aSI, double alpha, bool from_aSI, const Src &src, cudaStream_t stream)
 {
-  if (drift)
-    launch_gw_sweep<R, Src, true>(g, N, dx, dt, w, kA, pd, aSI, alpha, from_aSI, src, stream);
-  else
-    launch_gw_sweep<R, Src, false>(g, N, dx, dt, w, kA, pd, aSI, alpha, from_aSI, src, stream);
+  R *u = static_cast<R *>(g->u), *pi = static_cast<R *>(g->pi);
+  if (!drift) {
+    k_gw_kick<R, Src><<<kGWBlocks, 256, 0, stream>>>(u, pi, N, 1.0 / (dx * dx), w * dt, kA, src);
+    return;
+  }
+  const int gz = (N + kGWTileZ - 1) / kGWTileZ, gy = (N + kGWTileY - 1) / kGWTileY;
+  int LX = 32;
+  while (LX > 4 && (long long)gz * gy * ((N + LX - 1) / LX) < 4LL * 148) LX /= 2;
+  k_gw_sweep<R, Src><<<dim3(gz, gy, (N + LX - 1) / LX), kGWTileZ * kGWTileY, 0, stream>>>(
+      u, pi, static_cast<R *>(g->u2), static_cast<R *>(g->pi2), N, LX, 1.0 / (dx * dx), dt, w * dt, kA, pd, aSI, alpha, from_aSI,
+      src);
+  std::swap(g->u, g->u2);
+  std::swap(g->pi, g->pi2);
 }
 
 // Launches the GW drift: with the tails' coefficient pd (VV, leapfrog), or from a_SI (position Verlet).
