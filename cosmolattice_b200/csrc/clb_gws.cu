@@ -193,27 +193,26 @@ cudaError_t gw_scratch(clb_handle *h, double **out)
 namespace clb {
 
 // The gauge models' GW kick and drift (clb_u1.cu, clb_su2.cu).
-void u1_gw_kick(clb_handle *h, double w, bool drift);
+void u1_gw_kick(clb_handle *h, double w);
 void u1_gw_drift(clb_handle *h);
-void su2_gw_kick(clb_handle *h, double w, bool drift);
+void su2_gw_kick(clb_handle *h, double w);
 void su2_gw_drift(clb_handle *h);
 bool su2_tangent_active(const clb_handle *h);
 
-// Runs one GW kick (weight w of dt) at the handle's current fields and a_I, with drift after the drift
-// of the step just taken in the same sweep.
-__attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w, bool drift)
+// The scalar singlets' GW kick (weight w of dt) at the handle's current fields and a_I, or with drift the
+// drift of the step just taken and the next step's whole kick in one sweep.
+static void scalar_gw_kick(clb_handle *h, double w, bool drift)
 {
   GWSector *g = h->gw;
-  g->synced = false;
-  h->rb_valid = false;
-  if (h->u1) return u1_gw_kick(h, w, drift);
-  if (h->su2) return su2_gw_kick(h, w, drift);
   auto go = [&](auto zero, auto ns) {
     using R = decltype(zero);
     using Src = ScalarGWSource<R, decltype(ns)::value>;
     const Src src{static_cast<const R *>(h->fld[h->cf]), h->pd, make_div(h->cfg.dx, (float)h->cfg.dx)};
-    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, Src>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &h->d_st->kick_A, &h->d_st->drift_p,
-                                                &h->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
+    if (drift)
+      CLB_LAUNCH(h, K_GW, (launch_gw_sweep<R, Src>(g, h->N, h->cfg.dx, h->cfg.dt, &h->d_st->kick_A, &h->d_st->drift_p,
+                                                   &h->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
+    else
+      CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, Src>(g, h->N, h->cfg.dx, h->cfg.dt, w, &h->d_st->kick_A, src, h->stream)));
   };
   using One = std::integral_constant<int, 1>;
   using Two = std::integral_constant<int, 2>;
@@ -221,6 +220,16 @@ __attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w, bool
     h->NS == 1 ? go(0.0f, One{}) : go(0.0f, Two{});
   else
     h->NS == 1 ? go(0.0, One{}) : go(0.0, Two{});
+}
+
+// Runs one GW kick (weight w of dt) at the handle's current fields and a_I.
+__attribute__((visibility("hidden"))) void gw_kick(clb_handle *h, double w)
+{
+  h->gw->synced = false;
+  h->rb_valid = false;
+  if (h->u1) return u1_gw_kick(h, w);
+  if (h->su2) return su2_gw_kick(h, w);
+  scalar_gw_kick(h, w, false);
 }
 
 // Runs one GW drift with the a_SI of the matter step just taken.
@@ -243,13 +252,16 @@ __attribute__((visibility("hidden"))) void gw_drift(clb_handle *h)
 }
 
 // The GW kick before a matter step (evolver.h:104-107): half a step after a sync, else a whole one.
-__attribute__((visibility("hidden"))) void gw_kick_step(clb_handle *h) { gw_kick(h, h->gw->synced ? 0.5 : 1.0, false); }
+__attribute__((visibility("hidden"))) void gw_kick_step(clb_handle *h) { gw_kick(h, h->gw->synced ? 0.5 : 1.0); }
 
 // The GW drift after a matter step and, with more to come in the call, the next step's GW kick: nothing
 // that either reads changes in between.
 __attribute__((visibility("hidden"))) void gw_between_steps(clb_handle *h, bool more)
 {
-  if (more && h->gw->u2) return gw_kick(h, 1.0, true);
+  if (more && h->gw->u2) {
+    h->rb_valid = false;
+    return scalar_gw_kick(h, 1.0, true);
+  }
   gw_drift(h);
   if (more) gw_kick_step(h);
 }
@@ -257,7 +269,7 @@ __attribute__((visibility("hidden"))) void gw_between_steps(clb_handle *h, bool 
 // Evolver::sync (evolver.h:132-138): the half kick to integer time, if the momenta are unsynced.
 __attribute__((visibility("hidden"))) void gw_sync(clb_handle *h)
 {
-  if (!h->gw->synced) gw_kick(h, 0.5, false);
+  if (!h->gw->synced) gw_kick(h, 0.5);
   h->gw->synced = true;
 }
 
@@ -298,8 +310,9 @@ int clb_gws_enable(clb_handle *h)
     gw_destroy(h);
     return h->fail(CLB_ENOMEM, std::string("clb_gws_enable: ") + cudaGetErrorString(e));
   }
+  // without a second pair the drift and the kick run as two sweeps
   const char *pair = std::getenv("CLB_GW_PAIR");
-  if (!pair || std::atoi(pair) != 0) alloc_pair(&g->u2, &g->pi2, bytes); // without it the drift and the kick run as two sweeps
+  if (!gauge && (pair ? std::atoi(pair) != 0 : gw_sweep_pays(2 * bytes))) alloc_pair(&g->u2, &g->pi2, bytes);
   return CLB_OK;
 }
 

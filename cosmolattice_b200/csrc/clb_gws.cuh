@@ -232,23 +232,51 @@ __global__ void __launch_bounds__(256) k_gw_drift_a(R *__restrict__ u, const R *
     u[i] = drift_val<R>(u[i], piu[i], pd, dt);
 }
 
-// A GW kick of weight w, with drift after the drift of the step before (launch_gw_drift) in one sweep,
-// whose runs are 32 planes, halved until there are four blocks per SM.
+// A GW kick of weight w.
 template <class R, class Src>
-inline void launch_gw_kick(GWSector *g, int N, double dx, double dt, double w, bool drift, const double *kA, const double *pd,
-                           const double *aSI, double alpha, bool from_aSI, const Src &src, cudaStream_t stream)
+inline void launch_gw_kick(GWSector *g, int N, double dx, double dt, double w, const double *kA, const Src &src, cudaStream_t stream)
 {
-  R *u = static_cast<R *>(g->u), *pi = static_cast<R *>(g->pi);
-  if (!drift) {
-    k_gw_kick<R, Src><<<kGWBlocks, 256, 0, stream>>>(u, pi, N, 1.0 / (dx * dx), w * dt, kA, src);
-    return;
+  k_gw_kick<R, Src><<<kGWBlocks, 256, 0, stream>>>(static_cast<const R *>(g->u), static_cast<R *>(g->pi), N, 1.0 / (dx * dx),
+                                                   w * dt, kA, src);
+}
+
+// Whether the sweep pays for a state (u and pi_u) of so many bytes.  Below 37 MB both pairs of it stay in
+// the 126 MB of L2, and from 60 MB on the state in place does not either; in between the in-place drift and
+// kick find it there and the sweep's two pairs do not fit.  One / two sweeps, us per VV2 step with GWs: FP64
+// 64^3 (21 MB) 22.1 / 26.9, 80^3 (41 MB) 39.1 / 37.2, 96^3 (71 MB) 53.8 / 64.0, 128^3 107 / 145, 256^3 695 /
+// 1043; FP32 96^3 (35 MB) 40.1 / 43.3, 100^3 (40 MB) 52.5 / 45.9, 112^3 (56 MB) 66.3 / 60.7, 128^3 (84 MB)
+// 82.5 / 94.1, 256^3 517 / 604.  (The gauge models' sources hold the sweep up at every size, lphi4U1 128^3
+// 498 / 413, so they always take two.)
+inline bool gw_sweep_pays(size_t state_bytes) { return state_bytes <= 37500000 || state_bytes > 60000000; }
+
+// The sweep's runs: whole waves of the resident blocks (two per SM) x (the run + 3 planes, a block's start),
+// between 4 and 32 planes.  128^3 FP64 107 us a step at this rule's 32 against 113 at 8 (four blocks per SM),
+// 96^3 53.8 at 12 against 57.8 at 4, 176^3 261 at 16 against 274 at 32.
+inline int gw_run(int N)
+{
+  const long long tiles = (long long)((N + kGWTileZ - 1) / kGWTileZ) * ((N + kGWTileY - 1) / kGWTileY), slots = 2 * 148;
+  int LX = 1;
+  long long best = 0;
+  for (int l = N < 32 ? N : 32; l >= (N < 4 ? N : 4); --l) {
+    const long long cost = (tiles * ((N + l - 1) / l) + slots - 1) / slots * (l + 3);
+    if (best == 0 || cost < best) {
+      best = cost;
+      LX = l;
+    }
   }
+  return LX;
+}
+
+// The drift of a step (launch_gw_drift) and the kick of the next.
+template <class R, class Src>
+inline void launch_gw_sweep(GWSector *g, int N, double dx, double dt, const double *kA, const double *pd, const double *aSI,
+                            double alpha, bool from_aSI, const Src &src, cudaStream_t stream)
+{
   const int gz = (N + kGWTileZ - 1) / kGWTileZ, gy = (N + kGWTileY - 1) / kGWTileY;
-  int LX = 32;
-  while (LX > 4 && (long long)gz * gy * ((N + LX - 1) / LX) < 4LL * 148) LX /= 2;
+  const int LX = gw_run(N);
   k_gw_sweep<R, Src><<<dim3(gz, gy, (N + LX - 1) / LX), kGWTileZ * kGWTileY, 0, stream>>>(
-      u, pi, static_cast<R *>(g->u2), static_cast<R *>(g->pi2), N, LX, 1.0 / (dx * dx), dt, w * dt, kA, pd, aSI, alpha, from_aSI,
-      src);
+      static_cast<const R *>(g->u), static_cast<const R *>(g->pi), static_cast<R *>(g->u2), static_cast<R *>(g->pi2), N, LX,
+      1.0 / (dx * dx), dt, dt, kA, pd, aSI, alpha, from_aSI, src);
   std::swap(g->u, g->u2);
   std::swap(g->pi, g->pi2);
 }

@@ -431,7 +431,7 @@ void gw_sync(clb_handle *h);
 __attribute__((visibility("hidden"))) bool su2_tangent_active(const clb_handle *h) { return h->su2->tangent; }
 
 // The GW kick (weight w of dt) with the lphi4SU2U1 source, at the current fields, momenta and a_I.
-__attribute__((visibility("hidden"))) void su2_gw_kick(clb_handle *h, double w, bool drift)
+__attribute__((visibility("hidden"))) void su2_gw_kick(clb_handle *h, double w)
 {
   SU2Sector *u = h->su2;
   GWSector *g = h->gw;
@@ -441,8 +441,7 @@ __attribute__((visibility("hidden"))) void su2_gw_kick(clb_handle *h, double w, 
     using R = decltype(zero);
     const SU2GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, u->prm.ddx,
                              (R)ndxg, (R)(r * r), &u->d_st->aI};
-    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, SU2GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &u->d_st->kA, &u->d_st->p3,
-                                                        &u->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
+    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, SU2GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, &u->d_st->kA, src, h->stream)));
   };
   if (u->fp32) go(0.0f);
   else go(0.0);

@@ -364,7 +364,7 @@ void gw_between_steps(clb_handle *h, bool more);
 void gw_sync(clb_handle *h);
 
 // The GW kick (weight w of dt) with the lphi4U1 source, at the current fields, momenta and a_I.
-__attribute__((visibility("hidden"))) void u1_gw_kick(clb_handle *h, double w, bool drift)
+__attribute__((visibility("hidden"))) void u1_gw_kick(clb_handle *h, double w)
 {
   U1Sector *u = h->u1;
   GWSector *g = h->gw;
@@ -373,8 +373,7 @@ __attribute__((visibility("hidden"))) void u1_gw_kick(clb_handle *h, double w, b
     using R = decltype(zero);
     const U1GWSource<R> src{static_cast<const R *>(u->f), static_cast<const R *>(u->p), h->n3, h->N, u->prm.ddx,
                             (R)u->prm.ndxg, (R)(r * r), &u->d_st->aI};
-    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, U1GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, drift, &u->d_st->kA, &u->d_st->cs_drift,
-                                                        &u->d_st->aSI, h->md.alpha, is_pv(h->cfg.evolver), src, h->stream)));
+    CLB_LAUNCH(h, K_GW, (launch_gw_kick<R, U1GWSource<R>>(g, h->N, h->cfg.dx, h->cfg.dt, w, &u->d_st->kA, src, h->stream)));
   };
   if (u->fp32) go(0.0f);
   else go(0.0);
