@@ -247,7 +247,7 @@ __attribute__((visibility("hidden"))) int su2_create(clb_handle *h)
   ok = ok && cudaMemset(u->f, 0, u->nf * u->esz) == cudaSuccess;
   ok = ok && cudaMemset(u->p, 0, NP * h->n3 * u->esz) == cudaSuccess;
   ok = ok && cudaMalloc(&u->ph, 12 * h->n3 * u->esz) == cudaSuccess;
-  u->stage_n = std::min(h->n3, kStageMax);
+  u->stage_n = std::min(NF * h->n3, kStageMax);
   ok = ok && cudaMalloc(&u->d_stage, u->stage_n * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_st, sizeof(State)) == cudaSuccess;
   ok = ok && cudaMalloc(&u->d_part, (size_t)kSU2Blocks * kMeas * sizeof(double)) == cudaSuccess;
@@ -321,38 +321,55 @@ CompView comp_view(const clb_handle *h, void *buf, bool field, int c)
   const double *p = comp_at<double>(h, buf, field, c, st);
   return CompView{p, st, false};
 }
-// The component from / to an FP64 array on the host or the device, in runs through the staging buffer
-// where the device holds it in FP32 or among others; ordered on the handle's stream.
-cudaError_t set_comp(clb_handle *h, void *buf, bool field, int c, const double *src)
+// A field or momentum buffer from / to its FP64 array on the host (or, to set, the device), ordered on the
+// handle's stream: components [c0, c1) that lie as in the array in one copy, others in runs through the
+// staging buffer.  A run spans components, and a state that fits the buffer is one run: a copy into
+// ordinary memory costs 12 to 26 us to start (16^3 FP64 read component by component 630 us, so 149).
+struct Segment {
+  int c0, c1;
+  bool direct;
+};
+std::vector<Segment> segments(const SU2Sector *u, bool field, size_t n3)
+{
+  if (u->fp32) return {{0, field ? NF : NP, false}};
+  if (!field) return {{0, NP, true}};
+  if (NF * n3 <= u->stage_n) return {{0, NF, false}};
+  return {{0, 3, true}, {3, 7, false}, {7, 10, true}, {10, NF, false}};
+}
+cudaError_t set_buf(clb_handle *h, void *buf, bool field, const double *src)
 {
   SU2Sector *u = h->su2;
-  const CompView v = comp_view(h, buf, field, c);
-  if (!v.f32 && v.stride == 1)
-    return cudaMemcpyAsync(const_cast<void *>(v.p), src, h->n3 * sizeof(double), cudaMemcpyDefault, h->stream);
-  for (size_t i = 0; i < h->n3; i += u->stage_n) {
-    const size_t n = std::min(u->stage_n, h->n3 - i);
-    const cudaError_t e = cudaMemcpyAsync(u->d_stage, src + i, n * sizeof(double), cudaMemcpyDefault, h->stream);
-    if (e != cudaSuccess) return e;
-    if (v.f32)
-      k_comp_set<float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, static_cast<float *>(const_cast<void *>(v.p)) + i * v.stride, v.stride, n);
-    else
-      k_comp_set<double><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, static_cast<double *>(const_cast<void *>(v.p)) + i * v.stride, v.stride, n);
+  for (const Segment &g : segments(u, field, h->n3)) {
+    const size_t j1 = (size_t)g.c1 * h->n3;
+    for (size_t j = (size_t)g.c0 * h->n3, n; j < j1; j += n) {
+      n = g.direct ? j1 - j : std::min(u->stage_n, j1 - j);
+      void *to = g.direct ? const_cast<void *>(comp_view(h, buf, field, g.c0).p) : u->d_stage;
+      const cudaError_t e = cudaMemcpyAsync(to, src + j, n * sizeof(double), cudaMemcpyDefault, h->stream);
+      if (e != cudaSuccess) return e;
+      if (g.direct) continue;
+      if (u->fp32)
+        k_state_set<float><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, u->prm, field, j, n, static_cast<float *>(buf));
+      else
+        k_state_set<double><<<kSU2Blocks, 256, 0, h->stream>>>(u->d_stage, u->prm, field, j, n, static_cast<double *>(buf));
+    }
   }
   return cudaGetLastError();
 }
-cudaError_t get_comp(clb_handle *h, void *buf, bool field, int c, double *dst)
+cudaError_t get_buf(clb_handle *h, void *buf, bool field, double *dst)
 {
   SU2Sector *u = h->su2;
-  const CompView v = comp_view(h, buf, field, c);
-  if (!v.f32 && v.stride == 1) return cudaMemcpyAsync(dst, v.p, h->n3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  for (size_t i = 0; i < h->n3; i += u->stage_n) {
-    const size_t n = std::min(u->stage_n, h->n3 - i);
-    if (v.f32)
-      k_comp_get<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(v.p) + i * v.stride, v.stride, u->d_stage, n);
-    else
-      k_comp_get<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(v.p) + i * v.stride, v.stride, u->d_stage, n);
-    const cudaError_t e = cudaMemcpyAsync(dst + i, u->d_stage, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e != cudaSuccess) return e;
+  for (const Segment &g : segments(u, field, h->n3)) {
+    const size_t j1 = (size_t)g.c1 * h->n3;
+    for (size_t j = (size_t)g.c0 * h->n3, n; j < j1; j += n) {
+      n = g.direct ? j1 - j : std::min(u->stage_n, j1 - j);
+      if (!g.direct && u->fp32)
+        k_state_get<float><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const float *>(buf), u->prm, field, j, n, u->d_stage);
+      else if (!g.direct)
+        k_state_get<double><<<kSU2Blocks, 256, 0, h->stream>>>(static_cast<const double *>(buf), u->prm, field, j, n, u->d_stage);
+      const void *from = g.direct ? comp_view(h, buf, field, g.c0).p : u->d_stage;
+      const cudaError_t e = cudaMemcpyAsync(dst + j, from, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+      if (e != cudaSuccess) return e;
+    }
   }
   return cudaGetLastError();
 }
@@ -364,8 +381,8 @@ __attribute__((visibility("hidden"))) int su2_set_state(clb_handle *h, const dou
   SU2Sector *u = h->su2;
   cudaError_t e = cudaStreamSynchronize(h->stream);
   free_tangent(u); // a new state ends the tangent-linear form
-  for (int c = 0; c < NF && e == cudaSuccess; ++c) e = set_comp(h, u->f, true, c, fields + (size_t)c * h->n3);
-  for (int c = 0; c < NP && e == cudaSuccess; ++c) e = set_comp(h, u->p, false, c, momenta + (size_t)c * h->n3);
+  if (e == cudaSuccess) e = set_buf(h, u->f, true, fields);
+  if (e == cudaSuccess) e = set_buf(h, u->p, false, momenta);
   if (e == cudaSuccess) {
     link_phases(h); // of the new A
     e = cudaGetLastError();
@@ -397,8 +414,8 @@ __attribute__((visibility("hidden"))) int su2_get_state(clb_handle *h, double *f
   SU2Sector *u = h->su2;
   State s;
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  for (int c = 0; c < NF && e == cudaSuccess && fields; ++c) e = get_comp(h, u->f, true, c, fields + (size_t)c * h->n3);
-  for (int c = 0; c < NP && e == cudaSuccess && momenta; ++c) e = get_comp(h, u->p, false, c, momenta + (size_t)c * h->n3);
+  if (e == cudaSuccess && fields) e = get_buf(h, u->f, true, fields);
+  if (e == cudaSuccess && momenta) e = get_buf(h, u->p, false, momenta);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&s, u->d_st, sizeof(s), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "clb_get_state");
@@ -788,10 +805,9 @@ __attribute__((visibility("hidden"))) int su2_tangent_begin(clb_handle *h, const
     free_tangent(u);
     return h->fail(CLB_ENOMEM, "clb_tangent_begin: tangent storage does not fit");
   }
-  e = cudaMemsetAsync(u->df, 0, u->nf * u->esz, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(u->dp, 0, NP * h->n3 * u->esz, h->stream);
-  for (int c = 0; c < NF && e == cudaSuccess && fields_dot; ++c) e = set_comp(h, u->df, true, c, fields_dot + (size_t)c * h->n3);
-  for (int c = 0; c < NP && e == cudaSuccess && momenta_dot; ++c) e = set_comp(h, u->dp, false, c, momenta_dot + (size_t)c * h->n3);
+  e = fields_dot ? set_buf(h, u->df, true, fields_dot) : cudaMemsetAsync(u->df, 0, u->nf * u->esz, h->stream);
+  if (e == cudaSuccess)
+    e = momenta_dot ? set_buf(h, u->dp, false, momenta_dot) : cudaMemsetAsync(u->dp, 0, NP * h->n3 * u->esz, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream); // the caller's arrays are read
   if (e != cudaSuccess) {
     free_tangent(u);
@@ -829,8 +845,8 @@ __attribute__((visibility("hidden"))) int su2_tangent_get_state(clb_handle *h, d
   SU2Sector *u = h->su2;
   if (!u->tangent) return h->fail(CLB_ESTATE, "clb_tangent_get_state: call clb_tangent_begin first");
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  for (int c = 0; c < NF && e == cudaSuccess && fields_dot; ++c) e = get_comp(h, u->df, true, c, fields_dot + (size_t)c * h->n3);
-  for (int c = 0; c < NP && e == cudaSuccess && momenta_dot; ++c) e = get_comp(h, u->dp, false, c, momenta_dot + (size_t)c * h->n3);
+  if (e == cudaSuccess && fields_dot) e = get_buf(h, u->df, true, fields_dot);
+  if (e == cudaSuccess && momenta_dot) e = get_buf(h, u->dp, false, momenta_dot);
   TState t;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&t, u->d_tst, sizeof(t), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);

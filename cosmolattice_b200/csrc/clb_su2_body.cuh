@@ -1379,17 +1379,32 @@ template <class S> __global__ void __launch_bounds__(256) k_unitarize_tan(S *__r
   }
 }
 
-// One field or momentum component between its place on the device (the elements base + stride s) and
-// an FP64 array.
-template <class S> __global__ void __launch_bounds__(256) k_comp_get(const S *__restrict__ src, int stride, double *__restrict__ dst, size_t n)
+// Elements [j0, j0 + n) of a state's FP64 array (component by component, N^3 each) from or to their places
+// in a field or momentum buffer.
+template <class Fn> __device__ __forceinline__ void for_state(const Params &a, bool field, size_t j0, size_t n, Fn fn)
 {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = (double)src[i * stride];
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  size_t c = (j0 + i) / a.n3, s = j0 + i - c * a.n3;
+  for (;;) {
+    fn(i, field ? fidx(a, (int)c, s) : c * a.n3 + s);
+    i += step;
+    if (i >= n) return;
+    for (s += step; s >= a.n3; s -= a.n3) ++c;
+  }
 }
-template <class S> __global__ void __launch_bounds__(256) k_comp_set(const double *__restrict__ src, S *__restrict__ dst, int stride, size_t n)
+template <class S>
+__global__ void __launch_bounds__(256)
+    k_state_get(const S *__restrict__ src, Params a, bool field, size_t j0, size_t n, double *__restrict__ dst)
 {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i * stride] = (S)src[i];
+  for_state(a, field, j0, n, [&](size_t i, size_t at) { dst[i] = (double)src[at]; });
+}
+template <class S>
+__global__ void __launch_bounds__(256)
+    k_state_set(const double *__restrict__ src, Params a, bool field, size_t j0, size_t n, S *__restrict__ dst)
+{
+  for_state(a, field, j0, n, [&](size_t i, size_t at) { dst[at] = (S)src[i]; });
 }
 
 } // namespace su2d
