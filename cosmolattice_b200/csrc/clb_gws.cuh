@@ -89,9 +89,8 @@ __global__ void __launch_bounds__(256) k_gw_kick(const R *__restrict__ u, R *__r
 // through shared memory (two planes, so one barrier per plane); the planes before and after stay in
 // registers.  (Loads one plane ahead: 145 us at 128^3 FP64; a cp.async ring of raw planes, drifted at each
 // read: 130, held by shared-memory reads.)  The neighbouring tiles read the undrifted state, so the sweep
-// writes another pair of arrays.  128^3 FP64: 81 us (ncu), against 36 (drift) + 76 (kick); what GWs add to
-// a step in the two forms, us: FP64 128^3 89 / 124, 192^3 246 / 397, 256^3 597 / 962; FP32 128^3 70 / 79,
-// 192^3 194 / 243.
+// writes another pair of arrays.  128^3 FP64: 76 us (ncu), against 36 (drift) + 74 (kick); what GWs add to
+// a step in the two forms, us: FP64 128^3 84 / 121, 256^3 580 / 944; FP32 128^3 67 / 77, 256^3 456 / 534.
 constexpr int kGWTileZ = 32, kGWTileY = 8;
 template <class R, class Src>
 __global__ void __launch_bounds__(kGWTileZ *kGWTileY, 2)
