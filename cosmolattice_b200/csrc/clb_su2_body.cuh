@@ -378,7 +378,9 @@ template <class S, class T> __device__ __forceinline__ T gB2(const Site<S, T> &v
 // a fine lattice, and the factor 4 / (dx^4 g^2) carries it through the start's a-dot into all momenta:
 // with links of rms 1e-3 the magnetic energy was off by 1e-5 to 2e-3 and the tangent observable by up to
 // a tenth, and every change of the products' rounding shifted a(t).  There plaq_dev is the gap, formed as
-// 2 (x^2 + y^2 + z^2) / (1 + w), the same for a unit quaternion and free of the cancellation.
+// 2 (x^2 + y^2 + z^2) / (1 + w), the same for a unit quaternion and free of the cancellation.  Its tangent
+// stays -2 dw, which does not cancel, and is the reference expression's for link tangents of any kind (the
+// quotient's is the same along the group only).
 template <class S, class T> __device__ __forceinline__ T gap(T dev)
 {
   if constexpr (sizeof(S) == 4)
@@ -388,13 +390,11 @@ template <class S, class T> __device__ __forceinline__ T gap(T dev)
 }
 template <class S, class T> __device__ __forceinline__ T plaq_dev(const Q4<T> &P)
 {
-  if constexpr (sizeof(S) == 4) {
-    typename TanTraits<T>::base w;
-    if constexpr (TanTraits<T>::is)
-      w = P.w.v;
-    else
-      w = P.w;
-    return w > 0 ? kdiv(2 * ((P.x * P.x + P.y * P.y) + P.z * P.z), 1 + P.w) : 2 - 2 * P.w;
+  if constexpr (sizeof(S) == 4 && TanTraits<T>::is) {
+    using B = typename TanTraits<T>::base;
+    return T(plaq_dev<S>(Q4<B>{P.w.v, P.x.v, P.y.v, P.z.v}), -2 * P.w.d);
+  } else if constexpr (sizeof(S) == 4) {
+    return P.w > 0 ? kdiv(2 * ((P.x * P.x + P.y * P.y) + P.z * P.z), 1 + P.w) : 2 - 2 * P.w;
   } else {
     return P.w;
   }

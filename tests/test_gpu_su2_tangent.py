@@ -314,3 +314,27 @@ def test_plain_evolution_after_a_spectrum_and_a_second_tangent_begin_is_bitwise(
         out.append(lat.get_state())
         lat.close()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
+
+
+@pytest.mark.parametrize("N", [8, 17])
+def test_fp32_tangent_along_any_start_tangent_tracks_fp64(N):
+    # link tangents that leave the group too: the FP32 form's <B^2> has the reference expression's
+    # tangent (fewer steps than the FP32 form's first re-unitarisation, which projects them)
+    from cosmolattice_b200 import Lattice
+    from cosmolattice_b200.adjoint import SU2_GAUGE_FRACTION
+
+    rp, m, f, p, sf = make_fine_su2_case(N, N)
+    rng = np.random.default_rng(N)
+    df, dp = 1e-2 * rng.standard_normal(f.shape), 1e-2 * rng.standard_normal(p.shape)
+    res = {}
+    for prec in ("fp64", "fp32"):
+        lat = Lattice(m, rp, precision=prec)
+        lat.set_state(f, p, sf)
+        lat.tangent_begin([0.1, 0.2, 0.3, 0.4, 1.0, 0.5], df, dp)
+        lat.initialize()
+        lat.evolve(6)
+        res[prec] = [np.asarray(x) for x in (*lat.tangent_get_state()[:2], lat.tangent_observable(SU2_GAUGE_FRACTION))]
+        lat.close()
+    for x, y in zip(res["fp32"], res["fp64"]):
+        print(N, np.linalg.norm(x - y) / np.linalg.norm(y))
+        assert np.linalg.norm(x - y) <= REL * np.linalg.norm(y)
