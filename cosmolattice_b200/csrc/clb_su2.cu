@@ -808,7 +808,7 @@ __attribute__((visibility("hidden"))) int su2_tangent_begin(clb_handle *h, const
   e = fields_dot ? set_buf(h, u->df, true, fields_dot) : cudaMemsetAsync(u->df, 0, u->nf * u->esz, h->stream);
   if (e == cudaSuccess)
     e = momenta_dot ? set_buf(h, u->dp, false, momenta_dot) : cudaMemsetAsync(u->dp, 0, NP * h->n3 * u->esz, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream); // the caller's arrays are read
+  if (e == cudaSuccess && (fields_dot || momenta_dot)) e = cudaStreamSynchronize(h->stream); // the caller's arrays are read
   if (e != cudaSuccess) {
     free_tangent(u);
     return h->cuda_fail(e, "clb_tangent_begin");
